@@ -536,15 +536,15 @@ __global__ void __cluster_dims__(kEigCluster, 1, 1) __launch_bounds__(kEigThread
   cluster.sync();  // no CTA leaves while another may still write into its shared memory
 }
 
-__global__ void gamma_quantiles_kernel(const double *shape, int batch, int K, double *x, double *dxda) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= batch * K) return;
-  const int b = e / K, k = e - b * K;
+__global__ void __launch_bounds__(32) gamma_quantiles_kernel(const double *shape, int K, double *x, double *dxda) {
+  const int e = blockIdx.x, b = e / K, k = e - b * K;
   const double q = (2.0 * k + 1.0) / (2.0 * K);
   double xv = 0.0, dv = 0.0;
-  if (!gamma_quantile(shape[b], q, xv, dv)) xv = dv = __longlong_as_double(0x7ff8000000000000ll);  // NaN
-  x[e] = xv;
-  dxda[e] = dv;
+  if (!gamma_quantile_warp(shape[b], q, xv, dv)) xv = dv = __longlong_as_double(0x7ff8000000000000ll);  // NaN
+  if (threadIdx.x == 0) {
+    x[e] = xv;
+    dxda[e] = dv;
+  }
 }
 
 int efail(int code, const std::string &msg) { return record_error(code, msg.c_str()); }
@@ -600,9 +600,8 @@ int tt_gamma_quantiles(int32_t batch, int32_t category_count, const double *shap
   if (!shape || !x || !dx_dshape) return tt::efail(TT_ERR_INVALID_ARGUMENT, "NULL argument");
   if (batch < 1 || category_count < 1) return tt::efail(TT_ERR_INVALID_ARGUMENT, "batch and categories must be >= 1");
   const int n = batch * category_count;
-  // one warp per CTA: the quantiles' FP64 work spreads over as many SMs as warps
-  tt::gamma_quantiles_kernel<<<(n + 31) / 32, 32, 0, static_cast<cudaStream_t>(stream)>>>(
-      shape, batch, category_count, x, dx_dshape);
+  // one warp per quantile and per CTA: the FP64 work spreads over as many SMs as there are quantiles
+  tt::gamma_quantiles_kernel<<<n, 32, 0, static_cast<cudaStream_t>(stream)>>>(shape, category_count, x, dx_dshape);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TT_OK
                           : tt::efail(TT_ERR_CUDA, std::string("gamma quantile launch: ") + cudaGetErrorString(e));
