@@ -78,7 +78,7 @@ int dev_alloc(tt_plan *p, P **ptr, size_t bytes, const char *what) {
 void release(tt_plan *p) {
   void *bufs[] = {p->d_steps, p->d_steps_rev, p->d_steps_ws, p->d_branch_pos, p->d_codes,    p->d_table,   p->d_weights,
                   p->d_pmat,  p->d_partials,   p->d_tile_lnl, p->d_gpart,   p->d_rootpart,
-                  p->d_G,     p->d_rootgrad,   p->d_status, p->d_qpart};
+                  p->d_G,     p->d_rootgrad,   p->d_status, p->d_qpart,    p->d_expo};
   for (void *b : bufs)
     if (b) cudaFree(b);
   tt::wide_destroy(p);
@@ -305,6 +305,7 @@ tt::PruneArgs<T> make_args(tt_plan *p, const double *props, const double *freqs,
   a.status = p->d_status;
   a.timeout_ns = kTimeoutNs;
   a.slots = 0;
+  a.expo = p->d_expo;
   return a;
 }
 
@@ -325,9 +326,18 @@ int slab_round(long long patterns, int N) {
 // Bytes of the gradient buffers (stored partials, per-tile gradient blocks,
 // per-tile root blocks) for `npat` patterns, with dev_alloc's 16-byte floor.
 struct GradBytes {
-  size_t partials, gpart, rootpart;
-  size_t total() const { return std::max(partials, size_t(16)) + std::max(gpart, size_t(16)) + std::max(rootpart, size_t(16)); }
+  size_t partials, gpart, rootpart, expo;
+  size_t total() const {
+    return std::max(partials, size_t(16)) + std::max(gpart, size_t(16)) + std::max(rootpart, size_t(16)) + expo;
+  }
 };
+
+// FP64 adjoint CTAs per sample for a pass over `n` patterns: at most td_slots,
+// with the tiles spread evenly over them.
+int td_pass_slots(const tt_plan *p, int n) {
+  const int nt = (n + p->tile_b - 1) / p->tile_b, per = (nt + p->td_slots - 1) / p->td_slots;
+  return (nt + per - 1) / per;
+}
 
 GradBytes grad_bytes(const tt_plan *p, int npat) {
   const bool f32 = p->precision == TT_PRECISION_F32;
@@ -337,15 +347,18 @@ GradBytes grad_bytes(const tt_plan *p, int npat) {
   const size_t kpad = f32 ? size_t(2 * tt::kpairs_for(p->K)) : size_t(p->K);
   const size_t ntb = (size_t(npat) + p->tile_b - 1) / p->tile_b;
   const size_t npad = f32 ? ntb * p->tile_b : size_t(npat);
+  // gradient blocks per (sample, branch): one per tile (FP32), one per adjoint CTA (FP64)
+  const size_t blocks = f32 ? ntb : std::min(ntb, size_t(p->td_slots));
   GradBytes g;
   g.partials = size_t(p->batch) * I1 * kpad * npad * p->S * p->elem;
-  g.gpart = size_t(p->batch) * p->B * ntb * kss * p->elem;
-  g.rootpart = size_t(p->batch) * ntb * (p->S + p->K) * p->elem;
+  g.gpart = size_t(p->batch) * p->B * blocks * kss * p->elem;
+  g.rootpart = size_t(p->batch) * blocks * (p->S + p->K) * p->elem;
+  g.expo = f32 ? 0 : size_t(p->batch) * I1 * npat * sizeof(int);
   return g;
 }
 
 void free_grad_buffers(tt_plan *p) {
-  for (void **b : {&p->d_partials, &p->d_gpart, &p->d_rootpart})
+  for (void **b : {&p->d_partials, &p->d_gpart, &p->d_rootpart, reinterpret_cast<void **>(&p->d_expo)})
     if (*b) {
       cudaFree(*b);
       *b = nullptr;
@@ -366,6 +379,7 @@ int alloc_grad_buffers(tt_plan *p, int slab) {
   int rc = dev_alloc(p, &p->d_partials, g.partials, "partials");
   if (!rc) rc = dev_alloc(p, &p->d_gpart, g.gpart, "gradient tiles");
   if (!rc) rc = dev_alloc(p, &p->d_rootpart, g.rootpart, "root tiles");
+  if (!rc && g.expo) rc = dev_alloc(p, &p->d_expo, g.expo, "scale exponents");
   p->grad_bytes = p->bytes - before;
   if (rc) {
     const std::string msg = g_last_error;
@@ -376,11 +390,13 @@ int alloc_grad_buffers(tt_plan *p, int slab) {
   return TT_OK;
 }
 
-// Slab size of a new plan whose pattern-sized buffers take `full` bytes for
-// the whole alignment: none when they fit in 7/8 of the free device memory
-// (or TT_GRADIENT_BUDGET_BYTES), else slabs sized to that budget.
+// Slab size of a new plan whose pattern-sized buffers take bytes(n) for n
+// patterns: none when the whole alignment's fit in 7/8 of the free device
+// memory (or TT_GRADIENT_BUDGET_BYTES), else slabs sized to that budget.
 // TT_SLAB_PATTERNS sets the slab explicitly.
-int choose_slab(const tt_plan *p, size_t full) {
+template <typename Bytes>
+int choose_slab(const tt_plan *p, Bytes bytes) {
+  const size_t full = bytes(p->N);
   if (const char *env = getenv("TT_SLAB_PATTERNS")) return slab_round(atoll(env), p->N);
   size_t free_b = 0, total_b = 0;
   size_t budget = SIZE_MAX;  // no slabs when the free memory cannot be read
@@ -391,7 +407,8 @@ int choose_slab(const tt_plan *p, size_t full) {
   if (const char *env = getenv("TT_GRADIENT_BUDGET_BYTES")) budget = std::min(budget, size_t(atoll(env)));
   if (full <= budget) return 0;
   const double per_pattern = double(full) / p->N;
-  const long long fit = (long long)(double(budget) / per_pattern) / kSlabAlign * kSlabAlign;
+  long long fit = (long long)(double(budget) / per_pattern) / kSlabAlign * kSlabAlign;
+  while (fit > kSlabAlign && bytes(int(fit)) > budget) fit -= kSlabAlign;  // parts that do not shrink with the slab
   return slab_round(std::max<long long>(kSlabAlign, fit), p->N);
 }
 
@@ -417,8 +434,8 @@ cudaError_t post_order(tt_plan *p, const double *props, const double *freqs, int
     return tt::launch_prune_f32(a, false, p->tile_f, plan_run_samples(p),
                                 (p->pair_threads ? tt::kF32PairThreads : 0) | (p->producer_warp ? tt::kF32ProducerWarp : 0), s);
   } else {
-    a.slots = p->slots_fwd;
-    return tt::launch_prune_f64(a, false, p->tile_f, plan_run_samples(p), s);
+    a.slots = p->slots_ws;
+    return tt::launch_td_f64(a, false, plan_run_samples(p), s);
   }
 }
 
@@ -467,7 +484,7 @@ int tt_plan_create(tt_plan **plan, int32_t tip_count, const int32_t *postorder,
   }
   if (p->S != 4) {  // amino-acid / codon / general models: level-scheduled wide-state kernels
     rc = tt::wide_create(p);
-    if (rc == TT_OK) rc = tt::wide_alloc_slab(p, choose_slab(p, tt::wide_pattern_bytes(p, p->N)));
+    if (rc == TT_OK) rc = tt::wide_alloc_slab(p, choose_slab(p, [p](int n) { return tt::wide_pattern_bytes(p, n); }));
     if (rc != TT_OK) {
       release(p);
       delete p;
@@ -479,28 +496,25 @@ int tt_plan_create(tt_plan **plan, int32_t tip_count, const int32_t *postorder,
   int smem_max = 0;
   cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device);
   const bool f32 = precision == TT_PRECISION_F32;
-  const int *ftiles = f32 ? tt::kFwdTilesF32 : tt::kFwdTilesF64;
-  const int *btiles = f32 ? tt::kBwdTilesF32 : tt::kBwdTilesF64;
   if (f32) {  // ring depths of the FP32 kernels; TT_FWD_STAGES / TT_BWD_STAGES override
     p->nstage_f = getenv("TT_FWD_STAGES") ? std::max(2, atoi(getenv("TT_FWD_STAGES"))) : tt::kTlFwdStages;
     p->nstage_b = getenv("TT_BWD_STAGES") ? std::max(2, atoi(getenv("TT_BWD_STAGES"))) : tt::kTlBwdStages;
   }
-  auto smem_of = [&](int tile, bool bwd) {
+  auto smem_of = [&](bool bwd) {
     const int slots = bwd ? p->slots_bwd : p->slots_fwd;
     const int ns = bwd ? p->nstage_b : p->nstage_f;
-    return f32 ? std::max({tt::tl_smem_bytes(p->K, 256, slots, bwd, ns), tt::tq_smem_bytes(p->K, 256, slots, bwd, ns),
+    return std::max({tt::tl_smem_bytes(p->K, 256, slots, bwd, ns), tt::tq_smem_bytes(p->K, 256, slots, bwd, ns),
                            bwd ? size_t(0) : tt::tl_ws_smem_bytes(p->K, 256, p->slots_ws, ns),
                            bwd ? std::max(tt::ta_smem_bytes(p->K, 256, ns), tt::tp_smem_bytes(p->K, 256, ns))
-                               : size_t(0)})
-               : tt::prune_smem_bytes<double>(4, p->K, 256, slots, tile, bwd);
+                               : size_t(0)});
   };
   // optional overrides for tuning sweeps: TT_FWD_TILE / TT_BWD_TILE.  FP32 rings
   // shrink (down to 3 stages) before a smaller tile is tried.
-  auto fits = [&](int tile, bool bwd) {
+  auto fits = [&](bool bwd) {
     int &ns = bwd ? p->nstage_b : p->nstage_f;
     const int want = ns;
-    for (; ns >= (f32 ? std::min(3, want) : want); --ns)
-      if (smem_of(tile, bwd) <= size_t(smem_max)) return true;
+    for (; ns >= std::min(3, want); --ns)
+      if (smem_of(bwd) <= size_t(smem_max)) return true;
     ns = want;
     return false;
   };
@@ -509,14 +523,24 @@ int tt_plan_create(tt_plan **plan, int32_t tip_count, const int32_t *postorder,
     if (o) {
       const int want = atoi(o);
       for (int i = 0; i < 2; ++i)
-        if (cand[i] == want && fits(want, bwd)) return want;
+        if (cand[i] == want && fits(bwd)) return want;
     }
     for (int i = 0; i < 2; ++i)
-      if (fits(cand[i], bwd)) return cand[i];
+      if (fits(bwd)) return cand[i];
     return 0;
   };
-  p->tile_f = pick(ftiles, false, "TT_FWD_TILE");
-  p->tile_b = pick(btiles, true, "TT_BWD_TILE");
+  if (f32) {
+    p->tile_f = pick(tt::kFwdTilesF32, false, "TT_FWD_TILE");
+    p->tile_b = pick(tt::kBwdTilesF32, true, "TT_BWD_TILE");
+  } else if (tt::td_smem_bytes(p->K, 256, p->slots_ws, false) <= size_t(smem_max) &&
+             tt::td_smem_bytes(p->K, 256, p->slots_bwd, true) <= size_t(smem_max)) {
+    p->tile_f = p->tile_b = tt::td_tile_patterns(p->K);
+    // adjoint CTAs (one warp each) per sample: kTdCtasPerSm on every SM over the batch, fewer where
+    // the shared memory of a deep tree's stack holds fewer
+    const size_t smem = tt::td_smem_bytes(p->K, 16, p->slots_bwd, true) + 1024;
+    const int per_sm = std::max(1, std::min(tt::kTdCtasPerSm, int(size_t(smem_max) / smem)));
+    p->td_slots = std::max(1, 152 * per_sm / batch);
+  }
   if (!p->tile_f || !p->tile_b) {
     delete p;
     return fail(TT_ERR_UNSUPPORTED, "tree needs " + std::to_string(std::max(p->slots_fwd, p->slots_bwd)) +
@@ -559,7 +583,7 @@ int tt_plan_create(tt_plan **plan, int32_t tip_count, const int32_t *postorder,
   if (!rc) rc = dev_alloc(p, &p->d_rootgrad, size_t(batch) * (p->S + p->K) * sizeof(double), "root grads");
   if (!rc) rc = dev_alloc(p, &p->d_status, sizeof(int), "status");
   if (!rc) {
-    rc = alloc_grad_buffers(p, choose_slab(p, grad_bytes(p, p->N).total()));
+    rc = alloc_grad_buffers(p, choose_slab(p, [p](int n) { return grad_bytes(p, n).total(); }));
   }
   if (rc) {
     release(p);
@@ -936,8 +960,8 @@ int tt_gradient(tt_plan *p, const double *props, const double *freqs, double *gr
       p->launches += 1;
       if (e != cudaSuccess) break;
     }
-    const int ntiles = (n + p->tile_b - 1) / p->tile_b;
     if (p->precision == TT_PRECISION_F32) {
+      const int ntiles = (n + p->tile_b - 1) / p->tile_b;
       auto a = make_args<float>(p, props, freqs, 1, true, nullptr);
       a.slots = p->slots_bwd;
       a.nstage = p->nstage_b;
@@ -957,11 +981,12 @@ int tt_gradient(tt_plan *p, const double *props, const double *freqs, double *gr
       auto a = make_args<double>(p, props, freqs, 1, true, nullptr);
       a.slots = p->slots_bwd;
       slab_args(a, p0, n, p->tile_b);
-      e = tt::launch_prune_f64(a, true, p->tile_b, plan_run_samples(p), s);
+      a.nslots = td_pass_slots(p, n);
+      e = tt::launch_td_f64(a, true, plan_run_samples(p), s);
       if (e == cudaSuccess)
         e = tt::launch_reduce_f64(static_cast<const double *>(p->d_gpart),
                                   static_cast<const double *>(p->d_rootpart), p->d_G, p->d_rootgrad,
-                                  p->d_rootgrad + size_t(p->batch) * p->S, plan_run_samples(p), p->B, ntiles, p->S,
+                                  p->d_rootgrad + size_t(p->batch) * p->S, plan_run_samples(p), p->B, a.nslots, p->S,
                                   p->K, p0 > 0, s);
     }
     p->launches += 3;

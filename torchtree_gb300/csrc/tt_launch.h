@@ -33,7 +33,6 @@ constexpr int kTlBwdThreads = 64;
 constexpr int kFwdTilesF32[2] = {kTlTile, kTlTile};
 constexpr int kBwdTilesF32[2] = {kTlTile, kTlTile};
 constexpr int kFwdTilesF64[2] = {64, 32};
-constexpr int kBwdTilesF64[2] = {64, 32};
 constexpr int kStages = 4;
 // default staging-ring depths of the FP32 kernels (reduced to fit shared memory)
 constexpr int kTlFwdStages = 3;
@@ -89,8 +88,14 @@ bool pair_adjoint_supported(int K);
 cudaError_t launch_forward_multi(const MultiPrune<float> &m, int total, size_t smem, cudaStream_t stream);
 cudaError_t launch_adjoint_multi(const MultiPrune<float> &m, int total, size_t smem, bool pair_adjoint,
                                  cudaStream_t stream);
-cudaError_t launch_prune_f64(const PruneArgs<double> &a, bool backward, int tile, int batch,
-                             cudaStream_t stream);
+// FP64 post-order without stored partials (tt_log_likelihood_static)
+cudaError_t launch_prune_f64(const PruneArgs<double> &a, int tile, int batch, cudaStream_t stream);
+// FP64 plans: post-order over a.ntiles tiles of td_tile(K) patterns, and the
+// adjoint with a.nslots CTAs per sample
+cudaError_t launch_td_f64(const PruneArgs<double> &a, bool backward, int batch, cudaStream_t stream);
+size_t td_smem_bytes(int K, int C, int slots, bool backward);
+int td_tile_patterns(int K);
+constexpr int kTdCtasPerSm = 8;
 
 // Sum the per-tile gradient blocks into G / dfreq / dprop; accumulate = 1
 // adds to what is there (pattern slabs after the first).

@@ -49,6 +49,8 @@ struct tt_plan {
   double *d_tile_lnl = nullptr;
   void *d_gpart = nullptr;
   void *d_rootpart = nullptr;
+  int *d_expo = nullptr;  // FP64 4-state: the stored nodes' scale exponents
+  int td_slots = 0;       // FP64 4-state: most adjoint CTAs per sample
   double *d_G = nullptr;
   double *d_rootgrad = nullptr;
   int *d_status = nullptr;

@@ -80,6 +80,10 @@ struct PruneArgs {
   unsigned long long timeout_ns;
   // records of the producer-warp post-order (kWs* slots), or nullptr
   const int4 *steps_ws = nullptr;
+  // FP64 plans: the power of two taken out at each stored node, [batch][n_steps-1][N], and the
+  // adjoint's gradient blocks per branch (its CTAs per sample)
+  int *expo = nullptr;
+  int nslots = 0;
 };
 
 // Arguments of one launch over several plans (one kernel parameter block):
@@ -374,272 +378,6 @@ __global__ void __launch_bounds__(TILE) prune_forward_kernel(const PruneArgs<T> 
 #pragma unroll
     for (int w = 0; w < TILE / 32; ++w) tot += warp_tot[w];
     a.tile_lnl[size_t(b) * a.ntiles + tile] = tot;
-  }
-}
-
-// ----------------------------------------------------------------- backward
-template <typename T, int S, int KMAX, int TILE, int NSTAGE>
-__global__ void __launch_bounds__(TILE) prune_backward_kernel(const PruneArgs<T> a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  constexpr int NW = TILE / 32;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int b = blockIdx.y;
-  const int tile = blockIdx.x;
-  const int n = tile * TILE + tid;
-  const bool act = n < a.N;
-  const int rem = min(TILE, a.N - tile * TILE);
-  const int K = a.K;
-  const int KS = K * S;
-  const int KSS = K * S * S;
-  const int RK = S + K;
-  const int XS = KS + 16 / int(sizeof(T));  // padded row: conflict-free vector stores
-  const int nst = a.n_steps;
-  const StackLayout L = stack_layout<T>(S, K, a.C, a.slots, TILE, NSTAGE, KMAX, true);
-  const StageLayout G = stage_layout<T>(S, K, TILE, true);
-  unsigned char *stages = smem + L.stages;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
-  T *tab = reinterpret_cast<T *>(smem + L.table);
-  T *stk = reinterpret_cast<T *>(smem + L.stack);
-  T *xbuf = reinterpret_cast<T *>(smem + L.xbuf);  // [2][TILE][XS]  coef * outside partial
-  T *red = reinterpret_cast<T *>(smem + L.red);    // [2][rows][Q][S]
-  T *redr = reinterpret_cast<T *>(smem + L.red_root);
-  // transpose-reduction work split: rows (child, k, i), Q pattern chunks
-  const int rows = 2 * KS;
-  const int Q = TILE >= rows ? TILE / rows : 1;
-  const int chunk = (TILE + Q - 1) / Q;
-  const T w = act ? T(a.weights[n]) : T(0);
-
-  int4 nxt[3];
-  if (tid == 0) {
-#pragma unroll
-    for (int st = 0; st < NSTAGE; ++st) mbar_init(&bars[st], 1);
-    fence_barrier_init();
-  }
-  for (int i = tid; i < a.C * S; i += TILE) tab[i] = a.table[i];
-  double props[KMAX], freqs[S];
-#pragma unroll
-  for (int k = 0; k < KMAX; ++k) props[k] = k < K ? a.props[b * K + k] : 0.0;
-#pragma unroll
-  for (int i = 0; i < S; ++i) freqs[i] = a.freqs[b * S + i];
-  __syncthreads();
-  // iteration j handles step nst-1-j and uses stage j % NSTAGE
-  if (tid == 0) {
-    load_rec(nxt, a.steps, nst - 1);
-    for (int j = 0; j < NSTAGE - 1 && j < nst; ++j) {
-      int4 cur[3] = {nxt[0], nxt[1], nxt[2]};
-      if (j + 1 < nst) load_rec(nxt, a.steps, nst - 2 - j);
-      issue_step<T, S, true>(a, stages + j * G.bytes, &bars[j], cur, nst - 1 - j, b, tile, TILE, G);
-    }
-  }
-  bool timed_out = !mbar_wait_bounded(&bars[0], 0, a.timeout_ns);
-  if (__syncthreads_or(timed_out)) {
-    if (tid == 0) drain_after_timeout<NSTAGE>(bars, 0, min(NSTAGE - 2, nst - 1), a.status);
-    return;
-  }
-
-  int prev_left = -1, prev_right = -1;
-  for (int j = 0; j <= nst; ++j) {
-    // finish the transpose reduction of iteration j-1 (published by the barrier that closed it)
-    if (j > 0) {
-      const T *rb = red + size_t((j - 1) & 1) * rows * Q * S;
-      for (int e = tid; e < 2 * KSS; e += TILE) {
-        const int side = e >= KSS;
-        const int ei = side ? e - KSS : e;  // (k, i, jj) of this child
-        const int row = side * KS + ei / S;
-        const int jj = ei % S;
-        T acc = T(0);
-        for (int q = 0; q < Q; ++q) acc += rb[(row * Q + q) * S + jj];
-        const int branch = side ? prev_right : prev_left;
-        a.gpart[((size_t(b) * a.branch_count + branch) * a.ntiles + tile) * KSS + ei] = acc;
-      }
-    }
-    if (j == nst) break;
-    if (tid == 0 && j + NSTAGE - 1 < nst) {
-      const int jp = j + NSTAGE - 1;
-      int4 cur[3] = {nxt[0], nxt[1], nxt[2]};
-      if (jp + 1 < nst) load_rec(nxt, a.steps, nst - 2 - jp);
-      issue_step<T, S, true>(a, stages + (jp % NSTAGE) * G.bytes, &bars[jp % NSTAGE], cur, nst - 1 - jp, b,
-                             tile, TILE, G);
-    }
-    const unsigned char *stg = stages + (j % NSTAGE) * G.bytes;
-    const int4 *rec = reinterpret_cast<const int4 *>(stg + G.rec);
-    const int4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
-    const int left = r0.y, right = r0.z;
-    const int slot_in = r1.z, slot_l = r1.w, slot_r = r2.x;
-    const bool is_root = slot_in < 0;
-    const bool ltip = left < a.tip_count, rtip = right < a.tip_count;
-    const T *Pl = reinterpret_cast<const T *>(stg + G.pm);
-    const T *Pr = Pl + KSS;
-    const T *kidl = reinterpret_cast<const T *>(stg + G.kids);
-    const T *kidr = kidl + size_t(K) * TILE * S;
-    T tl[S], tr[S];
-    if (ltip) load_vec<T, S>(tl, tab + int(stg[G.codes + tid]) * S);
-    if (rtip) load_vec<T, S>(tr, tab + int(stg[G.codes + TILE + tid]) * S);
-
-    // ---- phase A: per pattern, all categories
-    T xl[KMAX][S], xr[KMAX][S];  // outside partials at the tops of the two branches
-    T ol[KMAX][S], orr[KMAX][S];  // outside partials at the bottoms of the children
-    T rg_pi[S], rg_c[KMAX];
-#pragma unroll
-    for (int i = 0; i < S; ++i) rg_pi[i] = T(0);
-    T den = T(0);
-#pragma unroll
-    for (int k = 0; k < KMAX; ++k) {
-      rg_c[k] = T(0);
-      if (k < K) {
-        T pre[S], vl[S], vr[S], al[S], ar[S];
-        if (is_root) {
-#pragma unroll
-          for (int i = 0; i < S; ++i) pre[i] = T(props[k] * freqs[i]);
-        } else {
-          load_vec<T, S>(pre, stk + (size_t(slot_in * K + k) * TILE + tid) * S);
-        }
-        if (ltip) {
-#pragma unroll
-          for (int i = 0; i < S; ++i) vl[i] = tl[i];
-        } else {
-          load_vec<T, S>(vl, kidl + (size_t(k) * TILE + tid) * S);
-        }
-        if (rtip) {
-#pragma unroll
-          for (int i = 0; i < S; ++i) vr[i] = tr[i];
-        } else {
-          load_vec<T, S>(vr, kidr + (size_t(k) * TILE + tid) * S);
-        }
-        T pl[S][S], pr[S][S];  // this category's two matrices, read once
-#pragma unroll
-        for (int i = 0; i < S; ++i) {
-          load_vec<T, S>(pl[i], Pl + (k * S + i) * S);
-          load_vec<T, S>(pr[i], Pr + (k * S + i) * S);
-        }
-#pragma unroll
-        for (int i = 0; i < S; ++i) {
-          T sa = T(0), sb = T(0);
-#pragma unroll
-          for (int jj = 0; jj < S; ++jj) {
-            sa = fma(pl[i][jj], vl[jj], sa);
-            sb = fma(pr[i][jj], vr[jj], sb);
-          }
-          al[i] = sa;
-          ar[i] = sb;
-        }
-#pragma unroll
-        for (int i = 0; i < S; ++i) {
-          xl[k][i] = pre[i] * ar[i];
-          xr[k][i] = pre[i] * al[i];
-          den = fma(xl[k][i], al[i], den);
-          if (is_root) {
-            const T r = al[i] * ar[i];
-            rg_pi[i] = fma(T(props[k]), r, rg_pi[i]);
-            rg_c[k] = fma(T(freqs[i]), r, rg_c[k]);
-          }
-        }
-        // outside partials of the children (scale-free: no coefficient)
-#pragma unroll
-        for (int jj = 0; jj < S; ++jj) {
-          T sa = T(0), sb = T(0);
-#pragma unroll
-          for (int i = 0; i < S; ++i) {
-            sa = fma(pl[i][jj], xl[k][i], sa);
-            sb = fma(pr[i][jj], xr[k][i], sb);
-          }
-          ol[k][jj] = sa;
-          orr[k][jj] = sb;
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < S; ++i) xl[k][i] = xr[k][i] = ol[k][i] = orr[k][i] = T(0);
-      }
-    }
-    // dlnL_n/dP = w_n * x (outer) v / L_n; every factor's per-pattern scale
-    // cancels against den, so no scaler bookkeeping is needed.
-    const T coef = (act && den > T(0)) ? w / den : T(0);
-    {
-      T *xl_dst = xbuf + size_t(tid) * XS;
-      T *xr_dst = xbuf + size_t(TILE + tid) * XS;
-#pragma unroll
-      for (int k = 0; k < KMAX; ++k)
-        if (k < K) {
-          T u[S], v[S];
-#pragma unroll
-          for (int i = 0; i < S; ++i) {
-            u[i] = coef * xl[k][i];
-            v[i] = coef * xr[k][i];
-          }
-          store_vec<T, S>(xl_dst + k * S, u);
-          store_vec<T, S>(xr_dst + k * S, v);
-        }
-    }
-    if (is_root) {
-#pragma unroll
-      for (int i = 0; i < S; ++i) {  // lanes past the last pattern hold stale data: mask them
-        const T acc = warp_sum(act ? coef * rg_pi[i] : T(0));
-        if (lane == 0) redr[warp * (S + KMAX) + i] = acc;
-      }
-#pragma unroll
-      for (int k = 0; k < KMAX; ++k)
-        if (k < K) {
-          const T acc = warp_sum(act ? coef * rg_c[k] : T(0));
-          if (lane == 0) redr[warp * (S + KMAX) + S + k] = acc;
-        }
-    }
-    if (!ltip) {
-      int E = 0;
-      rescale_pow2<T, S, KMAX>(ol, K, E);
-#pragma unroll
-      for (int k = 0; k < KMAX; ++k)
-        if (k < K) store_vec<T, S>(stk + (size_t(slot_l * K + k) * TILE + tid) * S, ol[k]);
-    }
-    if (!rtip) {
-      int E = 0;
-      rescale_pow2<T, S, KMAX>(orr, K, E);
-#pragma unroll
-      for (int k = 0; k < KMAX; ++k)
-        if (k < K) store_vec<T, S>(stk + (size_t(slot_r * K + k) * TILE + tid) * S, orr[k]);
-    }
-    __syncthreads();  // xbuf complete
-
-    // ---- phase C: G[c][k][i][:] = sum_n xbuf[c][n][k,i] * v_c[k][n][:]
-    {
-      T *rw = red + size_t(j & 1) * rows * Q * S;
-      for (int item = tid; item < rows * Q; item += TILE) {
-        const int row = item / Q, q = item % Q;
-        const int c = row >= KS;
-        const int ki = c ? row - KS : row;
-        const int k = ki / S;
-        const bool tipc = c ? rtip : ltip;
-        const T *xs = xbuf + size_t(c) * TILE * XS + ki;
-        const T *vs = (c ? kidr : kidl) + size_t(k) * TILE * S;
-        const unsigned char *cs = stg + G.codes + c * TILE;
-        T acc[S];
-#pragma unroll
-        for (int jj = 0; jj < S; ++jj) acc[jj] = T(0);
-        const int n0 = q * chunk, n1 = min(n0 + chunk, rem);
-        for (int m = n0; m < n1; ++m) {
-          const T x = xs[size_t(m) * XS];
-          T v[S];
-          load_vec<T, S>(v, tipc ? tab + int(cs[m]) * S : vs + size_t(m) * S);
-#pragma unroll
-          for (int jj = 0; jj < S; ++jj) acc[jj] = fma(x, v[jj], acc[jj]);
-        }
-        store_vec<T, S>(rw + (size_t(row) * Q + q) * S, acc);
-      }
-    }
-    prev_left = left;
-    prev_right = right;
-    if (j + 1 < nst)
-      timed_out = !mbar_wait_bounded(&bars[(j + 1) % NSTAGE], ((j + 1) / NSTAGE) & 1, a.timeout_ns);
-    if (__syncthreads_or(timed_out)) {
-      if (tid == 0) drain_after_timeout<NSTAGE>(bars, j + 1, min(j + NSTAGE - 1, nst - 1), a.status);
-      return;
-    }
-    if (is_root)
-      for (int e = tid; e < RK; e += TILE) {
-        T acc = T(0);
-#pragma unroll
-        for (int ww = 0; ww < NW; ++ww) acc += redr[ww * (S + KMAX) + e];
-        a.rootpart[(size_t(b) * a.ntiles + tile) * RK + e] = acc;
-      }
   }
 }
 

@@ -3,39 +3,56 @@
 #include "tt_launch.h"
 #include "tt_pmatrix.cuh"
 #include "tt_prune.cuh"
+#include "tt_prune_td.cuh"
 
 namespace tt {
 
 namespace {
 
-template <int KMAX, int TILE, bool BACKWARD>
+template <int KMAX, int TILE>
 cudaError_t launch_one(const PruneArgs<double> &a, int batch, cudaStream_t stream) {
-  const size_t smem = prune_smem_bytes<double>(4, a.K, a.C, a.slots, TILE, BACKWARD);
-  const dim3 grid(a.ntiles, batch);
-  if (BACKWARD) {
-    auto kern = prune_backward_kernel<double, 4, KMAX, TILE, kStages>;
-    cudaError_t e = kernel_smem(kern, smem);
-    if (e != cudaSuccess) return e;
-    kern<<<grid, TILE, smem, stream>>>(a);
-  } else {
-    auto kern = prune_forward_kernel<double, 4, KMAX, TILE, kStages>;
-    cudaError_t e = kernel_smem(kern, smem);
-    if (e != cudaSuccess) return e;
-    kern<<<grid, TILE, smem, stream>>>(a);
-  }
+  const size_t smem = prune_smem_bytes<double>(4, a.K, a.C, a.slots, TILE, false);
+  auto kern = prune_forward_kernel<double, 4, KMAX, TILE, kStages>;
+  cudaError_t e = kernel_smem(kern, smem);
+  if (e != cudaSuccess) return e;
+  kern<<<dim3(a.ntiles, batch), TILE, smem, stream>>>(a);
   return cudaGetLastError();
 }
 
-template <int TILE, bool BACKWARD>
+template <int TILE>
 cudaError_t by_k(const PruneArgs<double> &a, int batch, cudaStream_t stream) {
   switch (kmax_for(a.K)) {
-    case 1: return launch_one<1, TILE, BACKWARD>(a, batch, stream);
-    case 4: return launch_one<4, TILE, BACKWARD>(a, batch, stream);
-    default: return launch_one<8, TILE, BACKWARD>(a, batch, stream);
+    case 1: return launch_one<1, TILE>(a, batch, stream);
+    case 4: return launch_one<4, TILE>(a, batch, stream);
+    default: return launch_one<8, TILE>(a, batch, stream);
   }
 }
 
+template <int KP>
+cudaError_t launch_td(const PruneArgs<double> &a, bool backward, int batch, cudaStream_t stream) {
+  const size_t smem = size_t(td_layout(a.K, a.C, a.slots, backward).total);
+  cudaError_t e = backward ? kernel_smem(td_backward_kernel<KP>, smem, true) : kernel_smem(td_forward_kernel<KP>, smem, true);
+  if (e != cudaSuccess) return e;
+  if (backward)
+    td_backward_kernel<KP><<<dim3(a.nslots, batch), 32, smem, stream>>>(a);
+  else
+    td_forward_kernel<KP><<<dim3(a.ntiles, batch), 32, smem, stream>>>(a);
+  return cudaGetLastError();
+}
+
 }  // namespace
+
+size_t td_smem_bytes(int K, int C, int slots, bool backward) { return size_t(td_layout(K, C, slots, backward).total); }
+int td_tile_patterns(int K) { return td_tile(K); }
+
+cudaError_t launch_td_f64(const PruneArgs<double> &a, bool backward, int batch, cudaStream_t stream) {
+  switch (td_lanes(a.K)) {
+    case 1: return launch_td<1>(a, backward, batch, stream);
+    case 2: return launch_td<2>(a, backward, batch, stream);
+    case 4: return launch_td<4>(a, backward, batch, stream);
+    default: return launch_td<8>(a, backward, batch, stream);
+  }
+}
 
 __global__ void reduce_lnl_kernel(const double *tile_lnl, double *lnl, int ntiles, int accumulate) {
   __shared__ double part[8];
@@ -52,15 +69,9 @@ __global__ void reduce_lnl_kernel(const double *tile_lnl, double *lnl, int ntile
   }
 }
 
-cudaError_t launch_prune_f64(const PruneArgs<double> &a, bool backward, int tile, int batch,
-                             cudaStream_t stream) {
-  if (backward) {
-    if (tile == kBwdTilesF64[0]) return by_k<kBwdTilesF64[0], true>(a, batch, stream);
-    if (tile == kBwdTilesF64[1]) return by_k<kBwdTilesF64[1], true>(a, batch, stream);
-  } else {
-    if (tile == kFwdTilesF64[0]) return by_k<kFwdTilesF64[0], false>(a, batch, stream);
-    if (tile == kFwdTilesF64[1]) return by_k<kFwdTilesF64[1], false>(a, batch, stream);
-  }
+cudaError_t launch_prune_f64(const PruneArgs<double> &a, int tile, int batch, cudaStream_t stream) {
+  if (tile == kFwdTilesF64[0]) return by_k<kFwdTilesF64[0]>(a, batch, stream);
+  if (tile == kFwdTilesF64[1]) return by_k<kFwdTilesF64[1]>(a, batch, stream);
   return cudaErrorInvalidValue;
 }
 
