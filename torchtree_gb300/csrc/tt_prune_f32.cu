@@ -218,7 +218,7 @@ cudaError_t launch_reduce_f32(const float *gpart, const float *rootpart, double 
   const int kss = K * S * S;
   reduce_branch_grads_kernel<float><<<dim3(B, batch), kss <= 64 ? 64 : 128, 0, stream>>>(
       gpart, G, B, ntiles, kss, accumulate);
-  reduce_root_grads_kernel<float><<<batch, 32, 0, stream>>>(rootpart, dfreq, dprop, ntiles, S, K, accumulate);
+  reduce_root_grads_kernel<float><<<batch, 256, 0, stream>>>(rootpart, dfreq, dprop, ntiles, S, K, accumulate);
   return cudaGetLastError();
 }
 

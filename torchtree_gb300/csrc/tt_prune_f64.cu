@@ -81,7 +81,7 @@ cudaError_t launch_reduce_f64(const double *gpart, const double *rootpart, doubl
   const int kss = K * S * S;
   reduce_branch_grads_kernel<double><<<dim3(B, batch), kss <= 64 ? 64 : 128, 0, stream>>>(
       gpart, G, B, ntiles, kss, accumulate);
-  reduce_root_grads_kernel<double><<<batch, 32, 0, stream>>>(rootpart, dfreq, dprop, ntiles, S, K, accumulate);
+  reduce_root_grads_kernel<double><<<batch, 256, 0, stream>>>(rootpart, dfreq, dprop, ntiles, S, K, accumulate);
   return cudaGetLastError();
 }
 

@@ -17,36 +17,6 @@
 
 namespace tt {
 
-__global__ void wide_root_kernel(const double *root_site, const int *root_expo, const double *props,
-                                 const double *weights, double *site_lnl, double *log2L, double *block_lnl,
-                                 int K, int N, int Npad) {
-  __shared__ double part[8];
-  const int b = blockIdx.y, n = blockIdx.x * 256 + threadIdx.x;
-  double contrib = 0.0;
-  if (n < N) {
-    int emax = INT_MIN;
-    for (int k = 0; k < K; ++k) emax = max(emax, root_expo[(size_t(b) * K + k) * Npad + n]);
-    double s = 0.0;
-    for (int k = 0; k < K; ++k) {
-      const size_t o = (size_t(b) * K + k) * Npad + n;
-      s += props[size_t(b) * K + k] * ldexp(root_site[o], root_expo[o] - emax);
-    }
-    const double l2 = log2(s) + double(emax);
-    const double ll = l2 * 0.69314718055994530942;
-    if (site_lnl) site_lnl[size_t(b) * N + n] = ll;
-    log2L[size_t(b) * Npad + n] = l2;
-    contrib = weights[n] * ll;
-  }
-  contrib = warp_sum(contrib);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = contrib;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < 8; ++w) t += part[w];
-    block_lnl[size_t(b) * gridDim.x + blockIdx.x] = t;
-  }
-}
-
 __global__ void wide_pmatrix_grad_reduce_kernel(const double *part, int nchunks, int S, int K, double *dlam,
                                                 double *dU, double *dW, double *drates) {
   const int b = blockIdx.x;
@@ -90,7 +60,8 @@ struct WideState {
   int *d_expo = nullptr;
   double *d_root_site = nullptr;
   int *d_root_expo = nullptr;
-  double *d_log2L = nullptr;
+  void *d_coef = nullptr;  // the adjoint's per-pattern coefficients and exponents
+  int *d_cexp = nullptr;
   double *d_block_lnl = nullptr;
   void *d_gpart = nullptr;
   void *d_rootpart = nullptr;
@@ -257,7 +228,8 @@ struct Wide {
     a.weights = p->d_weights + p0;
     a.root_site = w.d_root_site;
     a.root_expo = w.d_root_expo;
-    a.log2L = w.d_log2L;
+    a.coef = static_cast<const T *>(w.d_coef);
+    a.cexp = w.d_cexp;
     a.gpart = static_cast<T *>(w.d_gpart);
     a.rootpart = static_cast<T *>(w.d_rootpart);
     a.prod = nullptr;
@@ -299,8 +271,9 @@ struct Wide {
       wide_forward_kernel<T, SP, PTF><<<grid, NT, smem, s>>>(a);
       p->launches += 1;
     }
-    wide_root_kernel<<<dim3(g.nblk, plan_run_samples(p)), 256, 0, s>>>(w.d_root_site, w.d_root_expo, props, a.weights,
-                                                           site_lnl, w.d_log2L, w.d_block_lnl, p->K, n, g.Npad);
+    wide_root_kernel<T><<<dim3(g.nblk, plan_run_samples(p)), 256, 0, s>>>(
+        w.d_root_site, w.d_root_expo, props, a.weights, site_lnl, static_cast<T *>(w.d_coef), w.d_cexp, w.d_block_lnl,
+        p->K, n, g.Npad);
     p->launches += 1;
     cudaError_t e = cudaSuccess;
     if (lnl) {
@@ -538,10 +511,10 @@ int wide_create(tt_plan *p) {
 namespace {
 
 struct SlabBuffers {
-  size_t part, expo, prod, root_site, root_expo, log2L, block, gpart, rootpart, site;
+  size_t part, expo, prod, root_site, root_expo, coef, cexp, block, gpart, rootpart, site;
   size_t total() const {
     size_t t = 0;
-    for (size_t x : {part, expo, prod, root_site, root_expo, log2L, block, gpart, rootpart, site})
+    for (size_t x : {part, expo, prod, root_site, root_expo, coef, cexp, block, gpart, rootpart, site})
       t += x ? std::max(x, size_t(16)) : 0;
     return t;
   }
@@ -559,7 +532,8 @@ SlabBuffers slab_buffers(const tt_plan *p, int n, bool slab) {
   x.prod = w.store_products ? b * I * K * 2 * SP * g.Npad * es : 0;
   x.root_site = b * K * g.Npad * sizeof(double);
   x.root_expo = b * K * g.Npad * sizeof(int);
-  x.log2L = b * g.Npad * sizeof(double);
+  x.coef = b * g.Npad * es;
+  x.cexp = b * g.Npad * sizeof(int);
   x.block = b * g.nblk * sizeof(double);
   x.gpart = b * p->B * g.cmax * K * SP * SP * es;
   x.rootpart = b * g.cmax * K * (SP + 1) * es;
@@ -571,7 +545,7 @@ void free_slab_buffers(tt_plan *p) {
   WideState &w = *p->wide;
   for (void **x : {reinterpret_cast<void **>(&w.d_part), reinterpret_cast<void **>(&w.d_expo),
                    reinterpret_cast<void **>(&w.d_prod), reinterpret_cast<void **>(&w.d_root_site),
-                   reinterpret_cast<void **>(&w.d_root_expo), reinterpret_cast<void **>(&w.d_log2L),
+                   reinterpret_cast<void **>(&w.d_root_expo), reinterpret_cast<void **>(&w.d_coef), reinterpret_cast<void **>(&w.d_cexp),
                    reinterpret_cast<void **>(&w.d_block_lnl), reinterpret_cast<void **>(&w.d_gpart),
                    reinterpret_cast<void **>(&w.d_rootpart), reinterpret_cast<void **>(&w.d_site)})
     if (*x) {
@@ -599,7 +573,8 @@ int wide_alloc_slab(tt_plan *p, int slab) {
   if (!rc && x.prod) rc = walloc(p, &w.d_prod, x.prod, "children's products");
   if (!rc) rc = walloc(p, &w.d_root_site, x.root_site, "root sums");
   if (!rc) rc = walloc(p, &w.d_root_expo, x.root_expo, "root exponents");
-  if (!rc) rc = walloc(p, &w.d_log2L, x.log2L, "site log-likelihoods");
+  if (!rc) rc = walloc(p, &w.d_coef, x.coef, "pattern coefficients");
+  if (!rc) rc = walloc(p, &w.d_cexp, x.cexp, "pattern exponents");
   if (!rc) rc = walloc(p, &w.d_block_lnl, x.block, "block sums");
   if (!rc) rc = walloc(p, &w.d_gpart, x.gpart, "gradient chunks");
   if (!rc) rc = walloc(p, &w.d_rootpart, x.rootpart, "root gradient chunks");
@@ -661,7 +636,7 @@ void wide_destroy(tt_plan *p) {
   WideState *w = p->wide;
   if (!w) return;
   void *bufs[] = {w->d_left, w->d_right, w->d_fwd, w->d_bwd, w->d_branch_lvn, w->d_part, w->d_expo, w->d_root_site, w->d_root_expo,
-                  w->d_log2L, w->d_block_lnl, w->d_gpart, w->d_rootpart, w->d_pgpart, w->d_prod, w->d_site,
+                  w->d_coef, w->d_cexp, w->d_block_lnl, w->d_gpart, w->d_rootpart, w->d_pgpart, w->d_prod, w->d_site,
                   w->d_pimg, w->d_pimg_f};
   for (void *x : bufs)
     if (x) cudaFree(x);

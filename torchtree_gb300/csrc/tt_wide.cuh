@@ -176,7 +176,9 @@ struct WideArgs {
   const double *weights;    // [N]
   double *root_site;        // [b][K][Npad]: sum_i pi_i L_root[k][i] at exponent root_expo
   int *root_expo;           // [b][K][Npad]
-  const double *log2L;      // [b][Npad] site log2-likelihoods (adjoint)
+  // the adjoint's per-pattern coefficient w_p 2^(E - log2 L_p) = coef 2^(E + cexp), [b][Npad]
+  const T *coef;
+  const int *cexp;
   T *gpart;                 // [b][B][nchunks][K][SP][SP]
   T *rootpart;              // [b][nchunks][K][SP + 1]
   // the children's products P_l x_l, P_r x_r of every internal node as the
@@ -212,6 +214,28 @@ template <typename T>
 __device__ __forceinline__ int wide_child_expo(const WideArgs<T> &a, int child, int b, int k, int n) {
   return child < a.tips ? 0 : a.expo[((size_t(b) * a.I + (child - a.tips)) * a.K + k) * a.Npad + n];
 }
+
+// Largest non-negative value of a column through shared memory: values as they
+// are in FP32, as integers of the same order in FP64 (an FP64 maximum is several
+// FP64 instructions; the integer pipe is free).
+template <typename T>
+struct MaxBits;
+template <>
+struct MaxBits<float> {
+  using type = float;
+  static __device__ __forceinline__ float of(float v) { return v; }
+  static __device__ __forceinline__ float zero() { return 0.0f; }
+  static __device__ __forceinline__ float larger(float a, float b) { return fmaxf(a, b); }
+  static __device__ __forceinline__ float value(float m) { return m; }
+};
+template <>
+struct MaxBits<double> {
+  using type = long long;  // negative values order below zero
+  static __device__ __forceinline__ long long of(double v) { return __double_as_longlong(v); }
+  static __device__ __forceinline__ long long zero() { return 0; }
+  static __device__ __forceinline__ long long larger(long long a, long long b) { return a > b ? a : b; }
+  static __device__ __forceinline__ double value(long long m) { return __longlong_as_double(m); }
+};
 
 // --------------------------------------------------------------- forward
 template <typename T, int SP, int PT>
@@ -292,18 +316,20 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
     return;
   }
   if (a.rescale) {
+    using M = MaxBits<T>;
+    typename M::type *mred = reinterpret_cast<typename M::type *>(red);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      T m = T(0);
+      typename M::type m = M::zero();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) m = fmax(m, al[i][q]);
-      red[ib * PT + pb * 4 + q] = double(m);
+      for (int i = 0; i < 4; ++i) m = M::larger(m, M::of(al[i][q]));
+      mred[ib * PT + pb * 4 + q] = m;
     }
     __syncthreads();
     if (tid < PT) {
-      double m = 0.0;
-      for (int u = 0; u < IB; ++u) m = fmax(m, red[u * PT + tid]);
-      ex[tid] = scale_exponent(T(m));
+      typename M::type m = M::zero();
+      for (int u = 0; u < IB; ++u) m = M::larger(m, mred[u * PT + tid]);
+      ex[tid] = scale_exponent(M::value(m));
     }
     __syncthreads();
 #pragma unroll
@@ -323,11 +349,51 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
   }
 }
 
-// Root combination: site log-likelihoods, log2 L_p for the adjoint and the
-// pattern-weighted per-block sums (FP64).  256 patterns per block.
+// Root combination: site log-likelihoods, the adjoint's coefficients and the
+// pattern-weighted per-block sums (FP64).  256 patterns per block.  The
+// coefficient w 2^(E - log2 L) is split once per pattern into coef = w 2^g and the
+// integer cexp, g in [0, 1) the fraction of -log2 L and cexp its floor, so that
+// the adjoint, which needs it per node and category, adds integers: FP64
+// instructions (an exponent difference, a floor, conversions; in FP64 plans an
+// exp2) take 16 cycles of an SM each.
+template <typename T>
 __global__ void wide_root_kernel(const double *root_site, const int *root_expo, const double *props,
-                                 const double *weights, double *site_lnl, double *log2L, double *block_lnl,
-                                 int K, int N, int Npad);
+                                 const double *weights, double *site_lnl, T *coef, int *cexp, double *block_lnl,
+                                 int K, int N, int Npad) {
+  __shared__ double part[8];
+  const int b = blockIdx.y, n = blockIdx.x * 256 + threadIdx.x;
+  double contrib = 0.0;
+  if (n < N) {
+    int emax = INT_MIN;
+    for (int k = 0; k < K; ++k) emax = max(emax, root_expo[(size_t(b) * K + k) * Npad + n]);
+    double s = 0.0;
+    for (int k = 0; k < K; ++k) {
+      const size_t o = (size_t(b) * K + k) * Npad + n;
+      s += props[size_t(b) * K + k] * ldexp(root_site[o], root_expo[o] - emax);
+    }
+    const double l2 = log2(s) + double(emax);
+    const double ll = l2 * 0.69314718055994530942;
+    if (site_lnl) site_lnl[size_t(b) * N + n] = ll;
+    // a likelihood of 0, inf or NaN (l2 not finite) has no exponent to split off: FP64 keeps
+    // w 2^-l2, FP32 a NaN
+    const bool finite = fabs(l2) < INFINITY;
+    const double fl = finite ? floor(-l2) : 0.0;
+    T c;
+    if constexpr (sizeof(T) == 8) c = weights[n] * exp2(-l2 - fl);
+    else c = finite ? float(weights[n]) * exp2f(float(-l2 - fl)) : __int_as_float(0x7fc00000);
+    coef[size_t(b) * Npad + n] = c;
+    cexp[size_t(b) * Npad + n] = int(fl);
+    contrib = weights[n] * ll;
+  }
+  contrib = warp_sum(contrib);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = contrib;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += part[w];
+    block_lnl[size_t(b) * gridDim.x + blockIdx.x] = t;
+  }
+}
 
 // --------------------------------------------------------------- adjoint
 // CTAs per SM the adjoint's registers are sized for: two for FP32 plans
@@ -421,15 +487,7 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
       er[tid] = Er;
       ep[tid] = Ep;
       T c = T(0);
-      if (n < a.N) {
-        const double dd = double(Ep + El + Er) - a.log2L[size_t(b) * a.Npad + n];
-        if constexpr (sizeof(T) == 8) {
-          c = a.weights[n] * exp2(dd);
-        } else {  // the fraction's power in FP32 (an FP64 exp2 costs thousands of FP64-pipe cycles per warp)
-          const double fl = floor(dd);
-          c = ldexpf(float(a.weights[n]) * exp2f(float(dd - fl)), int(fl));
-        }
-      }
+      if (n < a.N) c = ldexp(a.coef[size_t(b) * a.Npad + n], Ep + El + Er + a.cexp[size_t(b) * a.Npad + n]);
       cf[tid] = c;
     }
     // this thread's block of the outside partial of v
@@ -510,18 +568,20 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
           V4<T>::ld(us + i * XS + pb * 4, ua);
           outer4(o, pa, ua);
         }
+        using M = MaxBits<T>;
+        typename M::type *mred = reinterpret_cast<typename M::type *>(red);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          T m = T(0);
+          typename M::type m = M::zero();
 #pragma unroll
-          for (int s = 0; s < 4; ++s) m = fmax(m, o[s][q]);
-          red[ib * PT + pb * 4 + q] = double(m);
+          for (int s = 0; s < 4; ++s) m = M::larger(m, M::of(o[s][q]));
+          mred[ib * PT + pb * 4 + q] = m;
         }
         __syncthreads();
         if (tid < PT) {
-          double m = 0.0;
-          for (int u = 0; u < IB; ++u) m = fmax(m, red[u * PT + tid]);
-          const int e = scale_exponent(T(m));
+          typename M::type m = M::zero();
+          for (int u = 0; u < IB; ++u) m = M::larger(m, mred[u * PT + tid]);
+          const int e = scale_exponent(M::value(m));
           ex[tid] = e;
           const int n = n0 + tid;
           a.expo[((size_t(b) * a.I + (child - a.tips)) * a.K + k) * a.Npad + n] =

@@ -73,8 +73,8 @@ constexpr int kNR = 3;                    // raw slots
 constexpr int kMeta = kPT * 16 + 2 * kPT; // a tile's coefficients, exponents and tip codes
 constexpr int kOffRaw = kNS * kOpSlot;
 constexpr int kOffMeta = kOffRaw + kNR * kRawSlot;
-constexpr int kOffMraw = kOffMeta + 2 * kMeta;  // the next tile's weights and site log2 L (FP64) as copied
-constexpr int kOffRed = kOffMraw + 2 * kPT * 8; // float [4][128]
+constexpr int kOffMraw = kOffMeta + 2 * kMeta;  // the next tile's pattern coefficients and exponents as copied
+constexpr int kOffRed = kOffMraw + 2 * kPT * 4; // float [4][128]
 constexpr int kOffRoot = kOffRed + 4 * kPT * 4; // float [512] root partial sums
 constexpr int kTabRows = 64;               // code-table rows held in shared memory (tip children)
 constexpr int kOffTab = kOffRoot + kConv * 4;   // uint2 [kTabRows]: the rows of a 0 / 1 table as bit masks
@@ -178,9 +178,6 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
 }
 __device__ __forceinline__ void cp_async4(void *dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -432,16 +429,17 @@ __global__ void __launch_bounds__(tcb::kThreads, 1)
     __syncwarp();
   } else {
     // ------------------------------------------------------------ converter warps
-    double *mw = reinterpret_cast<double *>(smem + kOffMraw), *ml2 = mw + PT;
+    float *mc = reinterpret_cast<float *>(smem + kOffMraw);
+    int *me = reinterpret_cast<int *>(mc + PT);
     auto fetch_meta = [&](int t, TcbMeta m) {  // cp.async into buffer m (pattern tid; codes four per copy)
       const int n = t * PT + (tid & (PT - 1));
       if (tid < PT) {
         if (!is_root) cp_async4(&m.ep[tid], a.expo + size_t(vblk) * npad + n);
         if (int0) cp_async4(&m.el[tid], a.expo + size_t(lblk) * npad + n);
         if (int1) cp_async4(&m.er[tid], a.expo + size_t(rblk) * npad + n);
-        if (n < a.N) {  // padding patterns have neither (log2 L is written for n < N only)
-          cp_async8(&mw[tid], a.weights + n);
-          cp_async8(&ml2[tid], a.log2L + size_t(b) * npad + n);
+        if (n < a.N) {  // padding patterns have neither (they are written for n < N only)
+          cp_async4(&mc[tid], a.coef + size_t(b) * npad + n);
+          cp_async4(&me[tid], a.cexp + size_t(b) * npad + n);
         }
       } else if (tid < PT + 64) {
         const int sd = (tid - PT) >> 5, t4 = (tid - PT) & 31;
@@ -457,10 +455,7 @@ __global__ void __launch_bounds__(tcb::kThreads, 1)
         m.ep[tid] = Ep;
         m.el[tid] = El;
         m.er[tid] = Er;
-        // w 2^(E - log2 L): the exponent difference in FP64, its fraction's power in FP32 (an FP64
-        // exp2 costs thousands of cycles of this GPU's FP64 pipe per warp)
-        const double dd = double(Ep + El + Er) - ml2[tid], fl = floor(dd);
-        m.cf[tid] = n < a.N ? ldexpf(float(mw[tid]) * exp2f(float(dd - fl)), int(fl)) : 0.0f;
+        m.cf[tid] = n < a.N ? ldexpf(mc[tid], Ep + El + Er + me[tid]) : 0.0f;  // w 2^(E - log2 L)
       }
     };
     // a tip child's rows of the code table: as bit masks in shared memory when every entry is 0 or 1
