@@ -378,6 +378,76 @@ int tt_constant_coalescent(tt_time_tree *tree, int32_t batch,
                            double *grad_theta, void *stream);
 
 /*
+ * Per-call model set-up in one launch each (device double pointers):
+ *   tt_weibull_rates / tt_gamma_rates: mean-one category rates [b][K] of a
+ *     discretised site model (site_model.py:173-195, 237-247; Gamma as in
+ *     tt_gamma_quantiles) from the shapes [b], their derivatives with respect
+ *     to the shape [b][K] and the category weights 1/K [K]; K <= 32.
+ *   tt_rates_backward: dlnL/dshape [b] from dlnL/drates [b][K].
+ *   tt_exchangeability_q: unnormalised reversible rate matrix [b][S][S],
+ *     Q_ij = R_ij pi_j (abstract.py:49-57, nucleotide.py:238-374,
+ *     general.py:170-199, codon.py:57-77).  Without a map, params0 [b][S(S-1)/2] holds
+ *     the upper triangle of R row by row; with one (host int8
+ *     [2][S(S-1)/2]), each entry is the product of two of up to three scalar
+ *     parameters, params0..2 [b][1], by index (-1: 1).  param_counts[3] (host)
+ *     gives each array's parameters per sample.
+ *   tt_exchangeability_q_backward: gradients of the parameters and the
+ *     frequencies from dlnL/dQ (outputs may be NULL).
+ */
+int tt_weibull_rates(int32_t batch, int32_t category_count, const double *shape,
+                     double *rates, double *drates_dshape, double *weights,
+                     void *stream);
+int tt_gamma_rates(int32_t batch, int32_t category_count, const double *shape,
+                   double *rates, double *drates_dshape, double *weights,
+                   void *stream);
+int tt_rates_backward(int32_t batch, int32_t category_count,
+                      const double *grad_rates, const double *drates_dshape,
+                      double *grad_shape, void *stream);
+int tt_exchangeability_q(int32_t batch, int32_t state_count,
+                         const int32_t *param_counts, const double *params0,
+                         const double *params1, const double *params2,
+                         const int8_t *map, const double *frequencies, double *q,
+                         void *stream);
+int tt_exchangeability_q_backward(int32_t batch, int32_t state_count,
+                                  const int32_t *param_counts,
+                                  const double *params0, const double *params1,
+                                  const double *params2, const int8_t *map,
+                                  const double *frequencies, const double *grad_q,
+                                  double *grad_params0, double *grad_params1,
+                                  double *grad_params2, double *grad_frequencies,
+                                  void *stream);
+
+/*
+ * A whole evaluation of a reversible model and its gradient, one call each
+ * (TreeLikelihoodModel._call, tree_likelihood.py:313-356, and autograd through
+ * it): the rate matrix [b][S][S] is normalised (abstract.py:49-50) with its
+ * stationary frequencies [b][S], which are the root's too, and diagonalised;
+ * branch lengths [b][lengths_per_sample] fill nodes 0.. and the rest are zero
+ * (2T-3 free lengths of an unrooted tree, or all 2T-2); rates [b][K]; category
+ * weights with a row stride (0: one row for all samples).
+ *   tt_evaluate_workspace: doubles of `work` (kept from tt_evaluate to
+ *     tt_evaluate_gradient) and of `scratch`.
+ *   tt_evaluate: tt_reversible_eigen + tt_update_transition_matrices +
+ *     tt_log_likelihood; log_likelihood [b].
+ *   tt_evaluate_gradient: tt_gradient + tt_rate_matrix_gradient, chained to
+ *     the unnormalised rate matrix, each sample times grad_log_likelihood
+ *     (stride grad_stride); outputs may be NULL.
+ * The plan must still hold this evaluation's partials, as for tt_gradient.
+ */
+int tt_evaluate_workspace(const tt_plan *plan, int64_t *work, int64_t *scratch);
+int tt_evaluate(tt_plan *plan, const double *q, const double *frequencies,
+                const double *branch_lengths, int32_t lengths_per_sample,
+                const double *rates, const double *category_weights,
+                int64_t weights_stride, int32_t rescale, int32_t keep_partials,
+                double *work, double *log_likelihood, void *stream);
+int tt_evaluate_gradient(tt_plan *plan, double *work,
+                         const double *grad_log_likelihood, int64_t grad_stride,
+                         int32_t lengths_per_sample, double *scratch,
+                         double *grad_q, double *grad_frequencies,
+                         double *grad_branch_lengths, double *grad_rates,
+                         double *grad_weights, void *stream);
+
+/*
  * Self-test of the device-side failure path (no reference counterpart): one
  * kernel waits, with the bounded wait every staged kernel uses, on a barrier
  * that nothing completes, gives up after limit_ns (1 .. 1e10) and records

@@ -63,6 +63,14 @@ SIGNATURES = {
     "tt_gamma_quantiles_host": (ctypes.c_int, [_I32, _I32, _P, _P, _P]),
     "tt_transition_matrices_expm": (ctypes.c_int, [_I32, _I32, _I32, _I32, _P, _P, _P, _P, _P]),
     "tt_transition_matrices_expm_adjoint": (ctypes.c_int, [_I32, _I32, _I32, _I32, _P, _P, _P, _P, _P, _P, _P]),
+    "tt_weibull_rates": (ctypes.c_int, [_I32, _I32, _P, _P, _P, _P, _P]),
+    "tt_gamma_rates": (ctypes.c_int, [_I32, _I32, _P, _P, _P, _P, _P]),
+    "tt_rates_backward": (ctypes.c_int, [_I32, _I32, _P, _P, _P, _P]),
+    "tt_exchangeability_q": (ctypes.c_int, [_I32, _I32, _PI32] + [_P] * 7),
+    "tt_exchangeability_q_backward": (ctypes.c_int, [_I32, _I32, _PI32] + [_P] * 11),
+    "tt_evaluate_workspace": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)]),
+    "tt_evaluate": (ctypes.c_int, [_P] * 4 + [_I32, _P, _P, ctypes.c_int64, _I32, _I32, _P, _P, _P]),
+    "tt_evaluate_gradient": (ctypes.c_int, [_P, _P, _P, ctypes.c_int64, _I32] + [_P] * 7),
     "tt_plans_log_likelihood": (ctypes.c_int, [_I32, _P, _P, _P, _I32, _I32, _P, _P]),
     "tt_plans_gradient": (ctypes.c_int, [_I32, _P, _P, _P, _P, _P, _P]),
     "tt_log_likelihood_static": (ctypes.c_int, [_I32, _PI32, _I32, _I32, _I32, _I32, _P, _P, _I32, _P, _P, _P,

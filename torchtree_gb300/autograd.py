@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import torch
 
-from .substitution import device_eigen, eigen_of_normalised
+from .substitution import device_eigen, eigen_of_normalised, normalise
 
 
 def _scale(g: torch.Tensor, x: torch.Tensor, like: torch.Tensor) -> torch.Tensor:
@@ -86,6 +86,51 @@ class RateMatrixLikelihood(torch.autograd.Function):
         g = g.to(torch.float64)
         return (_scale(g, dq, ctx.q_like), None, _scale(g, dt, bls), _scale(g, dr, rates),
                 _scale(g, dc, props), _scale(g, dpi, freqs), None, None)
+
+
+class EvaluateLikelihood(torch.autograd.Function):
+    """``RateMatrixLikelihood`` from the unnormalised rate matrix and the free
+    branch lengths (zero for the nodes beyond), with the frequencies as the
+    stationary and the root distribution: the normalisation, the padding and
+    their backward are part of the engine's two calls (``tt_evaluate``,
+    ``tt_evaluate_gradient``).  Contiguous CUDA FP64 tensors."""
+
+    @staticmethod
+    def forward(ctx, lengths, q, freqs, rates, props, engine, rescale):
+        keep = any(ctx.needs_input_grad[:5])
+        lnl, work = engine.evaluate(q, freqs, lengths, rates, props, rescale, keep)
+        if keep:
+            ctx.engine = engine
+            ctx.token = engine.token
+            ctx.rescale = rescale
+            ctx.length_count = lengths.shape[1]
+            ctx.save_for_backward(work, q, freqs, rates, props)
+        return lnl
+
+    @staticmethod
+    def backward(ctx, g):
+        work, q, freqs, rates, props = ctx.saved_tensors
+        eng = ctx.engine
+        if eng.token != ctx.token:  # a later forward overwrote the stored partials
+            lam, u, w, bl, r, p, f = eng.evaluation_parts(work)
+            eng.set_eigen(lam, u, w, bl, r)
+            eng.log_likelihood(p, f, rescale=ctx.rescale, keep_partials=True)
+        if not torch.is_grad_enabled():
+            return (*eng.evaluate_gradient(work, g, ctx.length_count, ctx.needs_input_grad[:5]), None, None)
+        # create_graph: the graph that the separate steps would leave (through g and the normalisation)
+        lam, u, w, bl, r, p, f = eng.evaluation_parts(work)
+        _, dpi, dc = eng.gradient(p, f)
+        dq, dt, dr = eng.rate_matrix_gradient(lam, u, w, bl, r)
+        with torch.enable_grad():
+            ins = [t for t in (q, freqs) if t.requires_grad]
+            via = iter(torch.autograd.grad(normalise(q, freqs), ins, _scale(g, dq, q), create_graph=True)
+                       if ins else ())
+        gq = next(via) if q.requires_grad else None
+        gf = _scale(g, dpi, freqs)
+        if freqs.requires_grad:
+            gf = gf + next(via)
+        return (_scale(g, dt[:, :ctx.length_count], bl), gq, gf, _scale(g, dr, rates), _scale(g, dc, props), None,
+                None)
 
 
 class MatrixLikelihood(torch.autograd.Function):

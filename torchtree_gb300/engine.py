@@ -8,6 +8,7 @@ contiguous CUDA float64 tensors.
 from __future__ import annotations
 
 import ctypes
+import math
 
 import numpy as np
 import torch
@@ -62,6 +63,7 @@ class LikelihoodEngine:
             check(self.lib.tt_plan_set_tips(self._plan, ptr(codes), ptr(table), int(table.shape[0]),
                                             ptr(w)))
         self.token = 0  # bumped by every forward that keeps partials
+        self._eval_sizes = None  # doubles of evaluate's work and scratch buffers
 
     # ---------------------------------------------------------------- lifetime
     def close(self):
@@ -167,6 +169,54 @@ class LikelihoodEngine:
         check(self.lib.tt_transition_matrices_gradient(self._plan, *map(ptr, args), ptr(dlam), ptr(du),
                                                        ptr(dw), ptr(dt), ptr(dr), _stream()))
         return dlam, du, dw, dt, dr
+
+    def evaluate(self, q, freqs, lengths, rates, props, rescale: bool, keep_partials: bool):
+        """``(lnL [b], work)`` of an unnormalised reversible ``q [b,S,S]`` in one
+        call (``tt_evaluate``): ``freqs [b,S]`` are its stationary and the root
+        frequencies, ``lengths [b,n]`` nodes 0 .. n-1 (zero beyond), ``rates`` and
+        ``props`` ``[b,K]``; contiguous CUDA FP64 tensors (``props`` may repeat one
+        row).  ``work`` carries the evaluation to ``evaluate_gradient``."""
+        if self._eval_sizes is None:
+            n = (ctypes.c_int64(), ctypes.c_int64())
+            check(self.lib.tt_evaluate_workspace(self._plan, *map(ctypes.byref, n)))
+            self._eval_sizes = (int(n[0].value), int(n[1].value))
+        lnl = torch.empty(self.batch, dtype=torch.float64, device=self.device)
+        work = torch.empty(self._eval_sizes[0], dtype=torch.float64, device=self.device)
+        check(self.lib.tt_evaluate(self._plan, q.data_ptr(), freqs.data_ptr(), lengths.data_ptr(), lengths.shape[1],
+                                   rates.data_ptr(), props.data_ptr(), props.stride(0), rescale, keep_partials,
+                                   work.data_ptr(), lnl.data_ptr(),
+                                   torch.cuda.current_stream(self.device).cuda_stream))
+        if keep_partials:
+            self.token += 1
+        return lnl, work
+
+    def evaluation_parts(self, work):
+        """Views of an evaluation's ``(lam, u, w, node lengths, rates, props, freqs)``."""
+        b, S, K, B = self.batch, self.state_count, self.category_count, self.branch_count
+        shapes = ((b, S, S), (b, S, S), (b, S, S), (b, S), (b, S), (b, B), (b, K), (b, K))
+        parts, off = [], 0
+        for s in shapes:
+            n = math.prod(s)
+            parts.append(work[off:off + n].view(s))
+            off += n
+        _, u, w, lam, freqs, bl, rates, props = parts
+        return lam, u, w, bl, rates, props, freqs
+
+    def evaluate_gradient(self, work, grad, length_count: int, needs):
+        """Gradients of ``evaluate``'s ``(lengths, q, freqs, rates, props)``, each
+        sample times ``grad [b]``; None where ``needs`` is false."""
+        b, S, K = self.batch, self.state_count, self.category_count
+        kw = dict(dtype=torch.float64, device=self.device)
+        shapes = ((b, length_count), (b, S, S), (b, S), (b, K), (b, K))
+        dbl, dq, dpi, dr, dc = out = [torch.empty(s, **kw) if need else None for s, need in zip(shapes, needs)]
+        scratch = torch.empty(self._eval_sizes[1], **kw)
+        p = [None if t is None else t.data_ptr() for t in (dq, dpi, dbl, dr, dc)]
+        check(self.lib.tt_evaluate_gradient(self._plan, work.data_ptr(), grad.data_ptr(), grad.stride(0),
+                                            length_count, scratch.data_ptr(), *p,
+                                            torch.cuda.current_stream(self.device).cuda_stream))
+        if self.state_count != 4 or self.precision == "f32":  # these adjoints consume the stored partials
+            self.token += 1
+        return out
 
     def rate_matrix_gradient(self, lam, u, w, branch_lengths, rates):
         """Chain dlnL/dP to the rate matrix: ``(dQ [b,S,S], dt [b,B], dr [b,K])``."""

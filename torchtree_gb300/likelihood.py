@@ -17,7 +17,8 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from .autograd import EigenLikelihood, GeneralRateMatrixLikelihood, MatrixLikelihood, RateMatrixLikelihood
+from .autograd import (EigenLikelihood, EvaluateLikelihood, GeneralRateMatrixLikelihood, MatrixLikelihood,
+                       RateMatrixLikelihood)
 from .engine import LikelihoodEngine
 from .patterns import CompressedAlignment
 from .substitution import normalise
@@ -55,9 +56,37 @@ class PhyloLikelihood:
         ``clock_rates``; ``q_unnorm [b,S,S]`` reversible rate matrix;
         ``frequencies [b,S]``; ``rates``/``props`` ``[b,K]``.
         """
+        if clock_rates is None and self._one_call(branch_lengths, q_unnorm, frequencies, rates, props):
+            def run(rescale):
+                return EvaluateLikelihood.apply(branch_lengths, q_unnorm, frequencies, rates, props, self.engine,
+                                                rescale)
+
+            if self.rescale:
+                return run(True)
+            lnl = run(False)
+            if torch.isinf(lnl).any():
+                self.rescale = True
+                lnl = run(True)
+            return lnl
         bls = self.node_branch_lengths(branch_lengths, clock_rates)
         return self.evaluate_rate_matrix(normalise(q_unnorm, frequencies), frequencies, bls, rates, props,
                                          frequencies)
+
+    def _one_call(self, branch_lengths, q, frequencies, rates, props) -> bool:
+        """Whether the inputs are what the engine's one-call evaluation takes as they
+        are: FP64 on its device, one row per sample, contiguous (the weights may
+        repeat one row)."""
+        if (type(self).node_branch_lengths is not PhyloLikelihood.node_branch_lengths
+                or type(self).evaluate_rate_matrix is not PhyloLikelihood.evaluate_rate_matrix):
+            return False
+        b, S, K = self.batch, self.state_count, self.category_count
+        for t, shape in ((branch_lengths, (b, self.engine.branch_count - 1)), (q, (b, S, S)), (frequencies, (b, S)),
+                         (rates, (b, K)), (props, (b, K))):
+            if t.dtype != torch.float64 or t.device != self.device or t.shape != shape:
+                return False
+        return (branch_lengths.is_contiguous() and q.is_contiguous() and frequencies.is_contiguous()
+                and rates.is_contiguous() and (K == 1 or props.stride(1) == 1)
+                and self.device.index == torch.cuda.current_device())
 
     def evaluate_rate_matrix(self, q, pi_q, bls, rates, props, frequencies):
         """lnL from the normalised rate matrix; gradients reach ``q`` as dlnL/dQ."""

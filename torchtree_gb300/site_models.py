@@ -13,6 +13,8 @@ from __future__ import annotations
 
 import torch
 
+from . import fused
+
 
 def _quantiles(k: int, dtype, device):
     return (2.0 * torch.arange(k, dtype=dtype, device=device) + 1.0) / (2.0 * k)
@@ -31,8 +33,25 @@ def _finish(rates, categories, invariant, mu):
     return rates, probs.expand(rates.shape)
 
 
+def _one_launch(shape, categories, invariant, mu) -> bool:
+    """The plain model of FP64 device shapes: rates, weights and shape derivative from one kernel."""
+    return (invariant is None and mu is None and 1 <= categories <= 32 and shape.dim() > 0 and shape.shape[-1] == 1
+            and fused.plain_cuda(shape))
+
+
+def _fused_rates(shape, categories, kind, compose):
+    rates, probs = fused.CategoryRates.apply(shape, categories, kind, lambda s: compose(s, categories)[0])
+    return rates, probs.expand(rates.shape)
+
+
 def weibull_rates(shape: torch.Tensor, categories: int, invariant=None, mu=None):
     """``shape [...,1]`` -> ``(rates [...,K'], probabilities [...,K'])``."""
+    if _one_launch(shape, categories, invariant, mu):
+        return _fused_rates(shape, categories, "tt_weibull_rates", _weibull)
+    return _weibull(shape, categories, invariant, mu)
+
+
+def _weibull(shape, categories, invariant=None, mu=None):
     q = _quantiles(categories, shape.dtype, shape.device)
     rates = torch.pow(-torch.log(1.0 - q), 1.0 / shape)
     return _finish(rates, categories, invariant, mu)
@@ -77,6 +96,12 @@ class _GammaQuantile(torch.autograd.Function):
 
 def gamma_rates(shape: torch.Tensor, categories: int, invariant=None, mu=None):
     """Discretised Gamma rates; ``shape [...,1]`` (not in the reference)."""
+    if _one_launch(shape, categories, invariant, mu):
+        return _fused_rates(shape, categories, "tt_gamma_rates", _gamma)
+    return _gamma(shape, categories, invariant, mu)
+
+
+def _gamma(shape, categories, invariant=None, mu=None):
     rates = _GammaQuantile.apply(shape, categories)
     return _finish(rates, categories, invariant, mu)
 

@@ -14,9 +14,13 @@ keeps the autograd graph.
 """
 from __future__ import annotations
 
+import functools
 import itertools
 
+import numpy as np
 import torch
+
+from . import fused
 
 
 def normalise(q: torch.Tensor, pi: torch.Tensor) -> torch.Tensor:
@@ -82,29 +86,64 @@ def symmetric_from_upper(rates: torch.Tensor, state_count: int) -> torch.Tensor:
     return r + r.transpose(-1, -2)
 
 
+def _one_launch(pi, state_count, *params, scalars=False) -> bool:
+    """One row of parameters (of one scalar each, where mapped) and frequencies per
+    sample, FP64 on the device: the rate matrix from one kernel."""
+    return (2 <= state_count <= 64 and pi.dim() == 2 and pi.shape[1] == state_count
+            and all(t.dim() == 2 and t.shape[0] == pi.shape[0] and (not scalars or t.shape[1] == 1) for t in params)
+            and fused.plain_cuda(pi, *params))
+
+
+# upper-triangle entries AC, AG, AT, CG, CT, GT as parameter indices (kappa, or -1: 1)
+_HKY_INDEX = np.array([[-1, 0, -1, -1, 0, -1], [-1] * 6], dtype=np.int8)
+
+
+@functools.lru_cache(maxsize=8)
+def _mg94_index(table):
+    """``(map, sense codons)``: each pair's exchangeability as the product of
+    (alpha, beta, kappa) entries, kappa for transitions times alpha or beta."""
+    ts, syn, nonsyn, m = codon_pair_masks(table)
+    ts, syn, nonsyn = (t.numpy() for t in (ts, syn, nonsyn))
+    return np.stack((np.where(ts, 2, -1), np.where(syn, 0, np.where(nonsyn, 1, -1)))).astype(np.int8), m
+
+
 def gtr_q(rates: torch.Tensor, pi: torch.Tensor) -> torch.Tensor:
     """GTR (torchtree/evolution/substitution_model/nucleotide.py:328-374).
 
     ``rates [...,6]`` ordered AC, AG, AT, CG, CT, GT; ``pi [...,4]``.
     """
+    if _one_launch(pi, 4, rates) and rates.shape[1] == 6:
+        return general_symmetric_q(rates, pi, 4)
     batch = torch.broadcast_shapes(rates.shape[:-1], pi.shape[:-1])
     rates = rates.expand(batch + (6,))
     pi = pi.expand(batch + (4,))
-    return exchangeability_q(symmetric_from_upper(rates, 4), pi)
+    return _general(rates, pi, 4)
 
 
 def hky_q(kappa: torch.Tensor, pi: torch.Tensor) -> torch.Tensor:
     """HKY (nucleotide.py:238-264): transitions A<->G, C<->T scaled by kappa."""
+    if _one_launch(pi, 4, kappa, scalars=True):
+        return fused.ExchangeabilityQ.apply(pi, _HKY_INDEX, _hky, kappa)
+    return _hky(kappa, pi)
+
+
+def _hky(kappa, pi):
     batch = torch.broadcast_shapes(kappa.shape[:-1], pi.shape[:-1])
     kappa = kappa.expand(batch + (1,))
     one = torch.ones_like(kappa)
     # upper triangle AC, AG, AT, CG, CT, GT
     rates = torch.cat([one, kappa, one, one, kappa, one], -1)
-    return gtr_q(rates, pi)
+    return _general(rates, pi, 4)
 
 
 def general_symmetric_q(rates: torch.Tensor, pi: torch.Tensor, state_count: int) -> torch.Tensor:
     """M-state symmetric model from its M(M-1)/2 exchangeabilities (general.py:267-281)."""
+    if _one_launch(pi, state_count, rates) and rates.shape[1] == state_count * (state_count - 1) // 2:
+        return fused.ExchangeabilityQ.apply(pi, None, lambda r, f: _general(r, f, state_count), rates)
+    return _general(rates, pi, state_count)
+
+
+def _general(rates, pi, state_count):
     batch = torch.broadcast_shapes(rates.shape[:-1], pi.shape[:-1])
     rates = rates.expand(batch + rates.shape[-1:])
     pi = pi.expand(batch + (state_count,))
@@ -116,6 +155,12 @@ UNIVERSAL_CODE = "KNKNTTTTRSRSIIMIQHQHPPPPRRRRLLLLEDEDAAAAGGGGVVVV*Y*YSSSS*CWCLF
 
 def codon_pair_masks(table: str = UNIVERSAL_CODE):
     """MG94 pair classes over sense-codon pairs in combinations order (codon.py:33-55)."""
+    ts, syn, nonsyn, m = _codon_pair_masks(table)
+    return ts.clone(), syn.clone(), nonsyn.clone(), m
+
+
+@functools.lru_cache(maxsize=8)
+def _codon_pair_masks(table):
     trip = ["".join(t) for t in itertools.product("ACGT", repeat=3)]
     sense = [i for i, a in enumerate(table[:64]) if a != "*"]
     m = len(sense)
@@ -136,10 +181,19 @@ def codon_pair_masks(table: str = UNIVERSAL_CODE):
 def mg94_q(alpha, beta, kappa, pi, table: str = UNIVERSAL_CODE) -> torch.Tensor:
     """MG94 as torchtree computes it (codon.py:57-77): exchangeability
     kappa^ts alpha^syn beta^nonsyn; pairs differing at 2-3 positions get 1."""
+    if _one_launch(pi, pi.shape[-1], alpha, beta, kappa, scalars=True):
+        index, m = _mg94_index(table)
+        if m == pi.shape[-1]:
+            return fused.ExchangeabilityQ.apply(pi, index, lambda a, b, k, f: _mg94(a, b, k, f, table), alpha, beta,
+                                                kappa)
+    return _mg94(alpha, beta, kappa, pi, table)
+
+
+def _mg94(alpha, beta, kappa, pi, table):
     ts, syn, nonsyn, m = codon_pair_masks(table)
     dev = pi.device
     ts, syn, nonsyn = ts.to(dev), syn.to(dev), nonsyn.to(dev)
     kappa, alpha, beta = torch.broadcast_tensors(kappa, alpha, beta)
     one = torch.ones_like(kappa)
     off = torch.where(ts, kappa, one) * torch.where(syn, alpha, one) * torch.where(nonsyn, beta, one)
-    return general_symmetric_q(off, pi, m)
+    return _general(off, pi, m)
