@@ -12,6 +12,7 @@
 #include "../../include/torchtree_gb300.h"
 #include "tt_plan.h"
 #include "tt_wide.cuh"
+#include "tt_wide_col.cuh"
 #include "tt_wide_tc.cuh"
 #include "tt_wide_tc_bwd.cuh"
 
@@ -267,7 +268,23 @@ struct Wide {
           continue;
         }
       }
-      const dim3 grid(g.ntiles_f, w.fwd_off[lv + 1] - w.fwd_off[lv], plan_run_samples(p) * p->K);
+      const int nodes = w.fwd_off[lv + 1] - w.fwd_off[lv];
+      if constexpr (SP == kColStates) {
+        if (lv + 2 < w.fwd_off.size()) {  // every level but the root's: about eight waves of three CTAs per SM
+          constexpr int tile = kColThreads * kColPatterns<T>;
+          WideArgs<T> ac = a;
+          ac.ntiles = (g.Npad + tile - 1) / tile;
+          const int chunks = tc_level_chunks(nodes, p->batch * p->K, ac.ntiles, ac.ntiles, 8 * 152 * 3);
+          ac.tiles_per_chunk = (ac.ntiles + chunks - 1) / chunks;
+          const size_t sm = col_fwd_smem<T>(p->C);
+          const cudaError_t e = kernel_smem(wide_col_forward_kernel<T>, sm, true);
+          if (e != cudaSuccess) return e;
+          wide_col_forward_kernel<T><<<dim3(chunks, nodes, plan_run_samples(p) * p->K), kColThreads, sm, s>>>(ac, p->C);
+          p->launches += 1;
+          continue;
+        }
+      }
+      const dim3 grid(g.ntiles_f, nodes, plan_run_samples(p) * p->K);
       wide_forward_kernel<T, SP, PTF><<<grid, NT, smem, s>>>(a);
       p->launches += 1;
     }
