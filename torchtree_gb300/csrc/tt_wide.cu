@@ -67,6 +67,10 @@ struct WideState {
   void *d_gpart = nullptr;
   void *d_rootpart = nullptr;
   double *d_pgpart = nullptr;
+  uint8_t *d_tip_row = nullptr;  // [256] code -> row of the staged P^T (WideArgs::tip_row)
+  void *d_tip_amb = nullptr;     // [kTipRows][SP] the ambiguous code vectors
+  int tip_ambs = 0;
+  bool tip_rows_ok = false;      // at most kTipRows ambiguous codes
   void *d_prod = nullptr;  // FP32: the children's products of the post-order, read by the adjoint
 };
 
@@ -86,8 +90,10 @@ WideGeo wide_geo(const tt_plan *p, int n) {
   const WideState &w = *p->wide;
   WideGeo g;
   g.Npad = (n + 127) / 128 * 128;
-  g.ntiles_f = g.Npad / w.PTf;
-  g.ntiles_b = g.Npad / w.PTb;
+  // FP64 plans skip the tiles past the last pattern
+  const int last = p->precision == TT_PRECISION_F64 ? n : g.Npad;
+  g.ntiles_f = (last + w.PTf - 1) / w.PTf;
+  g.ntiles_b = (last + w.PTb - 1) / w.PTb;
   g.nblk = (n + 255) / 256;
   const int want = (2 * 152 + p->batch * p->K - 1) / (p->batch * p->K);
   g.cmax = std::max(1, std::min({want, g.ntiles_b, 64}));
@@ -221,6 +227,9 @@ struct Wide {
     a.right = w.d_right;
     a.codes = p->d_codes + p0;
     a.table = static_cast<const T *>(p->d_table);
+    a.tip_row = w.tip_rows_ok ? w.d_tip_row : nullptr;
+    a.tip_amb = static_cast<const T *>(w.d_tip_amb);
+    a.tip_ambs = w.tip_ambs;
     a.pmat = static_cast<const T *>(p->d_pmat);
     a.part = static_cast<T *>(w.d_part);
     a.expo = w.d_expo;
@@ -490,6 +499,8 @@ int wide_create(tt_plan *p) {
   if (!rc) rc = walloc(p, &w->d_branch_lvn, size_t(p->B) * sizeof(int), "branch levels");
   if (!rc) rc = walloc(p, &p->d_codes, size_t(T) * p->code_stride, "tip codes");
   if (!rc) rc = walloc(p, &p->d_table, 256 * SP * es, "code table");
+  if (!rc) rc = walloc(p, &w->d_tip_row, 256, "tip rows");
+  if (!rc) rc = walloc(p, &w->d_tip_amb, kTipRows * SP * es, "ambiguous code vectors");
   if (!rc) rc = walloc(p, &p->d_weights, size_t(p->N) * sizeof(double), "weights");
   if (!rc) rc = walloc(p, &p->d_pmat, b * p->B * K * SP * SP * es, "transition matrices");
   {  // FP32 codon plans keep the children's products for the adjoint (TT_WIDE_STORE_PRODUCTS=0
@@ -654,7 +665,7 @@ void wide_destroy(tt_plan *p) {
   if (!w) return;
   void *bufs[] = {w->d_left, w->d_right, w->d_fwd, w->d_bwd, w->d_branch_lvn, w->d_part, w->d_expo, w->d_root_site, w->d_root_expo,
                   w->d_coef, w->d_cexp, w->d_block_lnl, w->d_gpart, w->d_rootpart, w->d_pgpart, w->d_prod, w->d_site,
-                  w->d_pimg, w->d_pimg_f};
+                  w->d_pimg, w->d_pimg_f, w->d_tip_row, w->d_tip_amb};
   for (void *x : bufs)
     if (x) cudaFree(x);
   delete w;
@@ -675,7 +686,34 @@ int wide_set_tips(tt_plan *p, const uint8_t *codes, const double *code_table, in
         std::memcpy(&table[(size_t(c) * SP + j) * 8], &v, 8);
       }
     }
+  // codes whose product is a row of the staged P^T: unit vectors, and the first kTipRows others
+  WideState &w = *p->wide;
+  std::vector<uint8_t> rows(256, 0);
+  std::vector<unsigned char> amb(size_t(kTipRows) * SP * p->elem, 0);
+  int ambs = 0;
+  bool ok = true;
+  for (int c = 0; c < code_count; ++c) {
+    int ones = 0, zeros = 0, s = 0;
+    for (int j = 0; j < p->S; ++j) {
+      const double v = code_table[size_t(c) * p->S + j];
+      if (v == 1.0) s = j, ++ones;
+      else zeros += v == 0.0;
+    }
+    if (ones == 1 && zeros == p->S - 1) {
+      rows[c] = uint8_t(s);
+    } else if (ambs < kTipRows) {
+      rows[c] = uint8_t(SP + ambs);
+      std::memcpy(&amb[size_t(ambs) * SP * p->elem], &table[size_t(c) * SP * p->elem], SP * p->elem);
+      ++ambs;
+    } else {
+      ok = false;
+    }
+  }
+  w.tip_ambs = ambs;
+  w.tip_rows_ok = ok;
   cudaError_t e = cudaMemset(p->d_codes, 0, size_t(p->T) * p->code_stride);
+  if (e == cudaSuccess) e = cudaMemcpy(w.d_tip_row, rows.data(), rows.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(w.d_tip_amb, amb.data(), amb.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy2D(p->d_codes, p->code_stride, codes, p->N, p->N, p->T, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(p->d_table, table.data(), table.size(), cudaMemcpyHostToDevice);

@@ -47,18 +47,26 @@ struct WideCfg {
   static_assert(NT >= IB * IB || (IB * IB) % NT == 0, "GEMM3 blocks must divide evenly");
 };
 
+// Tip children without a product: the product of P with a tip's unit vector is
+// a column of P, which the staged P^T holds as a row; the products with up to
+// kTipRows other code vectors (gaps, ambiguous states) are formed once per CTA,
+// term by term as the product, and staged as further rows.  Either way the bits
+// are the product's.  WideArgs::tip_row maps a code to its row (NULL: a plan with
+// more such codes, whose tips take the product).
+constexpr int kTipRows = 4;
+
 // shared-memory bytes of the two kernels
 template <typename T, int SP, int PT>
 constexpr size_t wide_fwd_smem() {
   using C = WideCfg<T, SP, PT>;
-  return sizeof(T) * (2 * SP * SP + 2 * SP * C::XS) + sizeof(double) * C::IB * PT + sizeof(int) * PT;
+  return sizeof(T) * (2 * (SP + kTipRows) * SP + 2 * SP * C::XS) + sizeof(double) * C::IB * PT + sizeof(int) * PT;
 }
 // (stored_products: the adjoint reads the post-order's products and keeps no P^T)
 template <typename T, int SP, int PT>
 constexpr size_t wide_bwd_smem(bool stored_products = false) {
   using C = WideCfg<T, SP, PT>;
-  return sizeof(T) * ((stored_products ? 2 : 4) * SP * SP + 3 * SP * C::XS + PT) + sizeof(double) * C::IB * PT +
-         sizeof(int) * 4 * PT;
+  return sizeof(T) * (2 * SP * SP + (stored_products ? 0 : 2 * (SP + kTipRows) * SP) + 3 * SP * C::XS + PT) +
+         sizeof(double) * C::IB * PT + sizeof(int) * 4 * PT;
 }
 
 template <int IB>
@@ -168,6 +176,9 @@ struct WideArgs {
   const int *left, *right;  // [I] children of internal node v - tips
   const uint8_t *codes;     // [tips][code_stride]
   const T *table;           // [C][SP]
+  const uint8_t *tip_row;   // [256] row of the staged P^T that is the code's product, or NULL
+  const T *tip_amb;         // [kTipRows][SP] code vectors of rows SP .. SP + tip_ambs - 1
+  int tip_ambs;
   const T *pmat;            // [b][B][K][SP][SP]
   T *part;                  // [b][I][K][SP][Npad]
   int *expo;                // [b][I][K][Npad]
@@ -237,14 +248,58 @@ struct MaxBits<double> {
   static __device__ __forceinline__ double value(long long m) { return __longlong_as_double(m); }
 };
 
+// rows SP .. of a tip child's staged P^T ([j][perm i]): its products with the ambiguous code vectors
+template <typename T, int SP, int NT>
+__device__ __forceinline__ void wide_tip_rows(const WideArgs<T> &a, T *plt) {
+  for (int e = threadIdx.x; e < a.tip_ambs * SP; e += NT) {
+    const int m = e / SP, i = e - m * SP;
+    T acc = T(0);
+#pragma unroll 4
+    for (int j = 0; j < SP; ++j) acc = fma(plt[j * SP + i], a.tip_amb[m * SP + j], acc);
+    plt[(SP + m) * SP + i] = acc;
+  }
+}
+
+// the thread's 4 rows x 4 patterns of a tip child's product
+template <typename T, int SP>
+__device__ __forceinline__ void wide_tip_product(const WideArgs<T> &a, T (&acc)[4][4], const T *plt, int child, int n,
+                                                 int ib) {
+  const uint32_t codes = *reinterpret_cast<const uint32_t *>(a.codes + size_t(child) * a.code_stride + n);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    T col[4];
+    V4<T>::ld(plt + int(__ldg(a.tip_row + ((codes >> (8 * q)) & 0xff))) * SP + ib * 4, col);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i][q] = col[i];
+  }
+}
+
+// ... of an internal child's (or any staged vector's)
+template <typename T, int SP, int XS>
+__device__ __forceinline__ void wide_product(T (&acc)[4][4], const T *plt, const T *xs, int S, int ib, int pb) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[i][q] = T(0);
+  const int J = sizeof(T) == 8 ? S : SP;  // FP64: no work for the padding states
+#pragma unroll 4
+  for (int j = 0; j < J; ++j) {
+    T pa[4], xa[4];
+    V4<T>::ld(plt + j * SP + ib * 4, pa);
+    V4<T>::ld(xs + j * XS + pb * 4, xa);
+    outer4(acc, pa, xa);
+  }
+}
+
 // --------------------------------------------------------------- forward
 template <typename T, int SP, int PT>
 __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(const WideArgs<T> a) {
   using C = WideCfg<T, SP, PT>;
   constexpr int IB = C::IB, NT = C::NT, XS = C::XS;
   extern __shared__ __align__(128) unsigned char smem[];
-  T *plt = reinterpret_cast<T *>(smem);                          // [2][SP j][SP perm i]
-  T *xs = plt + 2 * SP * SP;                                      // [2][SP][XS]
+  constexpr int PS = (SP + kTipRows) * SP;                        // one side's staged matrix and tip rows
+  T *plt = reinterpret_cast<T *>(smem);                          // [2][SP j + tip rows][SP perm i]
+  T *xs = plt + 2 * PS;                                           // [2][SP][XS]
   double *red = reinterpret_cast<double *>(xs + 2 * SP * XS);     // [IB][PT]
   int *ex = reinterpret_cast<int *>(red + IB * PT);               // [PT]
   const int tid = threadIdx.x, ib = tid % IB, pb = tid / IB;
@@ -256,27 +311,23 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
 
   for (int e = tid; e < 2 * SP * SP; e += NT) {
     const int c = e / (SP * SP), ij = e - c * SP * SP, i = ij / SP, j = ij - i * SP;
-    plt[c * SP * SP + j * SP + wperm<IB>(i)] = a.pmat[((size_t(b) * a.B + (c ? r : l)) * a.K + k) * SP * SP + ij];
+    plt[c * PS + j * SP + wperm<IB>(i)] = a.pmat[((size_t(b) * a.B + (c ? r : l)) * a.K + k) * SP * SP + ij];
   }
-  wide_stage_child<T, SP, PT>(a, l, b, k, n0, xs);
-  wide_stage_child<T, SP, PT>(a, r, b, k, n0, xs + SP * XS);
+  const bool look_l = l < a.tips && a.tip_row, look_r = r < a.tips && a.tip_row;
+  if (!look_l) wide_stage_child<T, SP, PT>(a, l, b, k, n0, xs);
+  if (!look_r) wide_stage_child<T, SP, PT>(a, r, b, k, n0, xs + SP * XS);
   __syncthreads();
+  if ((look_l || look_r) && a.tip_ambs) {
+    if (look_l) wide_tip_rows<T, SP, NT>(a, plt);
+    if (look_r) wide_tip_rows<T, SP, NT>(a, plt + PS);
+    __syncthreads();
+  }
 
   T al[4][4], ar[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) al[i][q] = ar[i][q] = T(0);
-#pragma unroll 4
-  for (int j = 0; j < SP; ++j) {
-    T pa[4], pc[4], xa[4], xc[4];
-    V4<T>::ld(plt + j * SP + ib * 4, pa);
-    V4<T>::ld(plt + SP * SP + j * SP + ib * 4, pc);
-    V4<T>::ld(xs + j * XS + pb * 4, xa);
-    V4<T>::ld(xs + SP * XS + j * XS + pb * 4, xc);
-    outer4(al, pa, xa);
-    outer4(ar, pc, xc);
-  }
+  if (look_l) wide_tip_product<T, SP>(a, al, plt, l, n0 + pb * 4, ib);
+  else wide_product<T, SP, XS>(al, plt, xs, a.S, ib, pb);
+  if (look_r) wide_tip_product<T, SP>(a, ar, plt + PS, r, n0 + pb * 4, ib);
+  else wide_product<T, SP, XS>(ar, plt + PS, xs + SP * XS, a.S, ib, pb);
   if (sizeof(T) == 4 && SP == 64 && a.prod) {
     T *pd = a.prod + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * 2 * SP * size_t(a.Npad) + n0 + pb * 4;
 #pragma unroll
@@ -413,8 +464,9 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
   // stored products: FP32 codon plans only (the other instantiations keep GEMM1)
   constexpr bool kProd = sizeof(T) == 4 && SP == 64;
   const bool prod = kProd && a.prod != nullptr;
-  T *plt = reinterpret_cast<T *>(smem);       // [2][SP j][SP perm i]   P^T (GEMM1, absent with stored products)
-  T *pl = prod ? plt : plt + 2 * SP * SP;     // [2][SP i][SP perm j]   P   (GEMM2)
+  constexpr int PS = (SP + kTipRows) * SP;
+  T *plt = reinterpret_cast<T *>(smem);       // [2][SP j + tip rows][SP perm i]   P^T (GEMM1, absent with stored products)
+  T *pl = prod ? plt : plt + 2 * PS;          // [2][SP i][SP perm j]   P   (GEMM2); a tip's gradient in FP64 plans
   T *xs = pl + 2 * SP * SP;              // [2][SP][XS] child tiles
   T *us = xs + 2 * SP * XS;              // [SP][XS]    u of the current side
   T *cf = us + SP * XS;                  // [PT]        coefficients
@@ -432,8 +484,21 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
   for (int e = tid; e < 2 * SP * SP; e += NT) {
     const int c = e / (SP * SP), ij = e - c * SP * SP, i = ij / SP, j = ij - i * SP;
     const T val = a.pmat[((size_t(b) * a.B + (c ? r : l)) * a.K + k) * SP * SP + ij];
-    if (!prod) plt[c * SP * SP + j * SP + wperm<IB>(i)] = val;
+    if (!prod) plt[c * PS + j * SP + wperm<IB>(i)] = val;
     pl[c * SP * SP + i * SP + wperm<IB>(j)] = val;
+  }
+  const bool look_l = !prod && l < a.tips && a.tip_row, look_r = !prod && r < a.tips && a.tip_row;
+  // FP64 plans: a tip's gradient takes one addition per row and pattern, G[i][state] += c u[i], into
+  // [state][i] sums held where the tip's P would be (GEMM2 has no use for it)
+  const bool sum_l = sizeof(T) == 8 && look_l, sum_r = sizeof(T) == 8 && look_r;
+  if ((look_l || look_r) && (a.tip_ambs || sizeof(T) == 8)) {
+    __syncthreads();
+    if (look_l) wide_tip_rows<T, SP, NT>(a, plt);
+    if (look_r) wide_tip_rows<T, SP, NT>(a, plt + PS);
+    for (int e = tid; e < SP * SP; e += NT) {
+      if (sum_l) pl[e] = T(0);
+      if (sum_r) pl[SP * SP + e] = T(0);
+    }
   }
   // GEMM3 ownership: block (gi, gj) of the SP x SP gradient, pattern quads grp, grp + NG, ...
   const int grp = NT >= IB * IB ? tid / (IB * IB) : 0;
@@ -477,8 +542,8 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
         asm volatile("prefetch.global.L2 [%0];" ::"l"(base + size_t(row) * a.Npad + n0 + PT + seg * (128 / int(sizeof(T)))));
       }
     }
-    wide_stage_child<T, SP, PT>(a, l, b, k, n0, xs);
-    wide_stage_child<T, SP, PT>(a, r, b, k, n0, xs + SP * XS);
+    if (!sum_l) wide_stage_child<T, SP, PT>(a, l, b, k, n0, xs);
+    if (!sum_r) wide_stage_child<T, SP, PT>(a, r, b, k, n0, xs + SP * XS);
     if (tid < PT) {
       const int n = n0 + tid;
       const int El = wide_child_expo(a, l, b, k, n), Er = wide_child_expo(a, r, b, k, n);
@@ -514,20 +579,10 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
         V4<T>::ldg(pd + size_t(SP + ib + IB * i) * a.Npad, ar[i]);
       }
     } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) al[i][q] = ar[i][q] = T(0);
-#pragma unroll 4
-      for (int j = 0; j < SP; ++j) {
-        T pa[4], pc[4], xa[4], xc[4];
-        V4<T>::ld(plt + j * SP + ib * 4, pa);
-        V4<T>::ld(plt + SP * SP + j * SP + ib * 4, pc);
-        V4<T>::ld(xs + j * XS + pb * 4, xa);
-        V4<T>::ld(xs + SP * XS + j * XS + pb * 4, xc);
-        outer4(al, pa, xa);
-        outer4(ar, pc, xc);
-      }
+      if (look_l) wide_tip_product<T, SP>(a, al, plt, l, n0 + pb * 4, ib);
+      else wide_product<T, SP, XS>(al, plt, xs, a.S, ib, pb);
+      if (look_r) wide_tip_product<T, SP>(a, ar, plt + PS, r, n0 + pb * 4, ib);
+      else wide_product<T, SP, XS>(ar, plt + PS, xs + SP * XS, a.S, ib, pb);
     }
     if (is_root) {
 #pragma unroll
@@ -561,8 +616,9 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int q = 0; q < 4; ++q) o[i][q] = T(0);
+        const int J = sizeof(T) == 8 ? a.S : SP;
 #pragma unroll 4
-        for (int i = 0; i < SP; ++i) {
+        for (int i = 0; i < J; ++i) {
           T pa[4], ua[4];
           V4<T>::ld(pm + i * SP + ib * 4, pa);
           V4<T>::ld(us + i * XS + pb * 4, ua);
@@ -598,7 +654,20 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
         }
       }
       // GEMM3: dlnL/dP_child += sum_p c_p u[i][p] x_child[j][p]
-      if (g3) {
+      if (side ? sum_r : sum_l) {
+        T *gt = pl + side * SP * SP;
+        const uint8_t *cd = a.codes + size_t(child) * a.code_stride + n0;
+        for (int i = tid; i < a.S; i += NT)
+          for (int p = 0; p < PT; ++p) {
+            const T cu = us[i * XS + p] * cf[p];
+            const int code = cd[p], row = a.tip_row[code];
+            if (row < SP) {
+              gt[row * SP + i] += cu;
+            } else {
+              for (int s = 0; s < a.S; ++s) gt[s * SP + i] = fma(cu, a.table[code * SP + s], gt[s * SP + i]);
+            }
+          }
+      } else if (g3) {
         const T *xc = xs + side * SP * XS;
 #pragma unroll
         for (int m = 0; m < GB; ++m) {
@@ -629,7 +698,10 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
   for (int side = 0; side < 2; ++side) {
     const int child = side ? r : l;
     T *dst = a.gpart + (((size_t(b) * a.B + child) * a.nchunks + chunk) * a.K + k) * SP * SP;
-    if (NG == 1) {
+    if (side ? sum_r : sum_l) {
+      __syncthreads();
+      for (int e = tid; e < SP * SP; e += NT) dst[e] = pl[side * SP * SP + (e % SP) * SP + e / SP];
+    } else if (NG == 1) {
       if (g3) {
 #pragma unroll
         for (int m = 0; m < GB; ++m) {
