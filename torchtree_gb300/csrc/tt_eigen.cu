@@ -91,11 +91,11 @@ __device__ __forceinline__ void jacobi_rotation_f64(double app, double aqq, doub
 // the rotations into V, in T arithmetic, until the off-diagonal norm squared
 // is at most tol2 times the Frobenius norm squared; true when converged within
 // max_sweeps.  cs and pq hold a round's rotations and pairs.  Called by the
-// whole CTA.
-template <typename T>
+// whole CTA, of NT threads; n <= NMAX, rows NMAX + 1 apart.
+template <typename T, int NMAX = kEigMax, int NT = kEigThreads>
 __device__ bool jacobi_sweeps(T *A, T *V, T *cs, int *pq, double *red, int *flag, int n, double tol2,
                               int max_sweeps) {
-  constexpr int NW = kEigThreads / 32;
+  constexpr int NW = NT / 32, LD = NMAX + 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m = n + (n & 1);  // an odd n gets a dummy player that never rotates
   const int npairs = m / 2;
@@ -104,7 +104,7 @@ __device__ bool jacobi_sweeps(T *A, T *V, T *cs, int *pq, double *red, int *flag
     double off = 0.0, tot = 0.0;
     for (int i = warp; i < n; i += NW)
       for (int j = lane; j < n; j += 32) {
-        const double v = double(A[i * kEigLd + j]);
+        const double v = double(A[i * LD + j]);
         tot += v * v;
         if (i != j) off += v * v;
       }
@@ -135,10 +135,10 @@ __device__ bool jacobi_sweeps(T *A, T *V, T *cs, int *pq, double *red, int *flag
         rr_pair(r, tid, m, p, qq);
         T c = T(1), s = T(0);
         if (qq < n) {
-          const T apq = A[p * kEigLd + qq];
+          const T apq = A[p * LD + qq];
           if (apq != T(0)) {
             if constexpr (sizeof(T) == 4) {
-              const T tau = (A[qq * kEigLd + qq] - A[p * kEigLd + p]) / (T(2) * apq);
+              const T tau = (A[qq * LD + qq] - A[p * LD + p]) / (T(2) * apq);
               T t;
               if (fabs(tau) > T(1e18)) t = T(0.5) / tau;
               else t = (tau >= T(0) ? T(1) : T(-1)) / (fabs(tau) + sqrt(T(1) + tau * tau));
@@ -146,7 +146,7 @@ __device__ bool jacobi_sweeps(T *A, T *V, T *cs, int *pq, double *red, int *flag
               s = t * c;
             } else {
               double cd, sd;
-              jacobi_rotation_f64(A[p * kEigLd + p], A[qq * kEigLd + qq], apq, cd, sd);
+              jacobi_rotation_f64(A[p * LD + p], A[qq * LD + qq], apq, cd, sd);
               c = T(cd);
               s = T(sd);
             }
@@ -162,8 +162,9 @@ __device__ bool jacobi_sweeps(T *A, T *V, T *cs, int *pq, double *red, int *flag
       // along the row.  Distinct pairs touch distinct rows, so all of a
       // thread's loads go first (independent shared-memory latencies).
       {
-        constexpr int PK = (kEigMax / 2 + NW - 1) / NW;  // pairs per warp
-        T ap[PK][2], aq[PK][2], cr[PK], sr[PK];
+        constexpr int PK = (NMAX / 2 + NW - 1) / NW;  // pairs per warp
+        constexpr int HC = (NMAX + 31) / 32;             // row parts per lane
+        T ap[PK][HC], aq[PK][HC], cr[PK], sr[PK];
         int pr[PK], qr[PK];
 #pragma unroll
         for (int k = 0; k < PK; ++k) {
@@ -173,28 +174,28 @@ __device__ bool jacobi_sweeps(T *A, T *V, T *cs, int *pq, double *red, int *flag
           cr[k] = i < npairs ? cs[2 * i] : T(1);
           sr[k] = i < npairs ? cs[2 * i + 1] : T(0);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
+          for (int h = 0; h < HC; ++h) {
             const int j = lane + 32 * h;
             const bool go = qr[k] < n && sr[k] != T(0) && j < n;  // not the dummy player nor the identity
-            ap[k][h] = go ? A[pr[k] * kEigLd + j] : T(0);
-            aq[k][h] = go ? A[qr[k] * kEigLd + j] : T(0);
+            ap[k][h] = go ? A[pr[k] * LD + j] : T(0);
+            aq[k][h] = go ? A[qr[k] * LD + j] : T(0);
           }
         }
 #pragma unroll
         for (int k = 0; k < PK; ++k)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
+          for (int h = 0; h < HC; ++h) {
             const int j = lane + 32 * h;
             if (qr[k] < n && sr[k] != T(0) && j < n) {
-              A[pr[k] * kEigLd + j] = cr[k] * ap[k][h] - sr[k] * aq[k][h];
-              A[qr[k] * kEigLd + j] = sr[k] * ap[k][h] + cr[k] * aq[k][h];
+              A[pr[k] * LD + j] = cr[k] * ap[k][h] - sr[k] * aq[k][h];
+              A[qr[k] * LD + j] = sr[k] * ap[k][h] + cr[k] * aq[k][h];
             }
           }
       }
       __syncthreads();
       // columns: A <- A J, V <- V J, a warp per row, lanes over the pairs
       {
-        constexpr int RK = (kEigMax + NW - 1) / NW;  // rows per warp
+        constexpr int RK = (NMAX + NW - 1) / NW;  // rows per warp
         const int i = lane;                           // npairs <= 32
         const int pc = i < npairs ? pq[2 * i] : 0, qc = i < npairs ? pq[2 * i + 1] : n;
         const T c = i < npairs ? cs[2 * i] : T(1), s = i < npairs ? cs[2 * i + 1] : T(0);
@@ -204,19 +205,19 @@ __device__ bool jacobi_sweeps(T *A, T *V, T *cs, int *pq, double *red, int *flag
         for (int k = 0; k < RK; ++k) {
           const int row = warp + k * NW;
           const bool g = go && row < n;
-          a0[k] = g ? A[row * kEigLd + pc] : T(0);
-          a1[k] = g ? A[row * kEigLd + qc] : T(0);
-          v0[k] = g ? V[row * kEigLd + pc] : T(0);
-          v1[k] = g ? V[row * kEigLd + qc] : T(0);
+          a0[k] = g ? A[row * LD + pc] : T(0);
+          a1[k] = g ? A[row * LD + qc] : T(0);
+          v0[k] = g ? V[row * LD + pc] : T(0);
+          v1[k] = g ? V[row * LD + qc] : T(0);
         }
 #pragma unroll
         for (int k = 0; k < RK; ++k) {
           const int row = warp + k * NW;
           if (go && row < n) {
-            A[row * kEigLd + pc] = c * a0[k] - s * a1[k];
-            A[row * kEigLd + qc] = s * a0[k] + c * a1[k];
-            V[row * kEigLd + pc] = c * v0[k] - s * v1[k];
-            V[row * kEigLd + qc] = s * v0[k] + c * v1[k];
+            A[row * LD + pc] = c * a0[k] - s * a1[k];
+            A[row * LD + qc] = s * a0[k] + c * a1[k];
+            V[row * LD + pc] = c * v0[k] - s * v1[k];
+            V[row * LD + qc] = s * v0[k] + c * v1[k];
           }
         }
       }
@@ -228,16 +229,16 @@ __device__ bool jacobi_sweeps(T *A, T *V, T *cs, int *pq, double *red, int *flag
 
 // sqrt(pi) of matrix b into sq, then A = Pi^1/2 Q Pi^-1/2 from the lower
 // triangle (mirrored) into A (leading dimension kEigLd) as T; whole CTA.
-template <typename T>
+template <typename T, int NMAX = kEigMax, int NT = kEigThreads>
 __device__ void load_symmetrised(const double *q, const double *pi, int b, int n, double *sq, T *A) {
-  constexpr int NW = kEigThreads / 32;
+  constexpr int NW = NT / 32, LD = NMAX + 1;
   const double *qb = q + size_t(b) * n * n;
-  for (int i = threadIdx.x; i < n; i += kEigThreads) sq[i] = sqrt(pi[size_t(b) * n + i]);
+  for (int i = threadIdx.x; i < n; i += NT) sq[i] = sqrt(pi[size_t(b) * n + i]);
   __syncthreads();
   for (int i = threadIdx.x >> 5; i < n; i += NW)
     for (int j = threadIdx.x & 31; j < n; j += 32) {
       const int r = i >= j ? i : j, c = i >= j ? j : i;
-      A[i * kEigLd + j] = T(sq[r] * qb[r * n + c] / sq[c]);
+      A[i * LD + j] = T(sq[r] * qb[r * n + c] / sq[c]);
     }
   __syncthreads();
 }
@@ -547,6 +548,71 @@ __global__ void __launch_bounds__(32) gamma_quantiles_kernel(const double *shape
   }
 }
 
+// Matrices of at most kEigSmall states: the three steps above in one launch, a warp
+// per matrix, with their arithmetic.  At 4 states each of the seven launches is a few
+// microseconds of one CTA, mostly barriers of eight warps: 52 -> 34 us and six
+// launches fewer.
+constexpr int kEigSmall = 4;
+
+__global__ void __launch_bounds__(32) eigen_small_kernel(const double *q, const double *pi, int n, double *lam,
+                                                         double *U, double *W, int *status) {
+  constexpr int N = kEigSmall, LD = N + 1;
+  __shared__ float Af[N * LD], Vf[N * LD], csf[N];
+  __shared__ double A[N * LD], X[N * LD], R[N * LD], M[N * LD], cs[N], red[2], sq[N];
+  __shared__ int pq[N], flag;
+  const int b = blockIdx.x, lane = threadIdx.x;
+  load_symmetrised<float, N, 32>(q, pi, b, n, sq, Af);
+  for (int e = lane; e < n * n; e += 32) Vf[e / n * LD + e % n] = e / n == e % n ? 1.0f : 0.0f;
+  __syncthreads();
+  jacobi_sweeps<float, N, 32>(Af, Vf, csf, pq, red, &flag, n, 1e-12, 6);
+  for (int e = lane; e < n * n; e += 32) X[e / n * LD + e % n] = double(Vf[e / n * LD + e % n]);
+  load_symmetrised<double, N, 32>(q, pi, b, n, sq, A);
+  const int i = lane / N, j = lane % N;  // lanes 0-15: an entry each
+  const bool in = i < n && j < n;
+  for (int it = 0; it < 2; ++it) {  // X <- X + X R / 2, R = I - X^T X
+    if (in && j <= i) {
+      double s = 0.0;
+      for (int k = 0; k < n; ++k) s = fma(X[k * LD + i], X[k * LD + j], s);
+      R[i * LD + j] = 0.5 * (j < i ? -s : 1.0 - s);
+    }
+    __syncthreads();
+    double s = 0.0;
+    if (in) {
+      s = X[i * LD + j];
+      for (int k = 0; k < n; ++k) s = fma(X[i * LD + k], R[max(k, j) * LD + min(k, j)], s);
+    }
+    __syncthreads();
+    if (in) X[i * LD + j] = s;
+    __syncthreads();
+  }
+  if (in) {  // S = X^T A X, upper triangle mirrored
+    double s = 0.0;
+    for (int k = 0; k < n; ++k) s = fma(X[k * LD + i], A[k * LD + j], s);
+    M[i * LD + j] = s;
+  }
+  __syncthreads();
+  if (in && j >= i) {
+    double s = 0.0;
+    for (int k = 0; k < n; ++k) s = fma(M[i * LD + k], X[k * LD + j], s);
+    A[i * LD + j] = s;
+    A[j * LD + i] = s;
+  }
+  __syncthreads();
+  const bool ok = jacobi_sweeps<double, N, 32>(A, X, cs, pq, red, &flag, n, 1e-28, 30);
+  if (lane == 0 && !ok) atomicExch(status, TT_ERR_UNSUPPORTED);
+  if (in) {  // eigenvalue j goes to its rank (ties by index)
+    const double lj = A[j * LD + j];
+    int rank = 0;
+    for (int k = 0; k < n; ++k) {
+      const double lk = A[k * LD + k];
+      rank += lk < lj || (lk == lj && k < j);
+    }
+    if (i == 0) lam[size_t(b) * n + rank] = lj;
+    U[(size_t(b) * n + i) * n + rank] = X[i * LD + j] / sq[i];
+    W[(size_t(b) * n + rank) * n + i] = X[i * LD + j] * sq[i];
+  }
+}
+
 int efail(int code, const std::string &msg) { return record_error(code, msg.c_str()); }
 
 }  // namespace
@@ -569,6 +635,11 @@ int tt_reversible_eigen(int32_t batch, int32_t state_count, const double *q, con
   const size_t finish_smem =
       (2 * size_t(kEigMax) * kEigLd + kEigMax + 2 * (kEigThreads / 32) + kEigMax) * sizeof(double) +
       kEigMax * sizeof(int);
+  if (n <= kEigSmall) {
+    eigen_small_kernel<<<batch, 32, 0, s>>>(q, frequencies, n, eigenvalues, u, w, status);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? TT_OK : tt::efail(TT_ERR_CUDA, std::string("eigen launch: ") + cudaGetErrorString(e));
+  }
   cudaError_t e = kernel_smem(eigen_gram_kernel, gram_smem);
   if (e == cudaSuccess) e = kernel_smem(eigen_orth_kernel, orth_smem);
   if (e == cudaSuccess) e = kernel_smem(eigen_finish_kernel, finish_smem);

@@ -11,6 +11,7 @@
 // are bound by launch latency (one CTA per sample, a few microseconds), so
 // they are written for few dependent steps, not for throughput.
 #include <algorithm>
+#include <cstring>
 #include <string>
 
 #include "../../include/torchtree_gb300.h"
@@ -61,16 +62,19 @@ __global__ void __launch_bounds__(32) weibull_rates_kernel(const double *shape, 
   finish_rates(r, dr, K, b, rates, drates, probs);
 }
 
-// one warp per quantile, a CTA per sample
-__global__ void gamma_rates_kernel(const double *shape, int K, double *rates, double *drates, double *probs) {
+// a CTA per sample, a warp per quantile (the first 8 at once)
+__global__ void __launch_bounds__(256) gamma_rates_kernel(const double *shape, int K, double *rates, double *drates,
+                                                          double *probs) {
   __shared__ double xs[32], ds[32];
-  const int b = blockIdx.x, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int b = blockIdx.x, lane = threadIdx.x & 31;
   const double a = shape[b];
-  double x = 0.0, d = 0.0;
-  if (!gamma_quantile_warp(a, (2.0 * k + 1.0) / (2.0 * K), x, d)) x = d = __longlong_as_double(0x7ff8000000000000ll);
-  if (lane == 0) xs[k] = x, ds[k] = d;
+  for (int k = threadIdx.x >> 5; k < K; k += blockDim.x >> 5) {
+    double x = 0.0, d = 0.0;
+    if (!gamma_quantile_warp(a, (2.0 * k + 1.0) / (2.0 * K), x, d)) x = d = __longlong_as_double(0x7ff8000000000000ll);
+    if (lane == 0) xs[k] = x, ds[k] = d;
+  }
   __syncthreads();
-  if (k) return;
+  if (threadIdx.x >= 32) return;
   const double r = lane < K ? xs[lane] / a : 0.0, dr = lane < K ? ds[lane] / a - xs[lane] / (a * a) : 0.0;
   finish_rates(r, dr, K, b, rates, drates, probs);
 }
@@ -89,7 +93,8 @@ __global__ void __launch_bounds__(32) rates_backward_kernel(const double *grad, 
 // of it has to be kept anywhere.
 struct NoMap {};
 struct PairMap {
-  int8_t m[2 * 64 * 63 / 2];  // [2][S (S-1) / 2] parameter indices (-1: 1)
+  static constexpr int kWords = 2 * 64 * 63 / 2 / 4;
+  uint32_t m[kWords];  // [2][S (S-1) / 2] parameter indices (-1: 1), four to a word
 };
 
 template <typename Map>
@@ -99,10 +104,6 @@ struct Exch {
   int n[3];
   int count;  // S (S-1) / 2
   Map map;
-  __device__ __forceinline__ int index(int which, int e) const {
-    if constexpr (kMapped) return map.m[which * count + e];
-    else return e;
-  }
   __device__ __forceinline__ double param(int b, int i) const {
     if (i < 0) return 1.0;
     if (i < n[0]) return p[0][size_t(b) * n[0] + i];
@@ -110,8 +111,17 @@ struct Exch {
     if (i < n[1]) return p[1][size_t(b) * n[1] + i];
     return p[2][size_t(b) * n[2] + i - n[1]];
   }
-  __device__ __forceinline__ double value(int b, int e) const {
-    if constexpr (kMapped) return param(b, index(0, e)) * param(b, index(1, e));
+  // the map into shared memory: a parameter indexed per lane is read one lane at a time (with
+  // the pairs read from it directly, 118 us at 61 states)
+  __device__ __forceinline__ const int8_t *stage(uint32_t *sm) const {
+    if constexpr (kMapped) {
+      for (int w = threadIdx.x; w < PairMap::kWords; w += blockDim.x) sm[w] = map.m[w];
+      __syncthreads();
+    }
+    return reinterpret_cast<const int8_t *>(sm);
+  }
+  __device__ __forceinline__ double value(int b, const int8_t *m, int e) const {
+    if constexpr (kMapped) return param(b, m[e]) * param(b, m[count + e]);
     else return p[0][size_t(b) * n[0] + e];
   }
 };
@@ -123,17 +133,19 @@ __device__ __forceinline__ int upper_index(int i, int j, int S) {  // i != j
 
 template <typename Map>
 __global__ void __launch_bounds__(256) exch_q_kernel(const __grid_constant__ Exch<Map> x, const double *pi, int S, double *q) {
+  __shared__ uint32_t sm[Exch<Map>::kMapped ? PairMap::kWords : 1];
+  const int8_t *m = x.stage(sm);
   const int b = blockIdx.x;
   const double *pb = pi + size_t(b) * S;
   double *qb = q + size_t(b) * S * S;
   for (int e = threadIdx.x; e < S * S; e += blockDim.x) {
     const int i = e / S, j = e - i * S;
-    if (i != j) qb[e] = x.value(b, upper_index(i, j, S)) * pb[j];
+    if (i != j) qb[e] = x.value(b, m, upper_index(i, j, S)) * pb[j];
   }
   for (int i = threadIdx.x; i < S; i += blockDim.x) {
     double s = 0.0;
     for (int j = 0; j < S; ++j)
-      if (j != i) s += x.value(b, upper_index(i, j, S)) * pb[j];
+      if (j != i) s += x.value(b, m, upper_index(i, j, S)) * pb[j];
     qb[i * S + i] = -s;
   }
 }
@@ -143,6 +155,8 @@ template <typename Map>
 __global__ void __launch_bounds__(256) exch_q_backward_kernel(const __grid_constant__ Exch<Map> x, const double *pi, const double *G, int S,
                                                               double *d0, double *d1, double *d2, double *dpi) {
   __shared__ double red[3][8];
+  __shared__ uint32_t sm[Exch<Map>::kMapped ? PairMap::kWords : 1];
+  const int8_t *m = x.stage(sm);
   const int b = blockIdx.x, tid = threadIdx.x;
   const double *pb = pi + size_t(b) * S, *g = G + size_t(b) * S * S;
   double acc[3] = {0.0, 0.0, 0.0};
@@ -154,7 +168,7 @@ __global__ void __launch_bounds__(256) exch_q_backward_kernel(const __grid_const
     if constexpr (!Exch<Map>::kMapped) {
       if (d0) d0[size_t(b) * x.count + u] = d;
     } else {
-      const int m0 = x.index(0, u), m1 = x.index(1, u);
+      const int m0 = m[u], m1 = m[x.count + u];
       const double v0 = x.param(b, m0), v1 = x.param(b, m1);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -167,7 +181,7 @@ __global__ void __launch_bounds__(256) exch_q_backward_kernel(const __grid_const
     for (int j = tid; j < S; j += 256) {
       double s = 0.0;
       for (int i = 0; i < S; ++i)
-        if (i != j) s = fma(g[i * S + j] - g[i * S + i], x.value(b, upper_index(i, j, S)), s);
+        if (i != j) s = fma(g[i * S + j] - g[i * S + i], x.value(b, m, upper_index(i, j, S)), s);
       dpi[size_t(b) * S + j] = s;
     }
   if (!Exch<Map>::kMapped) return;
@@ -275,7 +289,7 @@ Exch<Map> exch_of(int32_t S, const int32_t *counts, const double *p0, const doub
   x.p[0] = p0, x.p[1] = p1, x.p[2] = p2;
   for (int i = 0; i < 3; ++i) x.n[i] = counts[i];
   x.count = S * (S - 1) / 2;
-  if constexpr (Exch<Map>::kMapped) std::copy(map, map + 2 * x.count, x.map.m);
+  if constexpr (Exch<Map>::kMapped) std::memcpy(x.map.m, map, 2 * size_t(x.count));
   return x;
 }
 
@@ -318,7 +332,7 @@ int tt_gamma_rates(int32_t batch, int32_t category_count, const double *shape, d
   using namespace tt;
   if (!shape || !rates || !drates_dshape || !weights || batch < 1 || category_count < 1 || category_count > 32)
     return sfail(TT_ERR_INVALID_ARGUMENT, "category rates: NULL argument, empty batch or more than 32 categories");
-  gamma_rates_kernel<<<batch, 32 * category_count, 0, static_cast<cudaStream_t>(stream)>>>(
+  gamma_rates_kernel<<<batch, 32 * std::min(category_count, 8), 0, static_cast<cudaStream_t>(stream)>>>(
       shape, category_count, rates, drates_dshape, weights);
   return sdone(cudaGetLastError(), "Gamma rates launch");
 }
