@@ -35,11 +35,19 @@
 
 namespace tt {
 
+// Patterns of a thread's register tile.  FP64 codon plans take two, so that a
+// 32-pattern tile has 256 threads (two warps per SM quarter) and the adjoint's
+// gradient blocks one per thread: with four, 2.2 KB of them spilled.  60 taxa x 301
+// patterns: adjoint 3,088 -> 2,796 us, post-order 1,020 -> 970 us.
+template <typename T, int SP>
+constexpr int kTileQ = sizeof(T) == 8 && SP == 64 ? 2 : 4;
+
 template <typename T, int SP, int PT>
 struct WideCfg {
-  static_assert(SP % 4 == 0 && PT % 4 == 0, "tiles are 4 x 4");
+  static constexpr int PQ = kTileQ<T, SP>;
+  static_assert(SP % 4 == 0 && PT % 4 == 0, "tiles are 4 x PQ, gradient quads 4");
   static constexpr int IB = SP / 4;                                 // row blocks
-  static constexpr int PB = PT / 4;                                 // pattern blocks
+  static constexpr int PB = PT / PQ;                                // pattern blocks
   static constexpr int NT = IB * PB;                                // threads
   static constexpr int XS = PT + 16 / int(sizeof(T));               // padded tile row stride
   static constexpr int NG = NT >= IB * IB ? NT / (IB * IB) : 1;    // GEMM3 pattern groups
@@ -106,13 +114,32 @@ struct V4<double> {
   }
 };
 
-// acc[i][j] += a[i] b[j] over a 4 x 4 register tile; FP32 runs as packed
+// PQ consecutive values: four, or two in FP64
+template <typename T, int PQ>
+struct VP : V4<T> {};
+template <>
+struct VP<double, 2> {
+  static __device__ __forceinline__ void ld(const double *p, double (&v)[2]) {
+    const double2 a = *reinterpret_cast<const double2 *>(p);
+    v[0] = a.x, v[1] = a.y;
+  }
+  static __device__ __forceinline__ void ldg(const double *p, double (&v)[2]) {
+    const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
+    v[0] = a.x, v[1] = a.y;
+  }
+  static __device__ __forceinline__ void st(double *p, const double (&v)[2]) {
+    *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+  }
+};
+
+// acc[i][j] += a[i] b[j] over a 4 x 4 (FP64: 4 x PQ) register tile; FP32 runs as packed
 // FP32x2 FMAs (pairs along j), FP64 as scalar FMAs
-__device__ __forceinline__ void outer4(double (&acc)[4][4], const double (&a)[4], const double (&b)[4]) {
+template <int PQ>
+__device__ __forceinline__ void outer4(double (&acc)[4][PQ], const double (&a)[4], const double (&b)[PQ]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+    for (int j = 0; j < PQ; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
 }
 
 __device__ __forceinline__ void outer4(float (&acc)[4][4], const float (&a)[4], const float (&b)[4]) {
@@ -262,13 +289,14 @@ __device__ __forceinline__ void wide_tip_rows(const WideArgs<T> &a, T *plt) {
 
 // the thread's 4 rows x 4 patterns of a tip child's product
 template <typename T, int SP>
-__device__ __forceinline__ void wide_tip_product(const WideArgs<T> &a, T (&acc)[4][4], const T *plt, int child, int n,
-                                                 int ib) {
-  const uint32_t codes = *reinterpret_cast<const uint32_t *>(a.codes + size_t(child) * a.code_stride + n);
+__device__ __forceinline__ void wide_tip_product(const WideArgs<T> &a, T (&acc)[4][kTileQ<T, SP>], const T *plt,
+                                                 int child, int n, int ib) {
+  constexpr int PQ = kTileQ<T, SP>;
+  const uint8_t *codes = a.codes + size_t(child) * a.code_stride + n;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < PQ; ++q) {
     T col[4];
-    V4<T>::ld(plt + int(__ldg(a.tip_row + ((codes >> (8 * q)) & 0xff))) * SP + ib * 4, col);
+    V4<T>::ld(plt + int(__ldg(a.tip_row + __ldg(codes + q))) * SP + ib * 4, col);
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i][q] = col[i];
   }
@@ -276,17 +304,19 @@ __device__ __forceinline__ void wide_tip_product(const WideArgs<T> &a, T (&acc)[
 
 // ... of an internal child's (or any staged vector's)
 template <typename T, int SP, int XS>
-__device__ __forceinline__ void wide_product(T (&acc)[4][4], const T *plt, const T *xs, int S, int ib, int pb) {
+__device__ __forceinline__ void wide_product(T (&acc)[4][kTileQ<T, SP>], const T *plt, const T *xs, int S, int ib,
+                                             int pb) {
+  constexpr int PQ = kTileQ<T, SP>;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[i][q] = T(0);
+    for (int q = 0; q < PQ; ++q) acc[i][q] = T(0);
   const int J = sizeof(T) == 8 ? S : SP;  // FP64: no work for the padding states
 #pragma unroll 4
   for (int j = 0; j < J; ++j) {
-    T pa[4], xa[4];
+    T pa[4], xa[PQ];
     V4<T>::ld(plt + j * SP + ib * 4, pa);
-    V4<T>::ld(xs + j * XS + pb * 4, xa);
+    VP<T, PQ>::ld(xs + j * XS + pb * PQ, xa);
     outer4(acc, pa, xa);
   }
 }
@@ -295,7 +325,7 @@ __device__ __forceinline__ void wide_product(T (&acc)[4][4], const T *plt, const
 template <typename T, int SP, int PT>
 __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(const WideArgs<T> a) {
   using C = WideCfg<T, SP, PT>;
-  constexpr int IB = C::IB, NT = C::NT, XS = C::XS;
+  constexpr int IB = C::IB, NT = C::NT, XS = C::XS, PQ = C::PQ;
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int PS = (SP + kTipRows) * SP;                        // one side's staged matrix and tip rows
   T *plt = reinterpret_cast<T *>(smem);                          // [2][SP j + tip rows][SP perm i]
@@ -323,23 +353,23 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
     __syncthreads();
   }
 
-  T al[4][4], ar[4][4];
-  if (look_l) wide_tip_product<T, SP>(a, al, plt, l, n0 + pb * 4, ib);
+  T al[4][PQ], ar[4][PQ];
+  if (look_l) wide_tip_product<T, SP>(a, al, plt, l, n0 + pb * PQ, ib);
   else wide_product<T, SP, XS>(al, plt, xs, a.S, ib, pb);
-  if (look_r) wide_tip_product<T, SP>(a, ar, plt + PS, r, n0 + pb * 4, ib);
+  if (look_r) wide_tip_product<T, SP>(a, ar, plt + PS, r, n0 + pb * PQ, ib);
   else wide_product<T, SP, XS>(ar, plt + PS, xs + SP * XS, a.S, ib, pb);
   if (sizeof(T) == 4 && SP == 64 && a.prod) {
-    T *pd = a.prod + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * 2 * SP * size_t(a.Npad) + n0 + pb * 4;
+    T *pd = a.prod + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * 2 * SP * size_t(a.Npad) + n0 + pb * PQ;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      V4<T>::st(pd + size_t(ib + IB * i) * a.Npad, al[i]);
-      V4<T>::st(pd + size_t(SP + ib + IB * i) * a.Npad, ar[i]);
+      VP<T, PQ>::st(pd + size_t(ib + IB * i) * a.Npad, al[i]);
+      VP<T, PQ>::st(pd + size_t(SP + ib + IB * i) * a.Npad, ar[i]);
     }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) al[i][q] *= ar[i][q];
+    for (int q = 0; q < PQ; ++q) al[i][q] *= ar[i][q];
 
   if (is_root) {  // sum_i pi_i L[k][i] per pattern, FP64
     double f[4];
@@ -349,11 +379,11 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
       f[i] = row < a.S ? a.freqs[size_t(b) * a.S + row] : 0.0;
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < PQ; ++q) {
       double s = 0.0;
 #pragma unroll
       for (int i = 0; i < 4; ++i) s = fma(f[i], double(al[i][q]), s);
-      red[ib * PT + pb * 4 + q] = s;
+      red[ib * PT + pb * PQ + q] = s;
     }
     __syncthreads();
     if (tid < PT) {
@@ -370,11 +400,11 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
     using M = MaxBits<T>;
     typename M::type *mred = reinterpret_cast<typename M::type *>(red);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < PQ; ++q) {
       typename M::type m = M::zero();
 #pragma unroll
       for (int i = 0; i < 4; ++i) m = M::larger(m, M::of(al[i][q]));
-      mred[ib * PT + pb * 4 + q] = m;
+      mred[ib * PT + pb * PQ + q] = m;
     }
     __syncthreads();
     if (tid < PT) {
@@ -384,15 +414,15 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
     }
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = ex[pb * 4 + q];
+    for (int q = 0; q < PQ; ++q) {
+      const int e = ex[pb * PQ + q];
 #pragma unroll
       for (int i = 0; i < 4; ++i) al[i][q] = times_pow2_neg(al[i][q], e);
     }
   }
-  T *dst = a.part + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * SP * size_t(a.Npad) + n0 + pb * 4;
+  T *dst = a.part + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * SP * size_t(a.Npad) + n0 + pb * PQ;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) V4<T>::st(dst + size_t(ib + IB * i) * a.Npad, al[i]);
+  for (int i = 0; i < 4; ++i) VP<T, PQ>::st(dst + size_t(ib + IB * i) * a.Npad, al[i]);
   if (tid < PT) {
     const int n = n0 + tid;
     a.expo[((size_t(b) * a.I + (v - a.tips)) * a.K + k) * a.Npad + n] =
@@ -459,7 +489,7 @@ template <typename T, int SP, int PT>
 __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T, SP>())
     wide_backward_kernel(const WideArgs<T> a) {
   using C = WideCfg<T, SP, PT>;
-  constexpr int IB = C::IB, NT = C::NT, XS = C::XS, NG = C::NG, GB = C::GB;
+  constexpr int IB = C::IB, NT = C::NT, XS = C::XS, NG = C::NG, GB = C::GB, PQ = C::PQ;
   extern __shared__ __align__(128) unsigned char smem[];
   // stored products: FP32 codon plans only (the other instantiations keep GEMM1)
   constexpr bool kProd = sizeof(T) == 4 && SP == 64;
@@ -556,38 +586,38 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
       cf[tid] = c;
     }
     // this thread's block of the outside partial of v
-    T pre[4][4];
+    T pre[4][PQ];
     if (is_root) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) pre[i][q] = T(wk * fr[i]);
+        for (int q = 0; q < PQ; ++q) pre[i][q] = T(wk * fr[i]);
     } else {
-      const T *src = a.part + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * SP * size_t(a.Npad) + n0 + pb * 4;
+      const T *src = a.part + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * SP * size_t(a.Npad) + n0 + pb * PQ;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) V4<T>::ldg(src + size_t(ib + IB * i) * a.Npad, pre[i]);
+      for (int i = 0; i < 4; ++i) VP<T, PQ>::ldg(src + size_t(ib + IB * i) * a.Npad, pre[i]);
     }
     __syncthreads();
 
-    T al[4][4], ar[4][4];
+    T al[4][PQ], ar[4][PQ];
     if (prod) {  // the post-order's products
       const T *pd =
-          a.prod + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * 2 * SP * size_t(a.Npad) + n0 + pb * 4;
+          a.prod + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * 2 * SP * size_t(a.Npad) + n0 + pb * PQ;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        V4<T>::ldg(pd + size_t(ib + IB * i) * a.Npad, al[i]);
-        V4<T>::ldg(pd + size_t(SP + ib + IB * i) * a.Npad, ar[i]);
+        VP<T, PQ>::ldg(pd + size_t(ib + IB * i) * a.Npad, al[i]);
+        VP<T, PQ>::ldg(pd + size_t(SP + ib + IB * i) * a.Npad, ar[i]);
       }
     } else {
-      if (look_l) wide_tip_product<T, SP>(a, al, plt, l, n0 + pb * 4, ib);
+      if (look_l) wide_tip_product<T, SP>(a, al, plt, l, n0 + pb * PQ, ib);
       else wide_product<T, SP, XS>(al, plt, xs, a.S, ib, pb);
-      if (look_r) wide_tip_product<T, SP>(a, ar, plt + PS, r, n0 + pb * 4, ib);
+      if (look_r) wide_tip_product<T, SP>(a, ar, plt + PS, r, n0 + pb * PQ, ib);
       else wide_product<T, SP, XS>(ar, plt + PS, xs + SP * XS, a.S, ib, pb);
     }
     if (is_root) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const T c = cf[pb * 4 + q];
+      for (int q = 0; q < PQ; ++q) {
+        const T c = cf[pb * PQ + q];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const T R = c * al[i][q] * ar[i][q];
@@ -600,38 +630,47 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
       const int child = side ? r : l;
-      // u = pre .* (product of the other side)
+      // u = pre .* (product of the other side), for GEMM2; FP64 plans store c u for GEMM3 (scaled
+      // once, not at every use; in FP32 the registers that keeps alive spill: 3,271 -> 3,353 us)
+      auto store_u = [&](bool scaled) {
+        T c4[PQ];
+        VP<T, PQ>::ld(cf + pb * PQ, c4);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        T u4[4];
+        for (int i = 0; i < 4; ++i) {
+          T u4[PQ];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) u4[q] = pre[i][q] * (side ? al[i][q] : ar[i][q]);
-        V4<T>::st(us + (ib + IB * i) * XS + pb * 4, u4);
-      }
+          for (int q = 0; q < PQ; ++q) {
+            u4[q] = pre[i][q] * (side ? al[i][q] : ar[i][q]);
+            if (scaled) u4[q] *= c4[q];
+          }
+          VP<T, PQ>::st(us + (ib + IB * i) * XS + pb * PQ, u4);
+        }
+      };
+      store_u(sizeof(T) == 8 && child < a.tips);
       __syncthreads();
       if (child >= a.tips) {  // GEMM2: outside partial of the child, rescaled, in place of its forward partial
         const T *pm = pl + side * SP * SP;
-        T o[4][4];
+        T o[4][PQ];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) o[i][q] = T(0);
+          for (int q = 0; q < PQ; ++q) o[i][q] = T(0);
         const int J = sizeof(T) == 8 ? a.S : SP;
 #pragma unroll 4
         for (int i = 0; i < J; ++i) {
-          T pa[4], ua[4];
+          T pa[4], ua[PQ];
           V4<T>::ld(pm + i * SP + ib * 4, pa);
-          V4<T>::ld(us + i * XS + pb * 4, ua);
+          VP<T, PQ>::ld(us + i * XS + pb * PQ, ua);
           outer4(o, pa, ua);
         }
         using M = MaxBits<T>;
         typename M::type *mred = reinterpret_cast<typename M::type *>(red);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < PQ; ++q) {
           typename M::type m = M::zero();
 #pragma unroll
           for (int s = 0; s < 4; ++s) m = M::larger(m, M::of(o[s][q]));
-          mred[ib * PT + pb * 4 + q] = m;
+          mred[ib * PT + pb * PQ + q] = m;
         }
         __syncthreads();
         if (tid < PT) {
@@ -644,13 +683,17 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
               ep[tid] + (side ? el[tid] : er[tid]) + e;
         }
         __syncthreads();
-        T *dst = a.part + ((size_t(b) * a.I + (child - a.tips)) * a.K + k) * SP * size_t(a.Npad) + n0 + pb * 4;
+        T *dst = a.part + ((size_t(b) * a.I + (child - a.tips)) * a.K + k) * SP * size_t(a.Npad) + n0 + pb * PQ;
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-          T o4[4];
+          T o4[PQ];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) o4[q] = times_pow2_neg(o[s][q], ex[pb * 4 + q]);
-          V4<T>::st(dst + size_t(ib + IB * s) * a.Npad, o4);
+          for (int q = 0; q < PQ; ++q) o4[q] = times_pow2_neg(o[s][q], ex[pb * PQ + q]);
+          VP<T, PQ>::st(dst + size_t(ib + IB * s) * a.Npad, o4);
+        }
+        if constexpr (sizeof(T) == 8) {
+          store_u(true);  // GEMM2's reads ended before the maxima's barriers
+          __syncthreads();
         }
       }
       // GEMM3: dlnL/dP_child += sum_p c_p u[i][p] x_child[j][p]
@@ -659,7 +702,7 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
         const uint8_t *cd = a.codes + size_t(child) * a.code_stride + n0;
         for (int i = tid; i < a.S; i += NT)
           for (int p = 0; p < PT; ++p) {
-            const T cu = us[i * XS + p] * cf[p];
+            const T cu = us[i * XS + p];
             const int code = cd[p], row = a.tip_row[code];
             if (row < SP) {
               gt[row * SP + i] += cu;
@@ -674,13 +717,16 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
           const int blk = NT >= IB * IB ? tid % (IB * IB) : tid + m * NT;
           const int gi = blk / IB, gj = blk - gi * IB;
           for (int qd = grp; qd < PT / 4; qd += NG) {
-            T c4[4], uu[4][4], xx[4][4];
-            V4<T>::ld(cf + qd * 4, c4);
+            T uu[4][4], xx[4][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              V4<T>::ld(us + (gi + IB * i) * XS + qd * 4, uu[i]);
+            for (int i = 0; i < 4; ++i) V4<T>::ld(us + (gi + IB * i) * XS + qd * 4, uu[i]);
+            if constexpr (sizeof(T) == 4) {
+              T c4[4];
+              V4<T>::ld(cf + qd * 4, c4);
 #pragma unroll
-              for (int q = 0; q < 4; ++q) uu[i][q] *= c4[q];
+              for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) uu[i][q] *= c4[q];
             }
 #pragma unroll
             for (int s = 0; s < 4; ++s) V4<T>::ld(xc + (gj + IB * s) * XS + qd * 4, xx[s]);
