@@ -359,6 +359,10 @@ struct Wide {
     a.ntiles = ntc;
     a.tiles_per_chunk = tpc;
     a.nchunks = (ntc + tpc - 1) / tpc;
+    // The encoder is a driver call: it needs a current context, which a thread that has made no
+    // runtime call yet (autograd's) gets from cudaSetDevice.  The plan's device is current already.
+    const cudaError_t ctx = cudaSetDevice(p->device);
+    if (ctx != cudaSuccess) return ctx;
     // the raw rows as 2-D tensors: partials [b I K 64][Npad], products [b I K 128][Npad]
     TcbMaps maps;
     const uint64_t blocks = uint64_t(p->batch) * p->I * p->K;
