@@ -70,3 +70,55 @@ def test_tip_lookups_match_oracle(precision, S, N, K, b, extra):
         lnl2 = eng.log_likelihood(pd, fd, rescale=False)
         np.testing.assert_allclose(lnl2.cpu().numpy(), ref[0], rtol=1e-10)
     assert eng.device_status() == 0
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("S", [20, 61])
+def test_captured_pass_follows_tips_set_anew(precision, S):
+    """A pass captured before the plan's tips (none ambiguous) are replaced by others of as
+    many codes, with 3 and then 6 ambiguous ones, and its matrices by others: the replay
+    gives what a new plan of those tips and matrices gives (the same kernels: FP64 1e-12;
+    FP32 1e-6 and 1e-5 of the largest entry, for shared sums in another order)."""
+    from torchtree_gb300 import _native, synthetic
+    from torchtree_gb300.engine import LikelihoodEngine
+
+    T, N, K = 9, 400, 2
+    rng = np.random.default_rng(S)
+    topo = synthetic.yule_topology(T, rng)
+    tables = [np.concatenate([np.eye(S), np.eye(S)[:6 - e], _codes(S, e, rng)[S:]]) for e in (0, 3, 6)]
+    codes = rng.integers(0, S + 6, (T, N)).astype(np.uint8)
+    w = rng.integers(1, 4, N).astype(np.float64)
+    dev = torch.device("cuda")
+    pd = torch.tensor(rng.dirichlet(np.ones(K), size=1), device=dev)
+    fd = torch.tensor(rng.dirichlet(np.ones(S), size=1), device=dev)
+    mats = [torch.tensor(0.9 * np.eye(S) + 0.1 * rng.dirichlet(0.5 * np.ones(S), size=(1, 2 * T - 2, K, S)) + 1e-3,
+                         device=dev) for _ in tables]
+
+    def plan(table):
+        return LikelihoodEngine(topo.postorder, T, S, K, codes, table, w, batch=1, precision=precision)
+
+    def work(eng):
+        lnl = eng.log_likelihood(pd, fd, rescale=True, keep_partials=True)
+        return [lnl, *eng.gradient(pd, fd, want_matrices=True)]
+
+    eng = plan(tables[0])
+    eng.set_matrices(mats[0])
+    work(eng)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = work(eng)
+    for table, m in zip(tables, mats):
+        host = np.ascontiguousarray(table)
+        _native.check(eng.lib.tt_plan_set_tips(eng._plan, _native.ptr(codes), _native.ptr(host), host.shape[0],
+                                               _native.ptr(w)))
+        eng.set_matrices(m)
+        graph.replay()
+        fresh = plan(table)
+        fresh.set_matrices(m)
+        want = work(fresh)
+        torch.cuda.synchronize()
+        for i, (got, ref) in enumerate(zip(outs, want)):
+            tol = 1e-12 if precision == "f64" else (1e-5 if i else 1e-6)
+            np.testing.assert_allclose(got.cpu().numpy(), ref.cpu().numpy(), rtol=tol,
+                                       atol=tol * float(ref.abs().max()))

@@ -67,10 +67,8 @@ struct WideState {
   void *d_gpart = nullptr;
   void *d_rootpart = nullptr;
   double *d_pgpart = nullptr;
-  uint8_t *d_tip_row = nullptr;  // [256] code -> row of the staged P^T (WideArgs::tip_row)
+  uint8_t *d_tip_row = nullptr;  // [258] code -> row of the staged P^T (WideArgs::tip_row)
   void *d_tip_amb = nullptr;     // [kTipRows][SP] the ambiguous code vectors
-  int tip_ambs = 0;
-  bool tip_rows_ok = false;      // at most kTipRows ambiguous codes
   void *d_prod = nullptr;  // FP32: the children's products of the post-order, read by the adjoint
 };
 
@@ -227,9 +225,8 @@ struct Wide {
     a.right = w.d_right;
     a.codes = p->d_codes + p0;
     a.table = static_cast<const T *>(p->d_table);
-    a.tip_row = w.tip_rows_ok ? w.d_tip_row : nullptr;
+    a.tip_row = w.d_tip_row;
     a.tip_amb = static_cast<const T *>(w.d_tip_amb);
-    a.tip_ambs = w.tip_ambs;
     a.pmat = static_cast<const T *>(p->d_pmat);
     a.part = static_cast<T *>(w.d_part);
     a.expo = w.d_expo;
@@ -503,7 +500,7 @@ int wide_create(tt_plan *p) {
   if (!rc) rc = walloc(p, &w->d_branch_lvn, size_t(p->B) * sizeof(int), "branch levels");
   if (!rc) rc = walloc(p, &p->d_codes, size_t(T) * p->code_stride, "tip codes");
   if (!rc) rc = walloc(p, &p->d_table, 256 * SP * es, "code table");
-  if (!rc) rc = walloc(p, &w->d_tip_row, 256, "tip rows");
+  if (!rc) rc = walloc(p, &w->d_tip_row, 258, "tip rows");
   if (!rc) rc = walloc(p, &w->d_tip_amb, kTipRows * SP * es, "ambiguous code vectors");
   if (!rc) rc = walloc(p, &p->d_weights, size_t(p->N) * sizeof(double), "weights");
   if (!rc) rc = walloc(p, &p->d_pmat, b * p->B * K * SP * SP * es, "transition matrices");
@@ -692,7 +689,7 @@ int wide_set_tips(tt_plan *p, const uint8_t *codes, const double *code_table, in
     }
   // codes whose product is a row of the staged P^T: unit vectors, and the first kTipRows others
   WideState &w = *p->wide;
-  std::vector<uint8_t> rows(256, 0);
+  std::vector<uint8_t> rows(258, 0);
   std::vector<unsigned char> amb(size_t(kTipRows) * SP * p->elem, 0);
   int ambs = 0;
   bool ok = true;
@@ -713,8 +710,8 @@ int wide_set_tips(tt_plan *p, const uint8_t *codes, const double *code_table, in
       ok = false;
     }
   }
-  w.tip_ambs = ambs;
-  w.tip_rows_ok = ok;
+  rows[256] = ok;
+  rows[257] = uint8_t(ambs);
   cudaError_t e = cudaMemset(p->d_codes, 0, size_t(p->T) * p->code_stride);
   if (e == cudaSuccess) e = cudaMemcpy(w.d_tip_row, rows.data(), rows.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(w.d_tip_amb, amb.data(), amb.size(), cudaMemcpyHostToDevice);

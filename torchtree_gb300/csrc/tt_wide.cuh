@@ -59,8 +59,8 @@ struct WideCfg {
 // a column of P, which the staged P^T holds as a row; the products with up to
 // kTipRows other code vectors (gaps, ambiguous states) are formed once per CTA,
 // term by term as the product, and staged as further rows.  Either way the bits
-// are the product's.  WideArgs::tip_row maps a code to its row (NULL: a plan with
-// more such codes, whose tips take the product).
+// are the product's.  WideArgs::tip_row maps a code to its row (tips of
+// more such codes take the product).
 constexpr int kTipRows = 4;
 
 // shared-memory bytes of the two kernels
@@ -203,9 +203,10 @@ struct WideArgs {
   const int *left, *right;  // [I] children of internal node v - tips
   const uint8_t *codes;     // [tips][code_stride]
   const T *table;           // [C][SP]
-  const uint8_t *tip_row;   // [256] row of the staged P^T that is the code's product, or NULL
-  const T *tip_amb;         // [kTipRows][SP] code vectors of rows SP .. SP + tip_ambs - 1
-  int tip_ambs;
+  // [256] row of the staged P^T that is the code's product; [256] whether every code has one, [257] how
+  // many ambiguous codes: read on the device, so that a captured pass follows tips that are set anew
+  const uint8_t *tip_row;
+  const T *tip_amb;         // [kTipRows][SP] code vectors of rows SP .. SP + tip_row[257] - 1
   const T *pmat;            // [b][B][K][SP][SP]
   T *part;                  // [b][I][K][SP][Npad]
   int *expo;                // [b][I][K][Npad]
@@ -278,7 +279,8 @@ struct MaxBits<double> {
 // rows SP .. of a tip child's staged P^T ([j][perm i]): its products with the ambiguous code vectors
 template <typename T, int SP, int NT>
 __device__ __forceinline__ void wide_tip_rows(const WideArgs<T> &a, T *plt) {
-  for (int e = threadIdx.x; e < a.tip_ambs * SP; e += NT) {
+  const int ambs = __ldg(a.tip_row + 257);
+  for (int e = threadIdx.x; e < ambs * SP; e += NT) {
     const int m = e / SP, i = e - m * SP;
     T acc = T(0);
 #pragma unroll 4
@@ -343,11 +345,11 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
     const int c = e / (SP * SP), ij = e - c * SP * SP, i = ij / SP, j = ij - i * SP;
     plt[c * PS + j * SP + wperm<IB>(i)] = a.pmat[((size_t(b) * a.B + (c ? r : l)) * a.K + k) * SP * SP + ij];
   }
-  const bool look_l = l < a.tips && a.tip_row, look_r = r < a.tips && a.tip_row;
+  const bool rows = __ldg(a.tip_row + 256), look_l = l < a.tips && rows, look_r = r < a.tips && rows;
   if (!look_l) wide_stage_child<T, SP, PT>(a, l, b, k, n0, xs);
   if (!look_r) wide_stage_child<T, SP, PT>(a, r, b, k, n0, xs + SP * XS);
   __syncthreads();
-  if ((look_l || look_r) && a.tip_ambs) {
+  if ((look_l || look_r) && __ldg(a.tip_row + 257)) {
     if (look_l) wide_tip_rows<T, SP, NT>(a, plt);
     if (look_r) wide_tip_rows<T, SP, NT>(a, plt + PS);
     __syncthreads();
@@ -517,11 +519,11 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
     if (!prod) plt[c * PS + j * SP + wperm<IB>(i)] = val;
     pl[c * SP * SP + i * SP + wperm<IB>(j)] = val;
   }
-  const bool look_l = !prod && l < a.tips && a.tip_row, look_r = !prod && r < a.tips && a.tip_row;
+  const bool rows = !prod && __ldg(a.tip_row + 256), look_l = rows && l < a.tips, look_r = rows && r < a.tips;
   // FP64 plans: a tip's gradient takes one addition per row and pattern, G[i][state] += c u[i], into
   // [state][i] sums held where the tip's P would be (GEMM2 has no use for it)
   const bool sum_l = sizeof(T) == 8 && look_l, sum_r = sizeof(T) == 8 && look_r;
-  if ((look_l || look_r) && (a.tip_ambs || sizeof(T) == 8)) {
+  if ((look_l || look_r) && (sizeof(T) == 8 || __ldg(a.tip_row + 257))) {
     __syncthreads();
     if (look_l) wide_tip_rows<T, SP, NT>(a, plt);
     if (look_r) wide_tip_rows<T, SP, NT>(a, plt + PS);
