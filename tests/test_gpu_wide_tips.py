@@ -122,3 +122,39 @@ def test_captured_pass_follows_tips_set_anew(precision, S):
             tol = 1e-12 if precision == "f64" else (1e-5 if i else 1e-6)
             np.testing.assert_allclose(got.cpu().numpy(), ref.cpu().numpy(), rtol=tol,
                                        atol=tol * float(ref.abs().max()))
+
+
+@pytest.mark.parametrize("N,extra", [(704, 3), (769, 4), (768, 67), (700, 70)])
+def test_codon_tip_product_tables_match_oracle(N, extra):
+    """FP32 plans of 61 states large enough for the tips' tables of products: 64 codes and
+    65 (the larger table), 128 codes and 131 (no table), whole and ragged tiles of 128
+    patterns, two tips, one and none below a node.  Tolerances as above."""
+    test_tip_lookups_match_oracle("f32", 61, N, 4, 9, extra)
+
+
+def test_captured_codon_pass_rebuilds_tip_product_tables():
+    """Matrices replaced between a captured large pass and its replay: the tables of tip
+    products follow (the replay runs the same kernels as an eager pass: equal to 1e-12)."""
+    from torchtree_gb300 import synthetic
+    from torchtree_gb300.engine import LikelihoodEngine
+
+    S, T, N, K, b = 61, 11, 800, 4, 9
+    rng = np.random.default_rng(5)
+    codes = rng.integers(0, S + 1, (T, N)).astype(np.uint8)
+    eng = LikelihoodEngine(synthetic.yule_topology(T, rng).postorder, T, S, K, codes, _codes(S, 1, rng), np.ones(N),
+                           batch=b, precision="f32")
+    dev = torch.device("cuda")
+    pd = torch.full((b, K), 1.0 / K, dtype=torch.float64, device=dev)
+    fd = torch.full((b, S), 1.0 / S, dtype=torch.float64, device=dev)
+    mats = [torch.tensor(rng.dirichlet(np.ones(S), size=(b, 2 * T - 2, K, S)), device=dev) for _ in range(2)]
+    eng.set_matrices(mats[0])
+    eng.log_likelihood(pd, fd)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = eng.log_likelihood(pd, fd)
+    eng.set_matrices(mats[1])
+    graph.replay()
+    want = eng.log_likelihood(pd, fd)
+    torch.cuda.synchronize()
+    np.testing.assert_allclose(got.cpu().numpy(), want.cpu().numpy(), rtol=1e-12)

@@ -48,6 +48,10 @@ struct WideState {
   float *d_pimg_f = nullptr;  // the tensor-core post-order's B operands: split P images, same shape
   // the images hold the current transition matrices (written right after them, in one pass)
   bool img_f_valid = false, img_b_valid = false;
+  // tip products of the tensor-core post-order, [b][tips][K][64 or 128 codes][64]: one for either
+  // capacity, allocated with the first tips that need it and kept (a captured pass may hold it);
+  // a plan with more codes, or without the memory, sends its tips through the MMAs
+  float *d_tprod[2] = {nullptr, nullptr};
   // pattern slabs (p->slab != 0): the pattern-sized buffers below hold one
   // slab; tail_valid = they still hold the last slab's post-order (from a
   // tt_log_likelihood with keep_partials), which the gradient then reuses
@@ -187,6 +191,8 @@ struct Wide {
       e = cudaFuncSetAttribute(wide_forward_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                int(cudaSharedmemCarveoutMaxShared));
     if (std::is_same<T, float>::value && SP == 64 && e == cudaSuccess)
+      e = cudaFuncSetAttribute(wide_tip_products_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmem);
+    if (std::is_same<T, float>::value && SP == 64 && e == cudaSuccess)
       e = cudaFuncSetAttribute(wide_backward_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tcb::kSmem);
     if (std::is_same<T, float>::value && SP == 64 && e == cudaSuccess)
       e = cudaFuncSetAttribute(wide_backward_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -259,17 +265,52 @@ struct Wide {
         if (e != cudaSuccess) return e;
       }
     }
+    const float *tprod = nullptr;
+    const int tcodes = p->C <= 64 ? 64 : 128;
+    if constexpr (std::is_same<T, float>::value && SP == 64) {
+      // The tips' products by code, with every pass (a captured one has to follow the matrices).  The
+      // table costs each tip one tile and the pass a launch, and saves the products of all the tip's
+      // tiles.  Post-order of 200 taxa, without and with it: 4 categories, 1 sample, 250 / 510 / 800 /
+      // 1,500 patterns 216, 230 / 273, 273 / 363, 353 / 518, 475 us; 8 samples, 380 / 510 / 800 patterns
+      // 894, 913 / 1,123, 1,108 / 1,835, 1,684 us; 1 category, 1 sample (launch-bound), 800 / 1,500
+      // patterns 210, 214 / 244, 238 us.
+      const int ntf = g.Npad / tc::kPT;
+      if (w.tc && w.d_pimg_f && p->C <= 128 && ntf >= 6 && size_t(p->T) * plan_run_samples(p) * p->K * ntf >= 2048)
+        tprod = w.d_tprod[tcodes / 128];
+      if (tprod) {
+        wide_tip_products_tc_kernel<<<dim3(p->T, plan_run_samples(p) * p->K), tc::kThreads, tc::kSmem, s>>>(
+            a, w.d_pimg_f, tcodes, w.d_tprod[tcodes / 128], p->d_status, 2000000000ull);
+        p->launches += 1;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+      }
+    }
     for (size_t lv = 0; lv + 1 < w.fwd_off.size(); ++lv) {
       a.nodes = w.d_fwd + w.fwd_off[lv];
       if constexpr (std::is_same<T, float>::value && SP == 64) {
         if (w.tc) {  // tiles per CTA by level: about sixteen waves of two CTAs per SM
           const int nodes = w.fwd_off[lv + 1] - w.fwd_off[lv], ntf = g.Npad / tc::kPT;
+          if (lv == 0 && p->I > 1 && tprod) {  // two tips each (and not the root)
+            static_assert(kTipPairThreads == tc::kPT, "the tiles are alike");
+            const size_t sm = tip_pair_smem(tcodes);
+            const cudaError_t e = kernel_smem(wide_tip_pair_kernel, sm, true);
+            if (e != cudaSuccess) return e;
+            const int chunks = tc_level_chunks(nodes, p->batch * p->K, ntf, ntf, 8 * 152 * 5);
+            WideArgs<T> at = a;
+            at.ntiles = ntf;
+            at.tiles_per_chunk = (ntf + chunks - 1) / chunks;
+            wide_tip_pair_kernel<<<dim3(chunks, nodes, plan_run_samples(p) * p->K), kTipPairThreads, sm, s>>>(
+                at, tprod, tcodes);
+            p->launches += 1;
+            continue;
+          }
           const int chunks = tc_level_chunks(nodes, p->batch * p->K, ntf, ntf, 16 * 152 * 2);
           WideArgs<T> at = a;
           at.ntiles = ntf;
           at.tiles_per_chunk = (ntf + chunks - 1) / chunks;
           const dim3 grid(chunks, nodes, plan_run_samples(p) * p->K);
-          wide_forward_tc_kernel<<<grid, tc::kThreads, tc::kSmem, s>>>(at, w.d_pimg_f, p->d_status, 2000000000ull);
+          wide_forward_tc_kernel<<<grid, tc::kThreads, tc::kSmem, s>>>(at, w.d_pimg_f, tprod, tcodes, p->d_status,
+                                                                       2000000000ull);
           p->launches += 1;
           continue;
         }
@@ -666,7 +707,7 @@ void wide_destroy(tt_plan *p) {
   if (!w) return;
   void *bufs[] = {w->d_left, w->d_right, w->d_fwd, w->d_bwd, w->d_branch_lvn, w->d_part, w->d_expo, w->d_root_site, w->d_root_expo,
                   w->d_coef, w->d_cexp, w->d_block_lnl, w->d_gpart, w->d_rootpart, w->d_pgpart, w->d_prod, w->d_site,
-                  w->d_pimg, w->d_pimg_f, w->d_tip_row, w->d_tip_amb};
+                  w->d_pimg, w->d_pimg_f, w->d_tip_row, w->d_tip_amb, w->d_tprod[0], w->d_tprod[1]};
   for (void *x : bufs)
     if (x) cudaFree(x);
   delete w;
@@ -708,6 +749,14 @@ int wide_set_tips(tt_plan *p, const uint8_t *codes, const double *code_table, in
       ++ambs;
     } else {
       ok = false;
+    }
+  }
+  if (p->precision == TT_PRECISION_F32 && SP == 64 && code_count <= 128) {
+    const int cap = code_count <= 64 ? 64 : 128;
+    float *&tprod = w.d_tprod[cap / 128];
+    if (!tprod && walloc(p, &tprod, size_t(p->batch) * p->T * p->K * cap * SP * sizeof(float), "tip products")) {
+      tprod = nullptr;
+      cudaGetLastError();
     }
   }
   rows[256] = ok;

@@ -117,14 +117,132 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 
 }  // namespace tc
 
+// One side's split-TF32 product on the tensor cores, issued by one thread: D (64
+// TMEM columns at d) = A (split, at sA) x B (split, at sB), committed to bar.
+__device__ __forceinline__ void tc_side_mma(uint32_t d, const unsigned char *sA, const unsigned char *sB,
+                                            uint64_t *bar) {
+  constexpr uint32_t idesc = tc::idesc_tf32(128, 64);
+  const uint32_t ab = smem_u32(sA), as = ab + tc::kAbytes;
+  const uint32_t bb = smem_u32(sB), bs = bb + tc::kBbytes;
+#pragma unroll
+  for (int kk = 0; kk < 64 / 8; ++kk) {
+    const uint64_t dab = tc::smem_desc(ab + kk * 4096, 2048, 128), das = tc::smem_desc(as + kk * 4096, 2048, 128);
+    const uint64_t dbb = tc::smem_desc(bb + kk * 2048, 1024, 128), dbs = tc::smem_desc(bs + kk * 2048, 1024, 128);
+    tc::mma_tf32(d, dab, dbb, idesc, kk > 0 ? 1u : 0u);
+    tc::mma_tf32(d, dab, dbs, idesc, 1u);
+    tc::mma_tf32(d, das, dbb, idesc, 1u);
+  }
+  tc::mma_commit(bar);
+}
+
+// this thread's row of the A operand (64 values, split, four per 16-byte store)
+__device__ __forceinline__ void tc_store_a(unsigned char *sA, int row, const float (&xv)[64]) {
+#pragma unroll
+  for (int j = 0; j < 64; j += 4) {
+    float4 hb, hs;
+    tc::split_tf32(xv[j], hb.x, hs.x);
+    tc::split_tf32(xv[j + 1], hb.y, hs.y);
+    tc::split_tf32(xv[j + 2], hb.z, hs.z);
+    tc::split_tf32(xv[j + 3], hb.w, hs.w);
+    const uint32_t off = tc::kmajor_off(row, j, 2048);
+    *reinterpret_cast<float4 *>(sA + off) = hb;
+    *reinterpret_cast<float4 *>(sA + tc::kAbytes + off) = hs;
+  }
+}
+
+// Tip products of a plan with at most 128 tip codes: P_tip times every code's
+// vector, [b][tip][K][codes][64] (codes: the table's capacity, 64 or 128), one MMA
+// tile per (tip, sample, category) with the codes as its rows.  A row of the product depends on its own A row and on B
+// only, so each is, bit for bit, what the post-order's tile of patterns with that
+// code would hold; the post-order reads a tip's products from here and stages and
+// multiplies internal children only.
+__global__ void __launch_bounds__(tc::kThreads, 2)
+    wide_tip_products_tc_kernel(const WideArgs<float> a, const float *pimg, int codes, float *tprod, int *status,
+                                unsigned long long timeout_ns) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  unsigned char *sB = smem + tc::kOffB, *sA = smem + tc::kOffA;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + tc::kOffBar);
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + tc::kOffBar + 8);
+  uint64_t *bar_b = reinterpret_cast<uint64_t *>(smem + tc::kOffBar + 16);
+  const int tid = threadIdx.x, warp = tid >> 5, tip = blockIdx.x;
+  const int b = blockIdx.y / a.K, k = blockIdx.y - (blockIdx.y / a.K) * a.K;
+  if (warp == 0) tc::tmem_alloc(tslot, tc::kTmemCols);
+  if (tid == 0) {
+    mbar_init(bar, 1);
+    mbar_init(bar_b, 1);
+    fence_barrier_init();
+  }
+  float xv[64];
+#pragma unroll
+  for (int j = 0; j < 64; j += 4) {
+    const float4 t4 = tid < codes ? __ldg(reinterpret_cast<const float4 *>(a.table + size_t(tid) * 64 + j))
+                                  : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    xv[j] = t4.x, xv[j + 1] = t4.y, xv[j + 2] = t4.z, xv[j + 3] = t4.w;
+  }
+  tc_store_a(sA, tid, xv);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *tslot;
+  bool landed = true;  // thread 0: the image copy
+  if (tid == 0) {
+    mbar_arrive_expect_tx(bar_b, uint32_t(2 * tc::kBbytes));
+    bulk_copy_g2s(sB, pimg + ((size_t(b) * a.B + tip) * a.K + k) * 2 * 64 * 64, uint32_t(2 * tc::kBbytes), bar_b);
+    landed = mbar_wait_bounded(bar_b, 0, timeout_ns);
+    if (landed) tc_side_mma(tmem, sA, sB, bar);
+    else mbar_arrive(bar);  // no MMAs: complete the phase; the CTA fails below
+  }
+  bool ok = mbar_wait_bounded(bar, 0, timeout_ns) && landed;
+  tc::fence_after_sync();
+  ok = !__syncthreads_or(!ok);
+  if (ok) {
+    const uint32_t lane_addr = tmem + (uint32_t(32 * warp) << 16);
+    float *dst = tprod + (((size_t(b) * a.tips + tip) * a.K + k) * codes + tid) * 64;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float d[32];
+      tc::tmem_ld32(lane_addr + uint32_t(32 * h), d);  // the whole warp
+      if (tid < codes) {
+#pragma unroll
+        for (int i = 0; i < 32; i += 4)
+          *reinterpret_cast<float4 *>(dst + 32 * h + i) = make_float4(d[i], d[i + 1], d[i + 2], d[i + 3]);
+      }
+    }
+  } else {
+    if (tid == 0) {
+      atomicExch(status, kDeviceTimeout);
+      if (!landed) mbar_wait_bounded(bar_b, 0, 100000000ull);  // the image copy lands before exit
+    }
+    mbar_wait_bounded(bar, 0, 100000000ull);  // give the tensor cores a last chance before freeing TMEM
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, tc::kTmemCols);
+}
+
+// 32 consecutive products of a tip's code, from its table row
+__device__ __forceinline__ void tc_tip_row(const float *row, float (&v)[32]) {
+#pragma unroll
+  for (int i = 0; i < 32; i += 4) {
+    const float4 t = __ldg(reinterpret_cast<const float4 *>(row + i));
+    v[i] = t.x, v[i + 1] = t.y, v[i + 2] = t.z, v[i + 3] = t.w;
+  }
+}
+
 // Post-order level kernel for FP32 codon plans on the tensor cores.
 // pimg: split P images (row i, K element j, big then small; wide_pimages_kernel),
 // one 32 KB bulk copy per side; NULL stages P by the
 // threads.  The second side's child values are loaded into registers while
 // the first side's MMAs run.  A CTA walks a.tiles_per_chunk tiles of one
-// (node, sample, category), reusing its TMEM and barriers.
+// (node, sample, category), reusing its TMEM and barriers.  tprod: the tips'
+// products by code (`codes` rows each), or NULL: tips are staged and multiplied
+// as internal children are.  200 taxa x 2,608 patterns x 16 samples (half of all
+// children are tips): 9,960 us -> 6,770 here, 1,380 in the
+// tips-only level (wide_tip_pair_kernel) and 240 for the table.
 __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const WideArgs<float> a, const float *pimg,
-                                                                         int *status, unsigned long long timeout_ns) {
+                                                                         const float *tprod, int codes, int *status,
+                                                                         unsigned long long timeout_ns) {
   constexpr int SP = 64;
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char *sB = smem + tc::kOffB;
@@ -147,17 +265,23 @@ __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const 
     mbar_init(bar_b, 1);
     fence_barrier_init();
   }
+  tc::fence_before_sync();
   __syncthreads();  // barriers initialised before the first copy
+  tc::fence_after_sync();
+  const uint32_t tmem = *tslot;
+  // tips that have a table of products (uniform over the CTA)
+  const float *tab_l = tprod && l < a.tips ? tprod + ((size_t(b) * a.tips + l) * a.K + k) * codes * SP : nullptr;
+  const float *tab_r = tprod && r < a.tips ? tprod + ((size_t(b) * a.tips + r) * a.K + k) * codes * SP : nullptr;
+  const bool two = !tab_l && !tab_r;
   // per side c: stage, then one thread issues the side's MMAs into TMEM
   // columns [64c, 64c + 64); the next side's staging waits for their completion
   bool ok = true;
   int phase = 0, phase_b = 0;
   bool b_pending = false;  // thread 0: an image copy whose completion it has not seen
-  uint32_t tmem = 0;  // read from the slot after the first barrier
   // the A operand values of a side: x_c^T, M = pattern (this thread's), K = j, all 64 loads in
   // flight at once; the second side's are issued while the first side's MMAs run
   float xv[SP];
-  auto load_x = [&](int child) {
+  auto load_x = [&](int child, int n0) {
     if (child < a.tips) {
       const int code = a.codes[size_t(child) * a.code_stride + n0 + tid];
       const float4 *row = reinterpret_cast<const float4 *>(a.table + size_t(code) * SP);
@@ -172,15 +296,18 @@ __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const 
       for (int j = 0; j < SP; ++j) xv[j] = __ldg(src + size_t(j) * a.Npad);
     }
   };
+  if (!tab_l) load_x(l, n0);
+  else if (!tab_r) load_x(r, n0);
   for (int tile = t0; tile < t1 && ok; ++tile) {
     n0 = tile * tc::kPT;
-    load_x(l);
     for (int c = 0; c < 2 && ok; ++c) {
+      if (c ? tab_r : tab_l) continue;
       const int child = c ? r : l;
-      // B operand: P_c[i][j], N = i, K = j: the split image in one bulk copy, or
+      // B operand: P_c[i][j], N = i, K = j: the split image in one bulk copy (which one product
+      // a tile leaves in place), or
       // eight 16-byte loads per thread in flight before the split
       if (pimg) {
-        if (tid == 0) {
+        if (tid == 0 && (tile == t0 || two)) {
           b_pending = true;
           mbar_arrive_expect_tx(bar_b, uint32_t(2 * tc::kBbytes));
           bulk_copy_g2s(sB, pimg + ((size_t(b) * a.B + child) * a.K + k) * 2 * SP * SP, uint32_t(2 * tc::kBbytes),
@@ -207,26 +334,13 @@ __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const 
           *reinterpret_cast<float4 *>(sB + tc::kBbytes + off) = hs;
         }
       }
-      // A operand: the side's loaded values split, four j per 16-byte store
-      {
-#pragma unroll
-        for (int j = 0; j < SP; j += 4) {
-          float4 hb, hs;
-          tc::split_tf32(xv[j], hb.x, hs.x);
-          tc::split_tf32(xv[j + 1], hb.y, hs.y);
-          tc::split_tf32(xv[j + 2], hb.z, hs.z);
-          tc::split_tf32(xv[j + 3], hb.w, hs.w);
-          const uint32_t off = tc::kmajor_off(tid, j, 2048);
-          *reinterpret_cast<float4 *>(sA + off) = hb;
-          *reinterpret_cast<float4 *>(sA + tc::kAbytes + off) = hs;
-        }
-      }
+      // A operand: the side's loaded values split
+      tc_store_a(sA, tid, xv);
       // generic-proxy writes -> visible to the tensor cores (async proxy)
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tc::fence_before_sync();
       __syncthreads();
       tc::fence_after_sync();
-      tmem = *tslot;
       if (tid == 0 && b_pending) {  // the image has landed
         if (mbar_wait_bounded(bar_b, phase_b, timeout_ns)) {
           b_pending = false;
@@ -234,23 +348,11 @@ __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const 
         }
       }
       if (tid == 0 && !b_pending) {
-        constexpr uint32_t idesc = tc::idesc_tf32(128, 64);
-        const uint32_t d = tmem + uint32_t(64 * c);
-        const uint32_t ab = smem_u32(sA), as = ab + tc::kAbytes;
-        const uint32_t bb = smem_u32(sB), bs = bb + tc::kBbytes;
-#pragma unroll
-        for (int kk = 0; kk < SP / 8; ++kk) {
-          const uint64_t dab = tc::smem_desc(ab + kk * 4096, 2048, 128), das = tc::smem_desc(as + kk * 4096, 2048, 128);
-          const uint64_t dbb = tc::smem_desc(bb + kk * 2048, 1024, 128), dbs = tc::smem_desc(bs + kk * 2048, 1024, 128);
-          tc::mma_tf32(d, dab, dbb, idesc, kk > 0 ? 1u : 0u);
-          tc::mma_tf32(d, dab, dbs, idesc, 1u);
-          tc::mma_tf32(d, das, dbb, idesc, 1u);
-        }
-        tc::mma_commit(bar);
+        tc_side_mma(tmem + uint32_t(64 * c), sA, sB, bar);
       } else if (tid == 0) {
         mbar_arrive(bar);  // no MMAs (the image never landed): complete the phase; the side fails below
       }
-      if (c == 0) load_x(r);  // while the MMAs run: the other side's values into registers
+      if (c == 0 && !tab_r) load_x(r, n0);  // while the MMAs run: the other side's values into registers
       // every thread sees the side's MMAs complete before the shared memory is restaged or TMEM read
       ok = mbar_wait_bounded(bar, phase, timeout_ns) && !(tid == 0 && b_pending);
       tc::fence_after_sync();
@@ -258,17 +360,25 @@ __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const 
       if (ok) phase ^= 1;
     }
     if (ok) {
+      if (tile + 1 < t1) {  // the next tile's first values travel during this one's epilogue
+        if (!tab_l) load_x(l, n0 + tc::kPT);
+        else if (!tab_r) load_x(r, n0 + tc::kPT);
+      }
       // this thread's pattern = TMEM lane 32 * warp + lane
       const uint32_t lane_addr = tmem + (uint32_t(32 * warp) << 16);
       const int n = n0 + tid;
       float *pd = a.prod ? a.prod + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * 2 * SP * size_t(a.Npad) + n
                          : nullptr;
+      const float *row_l = tab_l ? tab_l + min(int(a.codes[size_t(l) * a.code_stride + n]), codes - 1) * SP : nullptr;
+      const float *row_r = tab_r ? tab_r + min(int(a.codes[size_t(r) * a.code_stride + n]), codes - 1) * SP : nullptr;
       float L[64];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         float dl[32], dr[32];
-        tc::tmem_ld32(lane_addr + uint32_t(32 * h), dl);
-        tc::tmem_ld32(lane_addr + uint32_t(64 + 32 * h), dr);
+        if (tab_l) tc_tip_row(row_l + 32 * h, dl);
+        else tc::tmem_ld32(lane_addr + uint32_t(32 * h), dl);
+        if (tab_r) tc_tip_row(row_r + 32 * h, dr);
+        else tc::tmem_ld32(lane_addr + uint32_t(64 + 32 * h), dr);
         if (pd) {  // the children's products for the adjoint
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -315,6 +425,62 @@ __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const 
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, tc::kTmemCols);
+}
+
+// Post-order of nodes whose children are both tips with product tables (the lowest
+// level): no matrix product is left, so a CTA of no tensor memory and 34 KB holds
+// the two tables (rows 68 floats apart, which spreads the lanes' rows over the
+// banks) and every thread joins a pattern's two rows.  Bound by the stores of the
+// partials and of the products the adjoint reads.  67 such nodes of 200 taxa x 2,608
+// patterns x 16 samples: 1,920 us in the kernel above, 1,380 here.
+constexpr int kTipPairThreads = 128, kTipPairStride = 68;
+
+inline size_t tip_pair_smem(int codes) { return size_t(2) * codes * kTipPairStride * sizeof(float); }
+
+__global__ void __launch_bounds__(kTipPairThreads) wide_tip_pair_kernel(const WideArgs<float> a, const float *tprod,
+                                                                        int codes) {
+  constexpr int SP = 64, ST = kTipPairStride;
+  extern __shared__ __align__(128) unsigned char smem[];
+  float *tab = reinterpret_cast<float *>(smem);  // [2][codes][ST]
+  const int tid = threadIdx.x, v = a.nodes[blockIdx.y];
+  const int b = blockIdx.z / a.K, k = blockIdx.z - (blockIdx.z / a.K) * a.K;
+  const int l = a.left[v - a.tips], r = a.right[v - a.tips];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const float4 *src =
+        reinterpret_cast<const float4 *>(tprod + ((size_t(b) * a.tips + (c ? r : l)) * a.K + k) * codes * SP);
+    for (int e = tid; e < codes * (SP / 4); e += kTipPairThreads)
+      *reinterpret_cast<float4 *>(tab + (c * codes + e / (SP / 4)) * ST + e % (SP / 4) * 4) = __ldg(src + e);
+  }
+  __syncthreads();
+  const size_t npad = size_t(a.Npad), blk = (size_t(b) * a.I + (v - a.tips)) * a.K + k;
+  const int t0 = blockIdx.x * a.tiles_per_chunk, t1 = min(a.ntiles, t0 + a.tiles_per_chunk);
+  for (int tile = t0; tile < t1; ++tile) {
+    const int n = tile * kTipPairThreads + tid;
+    const float *row_l = tab + min(int(a.codes[size_t(l) * a.code_stride + n]), codes - 1) * ST;
+    const float *row_r = tab + (codes + min(int(a.codes[size_t(r) * a.code_stride + n]), codes - 1)) * ST;
+    float *pd = a.prod ? a.prod + blk * 2 * SP * npad + n : nullptr;
+    float L[SP], m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < SP; i += 4) {
+      const float4 x = *reinterpret_cast<const float4 *>(row_l + i), y = *reinterpret_cast<const float4 *>(row_r + i);
+      const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        if (pd) {
+          pd[(i + t) * npad] = xs[t];
+          pd[(SP + i + t) * npad] = ys[t];
+        }
+        L[i + t] = xs[t] * ys[t];
+        m = fmaxf(m, L[i + t]);
+      }
+    }
+    const int e = a.rescale ? scale_exponent(m) : 0;
+    float *dst = a.part + blk * SP * npad + n;
+#pragma unroll
+    for (int i = 0; i < SP; ++i) dst[i * npad] = times_pow2_neg(L[i], e);
+    a.expo[blk * npad + n] = e;
+  }
 }
 
 }  // namespace tt
