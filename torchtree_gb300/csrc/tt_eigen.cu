@@ -12,7 +12,7 @@
 // FP64 arithmetic is scarce on this GPU (a few FP64 FMAs per cycle per SM),
 // so the solver does most of its sweeps in FP32 and spreads the FP64 matrix
 // products over many CTAs:
-//  1. eigen_start_kernel, one CTA per matrix: cyclic Jacobi in FP32 (parallel
+//  1. eigen_start_kernel, one or four CTAs per matrix: cyclic Jacobi in FP32 (parallel
 //     round-robin ordering of Brent and Luk, 1985; each rotation Golub & Van
 //     Loan, Algorithm 8.4.2 "sym.schur2"): eigenvectors X0 good to ~1e-5;
 //  2. two Newton-Schulz steps X <- X (3I - X^T X) / 2 (Higham, "Functions of
@@ -20,7 +20,7 @@
 //     (eigen_gram_kernel forms R = I - X^T X, eigen_orth_kernel X <- X + X R/2),
 //     kEigRows rows of the products per CTA;
 //  3. eigen_gram_kernel forms S = X^T A X (off-diagonal ~1e-5 of its norm) and
-//     eigen_finish_kernel, one CTA per matrix, diagonalises S by FP64 Jacobi
+//     eigen_finish_kernel, one or eight CTAs per matrix, diagonalises S by FP64 Jacobi
 //     sweeps accumulated into X (quadratic convergence from there: two or
 //     three sweeps) to 1e-14 of the Frobenius norm.
 // A matrix whose FP64 sweeps do not converge (30 of them) sets the status
@@ -54,8 +54,8 @@ __device__ __forceinline__ void rr_pair(int r, int i, int m, int &p, int &q) {
     p = r;
     q = m - 1;
   } else {
-    p = (r + i) % (m - 1);
-    q = (r - i + (m - 1)) % (m - 1);
+    p = r + i < m - 1 ? r + i : r + i - (m - 1);
+    q = r >= i ? r - i : r - i + (m - 1);
   }
   if (p > q) {
     const int t = p;
@@ -87,7 +87,7 @@ __device__ __forceinline__ void jacobi_rotation_f64(double app, double aqq, doub
   s = t * y;
 }
 
-// Cyclic Jacobi sweeps on A (n x n, leading dimension kEigLd) accumulating
+// Cyclic Jacobi sweeps on A (n x n, leading dimension NMAX + 1) accumulating
 // the rotations into V, in T arithmetic, until the off-diagonal norm squared
 // is at most tol2 times the Frobenius norm squared; true when converged within
 // max_sweeps.  cs and pq hold a round's rotations and pairs.  Called by the
@@ -243,25 +243,202 @@ __device__ void load_symmetrised(const double *q, const double *pi, int b, int n
   __syncthreads();
 }
 
-// Step 1, one CTA per matrix: FP32 Jacobi sweeps on A until the off-diagonal
-// norm is below 1e-6 of the Frobenius norm (at most 6 sweeps: FP32 rounding
-// may stop short of that); the eigenvector matrix X0, in FP64, into x.
-__global__ void __launch_bounds__(kEigThreads) eigen_start_kernel(const double *q, const double *pi, int n,
-                                                                  double *x) {
-  constexpr int NW = kEigThreads / 32;
-  __shared__ float A[kEigMax * kEigLd], V[kEigMax * kEigLd], cs[kEigMax];
-  __shared__ int pq[kEigMax];
-  __shared__ double red[2 * NW], sq[kEigMax];
-  __shared__ int flag;
-  const int b = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  load_symmetrised(q, pi, b, n, sq, A);
-  for (int i = warp; i < n; i += NW)
-    for (int j = lane; j < n; j += 32) V[i * kEigLd + j] = i == j ? 1.0f : 0.0f;
-  __syncthreads();
-  jacobi_sweeps<float>(A, V, cs, pq, red, &flag, n, 1e-12, 6);
+// A round of the sweeps below, of m players (m even): pair i is player a = r + i and
+// player b = r - i mod m - 1, pair 0 player r and player m - 1; p < q are the two.
+// advance() goes to the next round.
+struct EigPair {
+  int a, b, p, q;
+  __device__ __forceinline__ EigPair() : a(0), b(0), p(0), q(0) {}
+  __device__ __forceinline__ EigPair(int i, int m) : a(i), b(i ? m - 1 - i : m - 1) { sort(); }
+  __device__ __forceinline__ void sort() {
+    p = min(a, b);
+    q = max(a, b);
+  }
+  __device__ __forceinline__ void advance(int i, int m) {
+    a = a + 1 == m - 1 ? 0 : a + 1;
+    if (i) b = b + 1 == m - 1 ? 0 : b + 1;
+    sort();
+  }
+};
+// offset of element (u, v) of a symmetric matrix held in its upper triangle
+template <int LD>
+__device__ __forceinline__ int eig_at(int u, int v) {
+  return min(u, v) * LD + max(u, v);
+}
+
+// (u, v) <- (c u - s v, s u + c v), rounded alike wherever it is inlined: a matrix's
+// system does not depend on the number of CTAs
+__device__ __forceinline__ void eig_mix(float2 cs, float &u, float &v) {
+  const float a = __fmaf_rn(cs.x, u, -__fmul_rn(cs.y, v)), b = __fmaf_rn(cs.y, u, __fmul_rn(cs.x, v));
+  u = a;
+  v = b;
+}
+
+// Step 1, a cluster of C CTAs per matrix: FP32 Jacobi sweeps on A until the
+// off-diagonal norm is below 1e-6 of the Frobenius norm (at most kEigStartSweeps:
+// FP32 rounding may stop short of that); the eigenvector matrix X0, in FP64, into
+// x.  The first CTA rotates A alone: of the blocks of four elements that two
+// rotations of a round mix, a thread holds one or two (rows first, columns then;
+// each element belongs to one block, so a round takes two barriers and one pass over
+// A), and every CTA's shared memory is given the rotations.  A row of X0 is the unit
+// row under all the rotations, whatever the other rows do: afterwards each warp
+// carries its rows through them in registers, a pair per lane, the players moving
+// from lane to lane as the round-robin does.  Bound by the latency of a round (the
+// rotation's divisions and roots, two barriers).  61 states, 6 x 61 rounds: 534 us
+// with separate passes over rows and columns and X0 rotated along, 336 us so;
+// 20 states 119 -> 64 us, the same rotations and bits.
+constexpr int kEigStartSweeps = 6;
+
+template <int NMAX>
+constexpr int eig_start_threads() { return NMAX == 64 ? 512 : 256; }
+template <int NMAX>
+constexpr size_t eig_start_smem() {  // A, this round's rotations, all rounds' rotations
+  return (size_t(NMAX) * (NMAX + 1) + 2 * size_t(kEigStartSweeps) * (NMAX - 1) * (NMAX / 2)) * sizeof(float);
+}
+
+template <int NMAX, int C>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(eig_start_threads<NMAX>())
+    eigen_start_kernel(const double *q, const double *pi, int n, double *x) {
+  namespace cg = cooperative_groups;
+  constexpr int NT = eig_start_threads<NMAX>(), NW = NT / 32, LD = NMAX + 1, H = NMAX / 2;
+  constexpr int RPW = (NMAX + C * NW - 1) / (C * NW);  // rows of X0 per warp
+  constexpr int BPT = H * H / NT;                      // blocks per thread
+  extern __shared__ __align__(16) float esm[];
+  float2 *log = reinterpret_cast<float2 *>(esm);                  // [round][npairs] (c, s)
+  float *A = esm + 2 * kEigStartSweeps * (NMAX - 1) * H;          // [n + 1][LD], a zero dummy player
+  __shared__ double red[2 * NW], sq[NMAX];
+  __shared__ int flag, rounds;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = C > 1 ? int(cluster.block_rank()) : 0;
+  const int b = blockIdx.x / C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m = n + (n & 1), npairs = m / 2;
+  if constexpr (C > 1) cluster.sync();  // every CTA runs before the first one writes to it
+  if (rank == 0) {
+    load_symmetrised<float, NMAX, NT>(q, pi, b, n, sq, A);
+    if (n < m)
+      for (int k = tid; k < m; k += NT) A[n * LD + k] = A[k * LD + n] = 0.0f;
+    // this thread's blocks: a pair of columns, BPT pairs of rows
+    const int bj = tid % H, bi = tid / H;
+    EigPair pj(min(bj, npairs - 1), m), pr[BPT];
+#pragma unroll
+    for (int k = 0; k < BPT; ++k) pr[k] = EigPair(min(bi + k * (NT / H), npairs - 1), m);
+    __syncthreads();
+    int done = 0;
+    for (int sweep = 0; sweep <= kEigStartSweeps; ++sweep) {
+      double off = 0.0, tot = 0.0;
+      for (int i = warp; i < n; i += NW)
+        for (int j = lane; j < n; j += 32) {
+          const double v = double(A[i * LD + j]);
+          tot += v * v;
+          if (i != j) off += v * v;
+        }
+      for (int o = 16; o; o >>= 1) {
+        off += __shfl_xor_sync(0xffffffffu, off, o);
+        tot += __shfl_xor_sync(0xffffffffu, tot, o);
+      }
+      if (lane == 0) {
+        red[warp] = off;
+        red[NW + warp] = tot;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        double so = 0.0, st = 0.0;
+        for (int w = 0; w < NW; ++w) {
+          so += red[w];
+          st += red[NW + w];
+        }
+        flag = !(so > 1e-12 * st);
+      }
+      __syncthreads();
+      if (flag || sweep == kEigStartSweeps) break;
+      for (int r = 0; r < m - 1; ++r, ++done) {
+        if (tid < npairs) {  // this round's rotations
+          const float apq = A[pj.p * LD + pj.q];
+          float c = 1.0f, sn = 0.0f;
+          if (apq != 0.0f) {
+            const float tau = (A[pj.q * (LD + 1)] - A[pj.p * (LD + 1)]) / (2.0f * apq);
+            float t;
+            if (fabsf(tau) > 1e18f) t = 0.5f / tau;
+            else t = (tau >= 0.0f ? 1.0f : -1.0f) / (fabsf(tau) + sqrtf(__fmaf_rn(tau, tau, 1.0f)));
+            c = 1.0f / sqrtf(__fmaf_rn(t, t, 1.0f));
+            sn = t * c;
+          }
+          const float2 cs = make_float2(c, sn);
+          log[done * npairs + tid] = cs;
+#pragma unroll
+          for (int o = 1; o < C; ++o) cluster.map_shared_rank(log, o)[done * npairs + tid] = cs;
+        }
+        __syncthreads();
+        if (bj < npairs) {
+          const float2 rj = log[done * npairs + bj];
+#pragma unroll
+          for (int k = 0; k < BPT; ++k) {
+            const int i = bi + k * (NT / H);
+            if (i >= npairs) continue;
+            const float2 ri = log[done * npairs + i];
+            float *Ap = A + pr[k].p * LD, *Aq = A + pr[k].q * LD;
+            float a0 = Ap[pj.p], a1 = Ap[pj.q], b0 = Aq[pj.p], b1 = Aq[pj.q];
+            eig_mix(ri, a0, b0);  // rows
+            eig_mix(ri, a1, b1);
+            eig_mix(rj, a0, a1);  // columns
+            eig_mix(rj, b0, b1);
+            Ap[pj.p] = a0;
+            Ap[pj.q] = a1;
+            Aq[pj.p] = b0;
+            Aq[pj.q] = b1;
+            pr[k].advance(i, m);
+          }
+        }
+        pj.advance(bj, m);
+        __syncthreads();
+      }
+    }
+    if (tid == 0) {
+      rounds = done;
+#pragma unroll
+      for (int o = 1; o < C; ++o) *cluster.map_shared_rank(&rounds, o) = done;
+    }
+  }
+  if constexpr (C > 1) cluster.sync();
+  else __syncthreads();
+  // rows of X0: lane i carries the columns of pair i
+  const int total = rounds, last = npairs - 1;
+  EigPair at(lane, m);
+  const int row0 = (rank * NW + warp) * RPW;
+  if (row0 >= n) return;  // a whole warp; nothing reaches into this CTA any more
+  float va[RPW], vb[RPW];
+#pragma unroll
+  for (int k = 0; k < RPW; ++k) {
+    va[k] = lane <= last && at.a == row0 + k ? 1.0f : 0.0f;
+    vb[k] = lane <= last && at.b == row0 + k ? 1.0f : 0.0f;
+  }
+  const float2 *cs = log + min(lane, last);
+  for (int d = 0; d < total; ++d, cs += npairs) {
+    const float2 rot = *cs;
+    const bool swap = at.a > at.b;
+#pragma unroll
+    for (int k = 0; k < RPW; ++k) {
+      float vp = swap ? vb[k] : va[k], vq = swap ? va[k] : vb[k];
+      eig_mix(rot, vp, vq);
+      const float na = swap ? vq : vp, nb = swap ? vp : vq;
+      // the next round's pairs: p from the lane above (the last lane's is its q), q from the lane
+      // below (lane 1's is lane 0's p); player m - 1 stays in lane 0
+      const float da = __shfl_down_sync(0xffffffffu, na, 1);
+      const float ub = __shfl_up_sync(0xffffffffu, lane == 0 ? na : nb, 1);
+      va[k] = lane == last ? nb : da;
+      vb[k] = lane == 0 ? nb : ub;
+    }
+    at.advance(lane, m);
+  }
   double *xb = x + size_t(b) * n * n;
-  for (int i = warp; i < n; i += NW)
-    for (int j = lane; j < n; j += 32) xb[i * n + j] = double(V[i * kEigLd + j]);
+  if (lane <= last) {
+#pragma unroll
+    for (int k = 0; k < RPW; ++k)
+      if (row0 + k < n) {
+        xb[(row0 + k) * n + at.a] = double(va[k]);
+        if (at.b < n) xb[(row0 + k) * n + at.b] = double(vb[k]);
+      }
+  }
 }
 
 // Step 2 / 3, kEigRows rows per CTA (grid: row blocks x matrices), FP64: for
@@ -346,96 +523,81 @@ __global__ void __launch_bounds__(kEigThreads) eigen_orth_kernel(int n, double *
   }
 }
 
-// Step 3, one CTA per matrix, FP64: S = X^T A X (in W, upper triangle) and X
-// (in U); FP64 Jacobi sweeps on S, accumulated into X, to 1e-14 of the
-// Frobenius norm; a matrix that does not converge in 30 sweeps sets the
-// status word.  Eigenvalues ascending, with U = Pi^-1/2 X and W = X^T Pi^1/2.
-__global__ void __launch_bounds__(kEigThreads) eigen_finish_kernel(const double *pi, int n, double *lam, double *U,
-                                                                   double *W, int *status) {
-  constexpr int NW = kEigThreads / 32;
-  extern __shared__ __align__(16) double fsm[];
-  double *A = fsm;                       // [n][kEigLd] S, symmetric
-  double *V = A + kEigMax * kEigLd;      // [n][kEigLd] X
-  double *cs = V + kEigMax * kEigLd;     // [kEigMax/2][2]
-  double *red = cs + kEigMax;            // [2 * NW]
-  double *sq = red + 2 * NW;             // [n]
-  int *pq = reinterpret_cast<int *>(sq + kEigMax);  // [kEigMax/2][2]
-  __shared__ int flag;
-  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const size_t mo = size_t(b) * n * n;
-  for (int i = tid; i < n; i += kEigThreads) sq[i] = sqrt(pi[size_t(b) * n + i]);
-  for (int i = warp; i < n; i += NW)
-    for (int j = lane; j < n; j += 32) {
-      A[i * kEigLd + j] = W[mo + size_t(min(i, j)) * n + max(i, j)];
-      V[i * kEigLd + j] = U[mo + size_t(i) * n + j];
-    }
-  __syncthreads();
-  // (every thread's reads of U and W are done: the sweeps begin with a barrier)
-  const bool ok = jacobi_sweeps<double>(A, V, cs, pq, red, &flag, n, 1e-28, 30);
-  if (tid == 0 && !ok) atomicExch(status, TT_ERR_UNSUPPORTED);
-  // ascending order: the rank of each eigenvalue (ties by index)
-  for (int k = tid; k < n; k += kEigThreads) {
-    const double lk = A[k * kEigLd + k];
-    int rank = 0;
-    for (int j = 0; j < n; ++j) {
-      const double lj = A[j * kEigLd + j];
-      rank += lj < lk || (lj == lk && j < k);
-    }
-    lam[size_t(b) * n + rank] = lk;
-    for (int i = 0; i < n; ++i) {
-      U[(size_t(b) * n + i) * n + rank] = V[i * kEigLd + k] / sq[i];  // U = Pi^-1/2 V
-      W[(size_t(b) * n + rank) * n + i] = V[i * kEigLd + k] * sq[i];  // W = V^T Pi^1/2
-    }
-  }
+// Step 3, a cluster of C CTAs per matrix, FP64: S = X^T A X (in W, upper
+// triangle) and X (in U); FP64 Jacobi sweeps on S, accumulated into X, to 1e-14 of
+// the Frobenius norm; a matrix that does not converge in 30 sweeps sets the status
+// word.  Eigenvalues ascending, with U = Pi^-1/2 X and W = X^T Pi^1/2.
+// Every CTA keeps a copy of A's upper triangle, in two buffers.  A round: every CTA
+// forms the same rotations from its copy; of the blocks of four elements that two
+// rotations mix, each CTA updates its share, two threads a block, a row of it each,
+// rows first and columns then, and writes the results into every CTA's other buffer
+// through distributed shared memory (consecutive lanes along a row: the stores that
+// coalesce; the rotations of a round read the buffer that nobody writes); while they
+// travel it rotates its own rows of X.  One cluster barrier a round.  Bound by FP64
+// latency and arithmetic (64 cycles per warp instruction and SM quarter).  61 states:
+// 1 matrix 528 -> 352 us, 16 matrices 531 -> 431 us, against 4 CTAs with full copies
+// and rows and columns in separate passes.  Up to 32 states one CTA (20 states:
+// 216 -> 83 us).
+constexpr int kEigCluster = 8;
+
+template <int NMAX, int C>
+constexpr size_t eig_finish_smem() {  // A twice, rows of X, rotations twice, sqrt(pi)
+  return (2 * size_t(NMAX) * (NMAX + 1) + size_t((NMAX + C - 1) / C) * (NMAX + 1) + 2 * NMAX + NMAX) *
+         sizeof(double);
 }
 
-// Step 3 for matrices of more than 32 states: the same FP64 Jacobi sweeps on
-// a cluster of kEigCluster CTAs per matrix (FP64 arithmetic on one SM bounds
-// the single-CTA sweeps).  Every CTA keeps a copy of A; each round, all CTAs
-// form the same rotations from their identical copies, a CTA updates the rows
-// p, q of its share of the pairs (pairs i = rank mod kEigCluster) and writes
-// them into every copy through distributed shared memory, then, after a
-// cluster barrier, updates columns p, q of its share of the rows (rows = rank
-// mod kEigCluster) in every copy of A and in its own rows of V.  The
-// convergence test runs on each CTA's (identical) copy, so every CTA leaves
-// the sweeps together.  Each CTA writes its rows of U and W.
-constexpr int kEigCluster = 4;
-
-__global__ void __cluster_dims__(kEigCluster, 1, 1) __launch_bounds__(kEigThreads)
-    eigen_finish_cluster_kernel(const double *pi, int n, double *lam, double *U, double *W, int *status) {
+template <int NMAX, int C>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kEigThreads)
+    eigen_finish_kernel(const double *pi, int n, double *lam, double *U, double *W, int *status) {
   namespace cg = cooperative_groups;
-  constexpr int NW = kEigThreads / 32, C = kEigCluster;
-  extern __shared__ __align__(16) double csm[];
-  double *A = csm;                       // [n][kEigLd] S, symmetric (a copy per CTA)
-  double *V = A + kEigMax * kEigLd;      // [n][kEigLd] X (rows = rank mod C are this CTA's)
-  double *cs = V + kEigMax * kEigLd;     // [kEigMax/2][2]
-  double *red = cs + kEigMax;            // [2 * NW]
-  double *sq = red + 2 * NW;             // [n]
-  int *pq = reinterpret_cast<int *>(sq + kEigMax);  // [kEigMax/2][2]
+  constexpr int NT = kEigThreads, NW = NT / 32, LD = NMAX + 1, H = NMAX / 2, BUF = NMAX * LD;
+  constexpr int NB = ((H * (H + 1) / 2 + C - 1) / C + 31) / 32 * 32;  // this CTA's blocks, at most
+  constexpr int HB = (2 * NB + NT - 1) / NT;                          // half blocks per thread
+  extern __shared__ __align__(16) double fsm[];
+  double *A = fsm;                                        // [2][n + 1][LD]
+  double *V = A + 2 * BUF;                                // [rows][LD]: rows = rank mod C of X
+  double2 *cs = reinterpret_cast<double2 *>(V + (NMAX + C - 1) / C * LD + ((NMAX + C - 1) / C * LD & 1));
+  double *sq = reinterpret_cast<double *>(cs + 2 * H);    // [n]
+  __shared__ double red[2 * NW];
   __shared__ int flag;
   cg::cluster_group cluster = cg::this_cluster();
-  const int rank = int(cluster.block_rank());
+  const int rank = C > 1 ? int(cluster.block_rank()) : 0;
   const int b = blockIdx.x / C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double *Ac[C];
-#pragma unroll
-  for (int q = 0; q < C; ++q) Ac[q] = cluster.map_shared_rank(A, q);
-  const size_t mo = size_t(b) * n * n;
-  for (int i = tid; i < n; i += kEigThreads) sq[i] = sqrt(pi[size_t(b) * n + i]);
-  for (int i = warp; i < n; i += NW)
-    for (int j = lane; j < n; j += 32) {
-      A[i * kEigLd + j] = W[mo + size_t(min(i, j)) * n + max(i, j)];
-      if (i % C == rank) V[i * kEigLd + j] = U[mo + size_t(i) * n + j];
-    }
-  cluster.sync();  // every CTA has read U and W before any writes its outputs
   const int m = n + (n & 1), npairs = m / 2;
+  const size_t mo = size_t(b) * n * n;
+  for (int i = tid; i < n; i += NT) sq[i] = sqrt(pi[size_t(b) * n + i]);
+  for (int i = warp; i < m; i += NW)
+    for (int j = lane; j < m; j += 32) {
+      if (i <= j) A[i * LD + j] = j < n ? W[mo + size_t(i) * n + j] : 0.0;  // a dummy player of zeros
+      if (i % C == rank) V[i / C * LD + j] = i < n && j < n ? U[mo + size_t(i) * n + j] : 0.0;
+    }
+  if constexpr (C > 1) cluster.sync();  // every CTA has read U and W before any writes its outputs
+  else __syncthreads();
+  // this thread's half blocks, pairs i <= j and which row of pair i, and its lane's pair
+  int hi[HB], hj[HB];
+  const int blocks = npairs * (npairs + 1) / 2, share = (blocks + C - 1) / C;
+  EigPair row_pair(tid % H, m), pi_[HB], pj[HB];
+#pragma unroll
+  for (int k = 0; k < HB; ++k) {
+    const int h = tid + k * NT, at = h < NB ? h : h - NB;  // a warp's lanes along a row of the second pair
+    int e = rank * share + at, i = 0;
+    hi[k] = hj[k] = -1;
+    if (h >= 2 * NB || at >= share || e >= blocks) continue;
+    while (e >= npairs - i) e -= npairs - i, ++i;
+    hi[k] = i;
+    hj[k] = i + e;
+    pi_[k] = EigPair(hi[k], m);
+    pj[k] = EigPair(hj[k], m);
+  }
+  double *cur = A, *nxt = A + BUF;
   bool ok = false;
   for (int sweep = 0; sweep <= 30; ++sweep) {
     double off = 0.0, tot = 0.0;
     for (int i = warp; i < n; i += NW)
-      for (int j = lane; j < n; j += 32) {
-        const double v = A[i * kEigLd + j];
-        tot += v * v;
-        if (i != j) off += v * v;
+      for (int j = i + lane; j < n; j += 32) {
+        const double v = cur[i * LD + j];
+        if (i != j) off = fma(v, v, off);
+        else tot = fma(v, v, tot);
       }
     for (int o = 16; o; o >>= 1) {
       off += __shfl_xor_sync(0xffffffffu, off, o);
@@ -449,10 +611,10 @@ __global__ void __cluster_dims__(kEigCluster, 1, 1) __launch_bounds__(kEigThread
     if (tid == 0) {
       double so = 0.0, st = 0.0;
       for (int w = 0; w < NW; ++w) {
-        so += red[w];
+        so += 2.0 * red[w];
         st += red[NW + w];
       }
-      flag = !(so > 1e-28 * st) || n == 1;
+      flag = !(so > 1e-28 * (st + so));
     }
     __syncthreads();
     if (flag) {
@@ -461,80 +623,73 @@ __global__ void __cluster_dims__(kEigCluster, 1, 1) __launch_bounds__(kEigThread
     }
     if (sweep == 30) break;
     for (int r = 0; r < m - 1; ++r) {
+      double2 *rot = cs + (r & 1) * H;  // the last round's may still be read
       if (tid < npairs) {  // the round's rotations, the same in every CTA
-        int p, qq;
-        rr_pair(r, tid, m, p, qq);
-        double c = 1.0, sn = 0.0;
-        if (qq < n) jacobi_rotation_f64(A[p * kEigLd + p], A[qq * kEigLd + qq], A[p * kEigLd + qq], c, sn);
-        cs[2 * tid] = c;
-        cs[2 * tid + 1] = sn;
-        pq[2 * tid] = p;
-        pq[2 * tid + 1] = qq;
+        double c, sn;
+        jacobi_rotation_f64(cur[row_pair.p * (LD + 1)], cur[row_pair.q * (LD + 1)],
+                            cur[row_pair.p * LD + row_pair.q], c, sn);
+        rot[tid] = make_double2(c, sn);
       }
       __syncthreads();
-      // rows p, q of this CTA's pairs (a warp per pair), into every copy
-      for (int i = rank + C * warp; i < npairs; i += C * NW) {
-        const int p = pq[2 * i], qq = pq[2 * i + 1];
-        const double c = cs[2 * i], sn = cs[2 * i + 1];
-        if (qq >= n || sn == 0.0) continue;
-        double np_[2], nq_[2];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int j = lane + 32 * h;
-          const double ap = j < n ? A[p * kEigLd + j] : 0.0, aq = j < n ? A[qq * kEigLd + j] : 0.0;
-          np_[h] = c * ap - sn * aq;
-          nq_[h] = sn * ap + c * aq;
+      for (int k = 0; k < HB; ++k) {
+        if (hi[k] < 0) continue;
+        const double2 ri = rot[hi[k]], rj = rot[hj[k]];
+        const bool second = tid + k * NT >= NB, diag = hi[k] == hj[k];
+        const int own = second ? pi_[k].q : pi_[k].p;
+        const int o0 = eig_at<LD>(own, pj[k].p), o1 = eig_at<LD>(own, pj[k].q);
+        const double app = cur[eig_at<LD>(pi_[k].p, pj[k].p)], apq = cur[eig_at<LD>(pi_[k].p, pj[k].q)];
+        const double aqp = cur[eig_at<LD>(pi_[k].q, pj[k].p)], aqq = cur[eig_at<LD>(pi_[k].q, pj[k].q)];
+        pi_[k].advance(hi[k], m);
+        pj[k].advance(hj[k], m);
+        // the row of pair i: c p - s q, or s p + c q
+        const double u = second ? ri.y : ri.x, w = second ? ri.x : -ri.y;
+        const double x0 = u * app + w * aqp, x1 = u * apq + w * aqq;
+        const double n0 = rj.x * x0 - rj.y * x1, n1 = rj.y * x0 + rj.x * x1;
+        const int base = int(nxt - A);
+#pragma unroll
+        for (int o = 0; o < C; ++o) {
+          double *dst = C > 1 ? cluster.map_shared_rank(A, o) + base : nxt;
+          if (!(diag && second)) dst[o0] = n0;  // (q, p) is (p, q)
+          dst[o1] = n1;
         }
-#pragma unroll
-        for (int q = 0; q < C; ++q)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int j = lane + 32 * h;
-            if (j < n) {
-              Ac[q][p * kEigLd + j] = np_[h];
-              Ac[q][qq * kEigLd + j] = nq_[h];
-            }
-          }
       }
-      cluster.sync();
-      // columns p, q of this CTA's rows (a warp per row, lanes over the pairs), into every copy of
-      // A and this CTA's rows of V
-      for (int row = rank + C * warp; row < n; row += C * NW) {
-        const int i = lane;
-        if (i >= npairs) continue;
-        const int p = pq[2 * i], qq = pq[2 * i + 1];
-        const double c = cs[2 * i], sn = cs[2 * i + 1];
-        if (qq >= n || sn == 0.0) continue;
-        const double ap = A[row * kEigLd + p], aq = A[row * kEigLd + qq];
-        const double np_ = c * ap - sn * aq, nq_ = sn * ap + c * aq;
-#pragma unroll
-        for (int q = 0; q < C; ++q) {
-          Ac[q][row * kEigLd + p] = np_;
-          Ac[q][row * kEigLd + qq] = nq_;
+      __syncwarp();
+      if constexpr (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      // this CTA's rows of X, lanes over the pairs
+      if (tid % H < npairs) {
+        const double2 rl = rot[tid % H];
+        for (int row = tid / H; row * C + rank < n; row += NT / H) {
+          const double vp = V[row * LD + row_pair.p], vq = V[row * LD + row_pair.q];
+          V[row * LD + row_pair.p] = rl.x * vp - rl.y * vq;
+          V[row * LD + row_pair.q] = rl.y * vp + rl.x * vq;
         }
-        const double vp = V[row * kEigLd + p], vq = V[row * kEigLd + qq];
-        V[row * kEigLd + p] = c * vp - sn * vq;
-        V[row * kEigLd + qq] = sn * vp + c * vq;
       }
-      cluster.sync();
+      row_pair.advance(tid % H, m);
+      __syncwarp();
+      if constexpr (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      else __syncthreads();
+      double *t = cur;
+      cur = nxt;
+      nxt = t;
     }
   }
   if (tid == 0 && rank == 0 && !ok) atomicExch(status, TT_ERR_UNSUPPORTED);
+  __syncthreads();
   // ascending order: the rank of each eigenvalue (ties by index); this CTA's rows of U and W
-  for (int k = tid; k < n; k += kEigThreads) {
-    const double lk = A[k * kEigLd + k];
+  for (int k = tid; k < n; k += NT) {
+    const double lk = cur[k * LD + k];
     int rk = 0;
     for (int j = 0; j < n; ++j) {
-      const double lj = A[j * kEigLd + j];
+      const double lj = cur[j * LD + j];
       rk += lj < lk || (lj == lk && j < k);
     }
     if (rank == 0) lam[size_t(b) * n + rk] = lk;
     for (int i = rank; i < n; i += C) {
-      U[(size_t(b) * n + i) * n + rk] = V[i * kEigLd + k] / sq[i];  // U = Pi^-1/2 V
-      W[(size_t(b) * n + rk) * n + i] = V[i * kEigLd + k] * sq[i];  // W = V^T Pi^1/2
+      U[(size_t(b) * n + i) * n + rk] = V[i / C * LD + k] / sq[i];  // U = Pi^-1/2 V
+      W[(size_t(b) * n + rk) * n + i] = V[i / C * LD + k] * sq[i];  // W = V^T Pi^1/2
     }
   }
-  cluster.sync();  // no CTA leaves while another may still write into its shared memory
 }
 
 __global__ void __launch_bounds__(32) gamma_quantiles_kernel(const double *shape, int K, double *x, double *dxda) {
@@ -632,9 +787,6 @@ int tt_reversible_eigen(int32_t batch, int32_t state_count, const double *q, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t gram_smem = (2 * size_t(kEigMax) * kEigLd + kEigRows * kEigLd + kEigMax) * sizeof(double);
   const size_t orth_smem = (size_t(kEigMax) * kEigLd + kEigRows * kEigLd) * sizeof(double);
-  const size_t finish_smem =
-      (2 * size_t(kEigMax) * kEigLd + kEigMax + 2 * (kEigThreads / 32) + kEigMax) * sizeof(double) +
-      kEigMax * sizeof(int);
   if (n <= kEigSmall) {
     eigen_small_kernel<<<batch, 32, 0, s>>>(q, frequencies, n, eigenvalues, u, w, status);
     const cudaError_t e = cudaGetLastError();
@@ -642,8 +794,9 @@ int tt_reversible_eigen(int32_t batch, int32_t state_count, const double *q, con
   }
   cudaError_t e = kernel_smem(eigen_gram_kernel, gram_smem);
   if (e == cudaSuccess) e = kernel_smem(eigen_orth_kernel, orth_smem);
-  if (e == cudaSuccess) e = kernel_smem(eigen_finish_kernel, finish_smem);
-  if (e == cudaSuccess) e = kernel_smem(eigen_finish_cluster_kernel, finish_smem);
+  if (e == cudaSuccess) e = kernel_smem(eigen_start_kernel<64, 4>, eig_start_smem<64>());
+  if (e == cudaSuccess) e = kernel_smem(eigen_start_kernel<64, 1>, eig_start_smem<64>());
+  if (e == cudaSuccess) e = kernel_smem(eigen_finish_kernel<64, kEigCluster>, eig_finish_smem<64, kEigCluster>());
   // matrices in groups of at most 65,535 (the grid's y extent of the row-block kernels)
   for (int b0 = 0; e == cudaSuccess && b0 < batch; b0 += 65535) {
     const int nb = std::min(batch - b0, 65535);
@@ -651,16 +804,24 @@ int tt_reversible_eigen(int32_t batch, int32_t state_count, const double *q, con
     const double *qb = q + mo, *pib = frequencies + vo;
     double *ub = u + mo, *wb = w + mo, *lb = eigenvalues + vo;
     const dim3 rows_grid((n + kEigRows - 1) / kEigRows, nb);
-    eigen_start_kernel<<<nb, kEigThreads, 0, s>>>(qb, pib, n, ub);
+    if (n <= 32) {
+      eigen_start_kernel<32, 1><<<nb, eig_start_threads<32>(), eig_start_smem<32>(), s>>>(qb, pib, n, ub);
+    } else if (nb <= 76) {  // four CTAs each while 152 SMs hold them at two CTAs per SM (64 matrices 443 us);
+                            // more take one each (300 matrices 516 us, 719 before)
+      eigen_start_kernel<64, 4><<<4 * nb, eig_start_threads<64>(), eig_start_smem<64>(), s>>>(qb, pib, n, ub);
+    } else {
+      eigen_start_kernel<64, 1><<<nb, eig_start_threads<64>(), eig_start_smem<64>(), s>>>(qb, pib, n, ub);
+    }
     for (int it = 0; it < 2; ++it) {
       eigen_gram_kernel<<<rows_grid, kEigThreads, gram_smem, s>>>(qb, pib, n, ub, wb, lb, 0);
       eigen_orth_kernel<<<rows_grid, kEigThreads, orth_smem, s>>>(n, ub, wb, lb);
     }
     eigen_gram_kernel<<<rows_grid, kEigThreads, gram_smem, s>>>(qb, pib, n, ub, wb, lb, 1);
-    if (n > 32)  // FP64 sweeps on a cluster of CTAs per matrix
-      eigen_finish_cluster_kernel<<<nb * kEigCluster, kEigThreads, finish_smem, s>>>(pib, n, lb, ub, wb, status);
+    if (n > 32)
+      eigen_finish_kernel<64, kEigCluster><<<nb * kEigCluster, kEigThreads, eig_finish_smem<64, kEigCluster>(), s>>>(
+          pib, n, lb, ub, wb, status);
     else
-      eigen_finish_kernel<<<nb, kEigThreads, finish_smem, s>>>(pib, n, lb, ub, wb, status);
+      eigen_finish_kernel<32, 1><<<nb, kEigThreads, eig_finish_smem<32, 1>(), s>>>(pib, n, lb, ub, wb, status);
     e = cudaGetLastError();
   }
   return e == cudaSuccess ? TT_OK : tt::efail(TT_ERR_CUDA, std::string("eigen launch: ") + cudaGetErrorString(e));
