@@ -43,6 +43,7 @@ struct WideState {
   int bchunk = 8, nbchunks = 1;
   bool tc = false;  // FP32 codon post-order on the tensor cores
   bool store_products = false;  // FP32 codon: the adjoint reads the post-order's children's products
+  bool room_products = false;   // FP64 codon: ... of internal children, where there is room (product_room)
   bool tc_bwd = false;  // FP32 codon adjoint on the tensor cores (needs the stored products)
   float *d_pimg = nullptr;  // its GEMM2 operands: split P^T images [b][B][K][2][64][64]
   float *d_pimg_f = nullptr;  // the tensor-core post-order's B operands: split P images, same shape
@@ -73,7 +74,7 @@ struct WideState {
   double *d_pgpart = nullptr;
   uint8_t *d_tip_row = nullptr;  // [258] code -> row of the staged P^T (WideArgs::tip_row)
   void *d_tip_amb = nullptr;     // [kTipRows][SP] the ambiguous code vectors
-  void *d_prod = nullptr;  // FP32: the children's products of the post-order, read by the adjoint
+  void *d_prod = nullptr;  // the children's products of the post-order, read by the adjoint
 };
 
 namespace {
@@ -359,7 +360,7 @@ struct Wide {
       if (w.tc_bwd && a.prod && w.d_pimg) return backward_tc(p, a, g, accumulate, s);
     }
     constexpr int NT = WideCfg<T, SP, PTB>::NT;
-    const size_t smem = wide_bwd_smem<T, SP, PTB>(a.prod != nullptr);
+    const size_t smem = wide_bwd_smem<T, SP, PTB>(std::is_same<T, float>::value && a.prod);
     // FP32 20-state plans: a chunk count per level (three CTAs per SM), as the tensor-core adjoint does
     constexpr bool per_level = std::is_same<T, float>::value && SP == 20;
     const int bk = p->batch * p->K, target = 8 * 152 * 3;
@@ -550,6 +551,7 @@ int wide_create(tt_plan *p) {
      // states the extra stores cost more than the products they save
     const char *env = getenv("TT_WIDE_STORE_PRODUCTS");
     w->store_products = f32 && SP == 64 && !(env && atoi(env) == 0);
+    w->room_products = !f32 && SP == 64 && !(env && atoi(env) == 0);
   }
   {  // tensor-core adjoint for those plans (TT_WIDE_TC_BWD=0 selects the CUDA-core kernel)
     const char *env = getenv("TT_WIDE_TC_BWD");
@@ -611,6 +613,21 @@ SlabBuffers slab_buffers(const tt_plan *p, int n, bool slab) {
   return x;
 }
 
+// Whether an FP64 codon plan keeps its internal children's products beside buffers of `total` bytes:
+// they save the adjoint a third of its FP64 operations and are as large as the partials.  They are
+// no reason for slabs (choose_slab does not count them): kept if they take at most a quarter of the
+// device's free memory and stay within TT_GRADIENT_BUDGET_BYTES.
+bool product_room(size_t bytes, size_t total) {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (const char *env = getenv("TT_GRADIENT_BUDGET_BYTES"))
+    if (total + bytes > size_t(atoll(env))) return false;
+  return bytes <= free_b / 4;
+}
+
 void free_slab_buffers(tt_plan *p) {
   WideState &w = *p->wide;
   for (void **x : {reinterpret_cast<void **>(&w.d_part), reinterpret_cast<void **>(&w.d_expo),
@@ -649,6 +666,9 @@ int wide_alloc_slab(tt_plan *p, int slab) {
   if (!rc) rc = walloc(p, &w.d_gpart, x.gpart, "gradient chunks");
   if (!rc) rc = walloc(p, &w.d_rootpart, x.rootpart, "root gradient chunks");
   if (!rc && x.site) rc = walloc(p, &w.d_site, x.site, "slab site log-likelihoods");
+  if (!rc && w.room_products && product_room(x.part, x.total())) {
+    if (walloc(p, &w.d_prod, x.part, "children's products")) w.d_prod = nullptr;  // the adjoint forms them
+  }
   w.slab_bytes = p->bytes - before;
   if (rc) {
     free_slab_buffers(p);

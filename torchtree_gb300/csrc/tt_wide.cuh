@@ -360,6 +360,16 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
   else wide_product<T, SP, XS>(al, plt, xs, a.S, ib, pb);
   if (look_r) wide_tip_product<T, SP>(a, ar, plt + PS, r, n0 + pb * PQ, ib);
   else wide_product<T, SP, XS>(ar, plt + PS, xs + SP * XS, a.S, ib, pb);
+  if (sizeof(T) == 8 && SP == 64 && a.prod) {  // internal children's products, at the child's block
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int child = c ? r : l;
+      if (child < a.tips) continue;
+      T *pd = a.prod + ((size_t(b) * a.I + (child - a.tips)) * a.K + k) * SP * size_t(a.Npad) + n0 + pb * PQ;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) VP<T, PQ>::st(pd + size_t(ib + IB * i) * a.Npad, c ? ar[i] : al[i]);
+    }
+  }
   if (sizeof(T) == 4 && SP == 64 && a.prod) {
     T *pd = a.prod + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * 2 * SP * size_t(a.Npad) + n0 + pb * PQ;
 #pragma unroll
@@ -496,6 +506,9 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
   // stored products: FP32 codon plans only (the other instantiations keep GEMM1)
   constexpr bool kProd = sizeof(T) == 4 && SP == 64;
   const bool prod = kProd && a.prod != nullptr;
+  // FP64 codon plans with the room for it keep the internal children's products, [b][I][K][SP][Npad]
+  const bool prod_l = sizeof(T) == 8 && SP == 64 && a.prod && a.left[a.nodes[blockIdx.y] - a.tips] >= a.tips;
+  const bool prod_r = sizeof(T) == 8 && SP == 64 && a.prod && a.right[a.nodes[blockIdx.y] - a.tips] >= a.tips;
   constexpr int PS = (SP + kTipRows) * SP;
   T *plt = reinterpret_cast<T *>(smem);       // [2][SP j + tip rows][SP perm i]   P^T (GEMM1, absent with stored products)
   T *pl = prod ? plt : plt + 2 * PS;          // [2][SP i][SP perm j]   P   (GEMM2); a tip's gradient in FP64 plans
@@ -516,7 +529,7 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
   for (int e = tid; e < 2 * SP * SP; e += NT) {
     const int c = e / (SP * SP), ij = e - c * SP * SP, i = ij / SP, j = ij - i * SP;
     const T val = a.pmat[((size_t(b) * a.B + (c ? r : l)) * a.K + k) * SP * SP + ij];
-    if (!prod) plt[c * PS + j * SP + wperm<IB>(i)] = val;
+    if (!(prod || (c ? prod_r : prod_l))) plt[c * PS + j * SP + wperm<IB>(i)] = val;
     pl[c * SP * SP + i * SP + wperm<IB>(j)] = val;
   }
   const bool rows = !prod && __ldg(a.tip_row + 256), look_l = rows && l < a.tips, look_r = rows && r < a.tips;
@@ -555,7 +568,7 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
     if (tile + 1 < t1) {  // the next tile's rows into L2 while this one computes
       constexpr int LPR = PT * int(sizeof(T)) / 128;  // 128-byte lines per tile row
       const int rows_l = l >= a.tips ? SP : 0, rows_r = r >= a.tips ? SP : 0, rows_p = is_root ? 0 : SP;
-      const int rows_q = (kProd && a.prod) ? 2 * SP : 0;
+      const int rows_q = prod ? 2 * SP : (prod_l ? SP : 0) + (prod_r ? SP : 0);
       const int nrows = rows_l + rows_r + rows_p + rows_q;
       for (int e = tid; e < nrows * LPR; e += NT) {
         int row = e / LPR;
@@ -569,7 +582,13 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
           base = a.part + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * SP * size_t(a.Npad);
         } else {
           row -= rows_p;
-          base = a.prod + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * 2 * SP * size_t(a.Npad);
+          if (prod) {
+            base = a.prod + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * 2 * SP * size_t(a.Npad);
+          } else {
+            const bool second = !prod_l || row >= SP;
+            row -= second && prod_l ? SP : 0;
+            base = a.prod + ((size_t(b) * a.I + ((second ? r : l) - a.tips)) * a.K + k) * SP * size_t(a.Npad);
+          }
         }
         asm volatile("prefetch.global.L2 [%0];" ::"l"(base + size_t(row) * a.Npad + n0 + PT + seg * (128 / int(sizeof(T)))));
       }
@@ -611,9 +630,16 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
         VP<T, PQ>::ldg(pd + size_t(SP + ib + IB * i) * a.Npad, ar[i]);
       }
     } else {
-      if (look_l) wide_tip_product<T, SP>(a, al, plt, l, n0 + pb * PQ, ib);
+      auto stored = [&](T (&acc)[4][PQ], int child) {
+        const T *pd = a.prod + ((size_t(b) * a.I + (child - a.tips)) * a.K + k) * SP * size_t(a.Npad) + n0 + pb * PQ;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) VP<T, PQ>::ldg(pd + size_t(ib + IB * i) * a.Npad, acc[i]);
+      };
+      if (prod_l) stored(al, l);
+      else if (look_l) wide_tip_product<T, SP>(a, al, plt, l, n0 + pb * PQ, ib);
       else wide_product<T, SP, XS>(al, plt, xs, a.S, ib, pb);
-      if (look_r) wide_tip_product<T, SP>(a, ar, plt + PS, r, n0 + pb * PQ, ib);
+      if (prod_r) stored(ar, r);
+      else if (look_r) wide_tip_product<T, SP>(a, ar, plt + PS, r, n0 + pb * PQ, ib);
       else wide_product<T, SP, XS>(ar, plt + PS, xs + SP * XS, a.S, ib, pb);
     }
     if (is_root) {
