@@ -87,6 +87,7 @@ int wfail(int code, const std::string &m) { return record_error(code, m.c_str())
 // cmax bounds the chunk count of any pass over at most n patterns).
 struct WideGeo {
   int Npad, ntiles_f, ntiles_b, nblk, nchunks, tpc, cmax;
+  bool fine;  // FP64 codon passes whose levels choose between tiles of 32 and 16 patterns
 };
 
 WideGeo wide_geo(const tt_plan *p, int n) {
@@ -102,6 +103,13 @@ WideGeo wide_geo(const tt_plan *p, int n) {
   g.cmax = std::max(1, std::min({want, g.ntiles_b, 64}));
   g.tpc = (g.ntiles_b + g.cmax - 1) / g.cmax;
   g.nchunks = (g.ntiles_b + g.tpc - 1) / g.tpc;
+  // (whole alignments of up to 512 patterns, a chunk per tile: the gradient chunks stay small)
+  const int t16 = (n + 15) / 16;
+  g.fine = p->precision == TT_PRECISION_F64 && w.SP == 64 && n == p->N && t16 <= std::min(want, 32);
+  if (g.fine) {
+    g.cmax = g.nchunks = t16;
+    g.tpc = 1;
+  }
   return g;
 }
 
@@ -183,6 +191,14 @@ struct Wide {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(wide_backward_kernel<T, SP, PTB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                int(wide_bwd_smem<T, SP, PTB>()));
+    if constexpr (std::is_same<T, double>::value && SP == 64) {
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(wide_forward_kernel<T, SP, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(wide_fwd_smem<T, SP, 16>()));
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(wide_backward_kernel<T, SP, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(wide_bwd_smem<T, SP, 16>()));
+    }
     if (e == cudaSuccess)  // the CTAs the shared memory allows per SM all resident
       e = cudaFuncSetAttribute(wide_backward_kernel<T, SP, PTB>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                int(cudaSharedmemCarveoutMaxShared));
@@ -332,6 +348,14 @@ struct Wide {
           continue;
         }
       }
+      if constexpr (std::is_same<T, double>::value && SP == 64) {
+        if (g.fine && wide_fine_level(nodes, p->batch * p->K, n)) {
+          wide_forward_kernel<T, SP, 16><<<dim3((n + 15) / 16, nodes, plan_run_samples(p) * p->K),
+                                           WideCfg<T, SP, 16>::NT, wide_fwd_smem<T, SP, 16>(), s>>>(a);
+          p->launches += 1;
+          continue;
+        }
+      }
       const dim3 grid(g.ntiles_f, nodes, plan_run_samples(p) * p->K);
       wide_forward_kernel<T, SP, PTF><<<grid, NT, smem, s>>>(a);
       p->launches += 1;
@@ -366,19 +390,33 @@ struct Wide {
     const int bk = p->batch * p->K, target = 8 * 152 * 3;
     for (size_t lv = 0; lv + 1 < w.bwd_off.size(); ++lv) {
       const int nodes = w.bwd_off[lv + 1] - w.bwd_off[lv];
-      const int chunks = per_level ? tc_level_chunks(nodes, bk, g.ntiles_b, g.cmax, target) : g.nchunks;
       a.nodes = w.d_bwd + w.bwd_off[lv];
+      if constexpr (std::is_same<T, double>::value && SP == 64) {
+        if (g.fine && wide_fine_level(nodes, bk, n)) {
+          WideArgs<T> af = a;
+          af.ntiles = (n + 15) / 16;
+          wide_backward_kernel<T, SP, 16><<<dim3(af.ntiles, nodes, plan_run_samples(p) * p->K),
+                                            WideCfg<T, SP, 16>::NT, wide_bwd_smem<T, SP, 16>(), s>>>(af);
+          p->launches += 1;
+          continue;
+        }
+      }
+      const int chunks = per_level ? tc_level_chunks(nodes, bk, g.ntiles_b, g.cmax, target)
+                         : g.fine  ? g.ntiles_b
+                                   : g.nchunks;
       a.tiles_per_chunk = per_level ? (g.ntiles_b + chunks - 1) / chunks : g.tpc;
       const dim3 grid(chunks, nodes, plan_run_samples(p) * p->K);
       wide_backward_kernel<T, SP, PTB><<<grid, NT, smem, s>>>(a);
       p->launches += 1;
     }
-    wide_grad_reduce_kernel<T><<<dim3(p->B, plan_run_samples(p)), 256, 0, s>>>(
+    const int spread = p->B * plan_run_samples(p) < 8 * 152 ? 4 : 1;
+    wide_grad_reduce_kernel<T><<<dim3(p->B, plan_run_samples(p), spread), 256, 0, s>>>(
         static_cast<const T *>(w.d_gpart), p->d_G, p->B, g.nchunks, p->K, p->S, SP, accumulate,
-        per_level ? w.d_branch_lvn : nullptr, bk, g.ntiles_b, g.cmax, target);
+        per_level || g.fine ? w.d_branch_lvn : nullptr, bk, g.ntiles_b, g.cmax, target, g.fine ? n : 0);
+    const int root_used = g.fine && !wide_fine_level(1, bk, n) ? g.ntiles_b : g.nchunks;
     wide_root_reduce_kernel<T><<<plan_run_samples(p), 64, 0, s>>>(static_cast<const T *>(w.d_rootpart), p->d_rootgrad,
                                                        p->d_rootgrad + size_t(p->batch) * p->S, g.nchunks, p->K,
-                                                       p->S, SP, accumulate);
+                                                       p->S, SP, accumulate, root_used);
     p->launches += 2;
     return cudaGetLastError();
   }
@@ -428,7 +466,7 @@ struct Wide {
                                                                          accumulate, w.d_branch_lvn, bk, ntc, cmax);
     wide_root_reduce_kernel<float><<<plan_run_samples(p), 64, 0, s>>>(static_cast<const float *>(w.d_rootpart), p->d_rootgrad,
                                                            p->d_rootgrad + size_t(p->batch) * p->S, a.nchunks, p->K,
-                                                           p->S, 64, accumulate);
+                                                           p->S, 64, accumulate, a.nchunks);
     p->launches += 2;
     return cudaGetLastError();
   }

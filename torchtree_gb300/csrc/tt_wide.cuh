@@ -838,16 +838,29 @@ __host__ __device__ inline int tc_level_chunks(int nodes, int bk, int ntc, int c
   return (ntc + tpc - 1) / tpc;
 }
 
+// FP64 codon passes over few patterns: whether a level of `nodes` nodes runs in
+// tiles of 16 patterns rather than 32.  A CTA's tile is bound by its SM's FP64
+// units, so a level takes as many tile times as its CTAs go into 152 SMs: the
+// smaller tile where its waves, at 0.65 of the larger one's (the matrices are staged
+// as often), are cheaper.  60 taxa x 301 patterns x 4 categories (levels of 1 to 14
+// nodes): post-order 981 -> 847 us, adjoint 2,054 -> 1,958 us (with 16 everywhere 889
+// and 2,079).
+__host__ __device__ inline bool wide_fine_level(int nodes, int bk, int n) {
+  const long long c32 = (long long)nodes * bk * ((n + 31) / 32), c16 = (long long)nodes * bk * ((n + 15) / 16);
+  return 130 * ((c16 + 151) / 152) < 200 * ((c32 + 151) / 152);
+}
+
 // Fixed-order sums over chunks: G[b][branch][k][S][S] (FP64, unpadded) and
 // the root gradients dfreq[b][S], dprop[b][K]; accumulate = 1 adds to what
 // is there (pattern slabs after the first).  nchunks is the chunk stride of
 // gpart; with branch_lvn (the node count of each branch's parent level) a
 // branch sums only the chunks its level launched, tc_level_chunks(lvn, bk,
-// ntc, cmax).
+// ntc, cmax), or, with fine_n patterns in tiles by wide_fine_level, a chunk per
+// tile.  The entries are spread over gridDim.z CTAs.
 template <typename T>
 __global__ void wide_grad_reduce_kernel(const T *gpart, double *G, int B, int nchunks, int K, int S, int SP,
                                         int accumulate, const int *branch_lvn = nullptr, int bk = 0, int ntc = 0,
-                                        int cmax = 0, int target = 8 * 152) {
+                                        int cmax = 0, int target = 8 * 152, int fine_n = 0) {
   // four consecutive columns per thread, threads along the row: 16-byte (FP32) or 2 x 16-byte
   // (FP64) loads of every chunk's block, the chunk sum in the plan's precision and a fixed
   // order, then FP64 (FP64 arithmetic is scarce on this GPU and the chunk blocks themselves are
@@ -856,9 +869,12 @@ __global__ void wide_grad_reduce_kernel(const T *gpart, double *G, int B, int nc
   const int kss = K * S * S, q4 = SP / 4;
   const size_t cstride = size_t(K) * SP * SP;  // between chunks
   const T *base = gpart + (size_t(b) * B + br) * nchunks * cstride;
-  const int used = branch_lvn ? tc_level_chunks(branch_lvn[br], bk, ntc, cmax, target) : nchunks;
+  const int used = !branch_lvn ? nchunks
+                   : !fine_n   ? tc_level_chunks(branch_lvn[br], bk, ntc, cmax, target)
+                   : wide_fine_level(branch_lvn[br], bk, fine_n) ? (fine_n + 15) / 16
+                                                                 : (fine_n + 31) / 32;
   double *gb = G + (size_t(b) * B + br) * kss;
-  for (int e = threadIdx.x; e < K * S * q4; e += blockDim.x) {
+  for (int e = threadIdx.x + blockDim.x * blockIdx.z; e < K * S * q4; e += blockDim.x * gridDim.z) {
     const int kr = e / q4, j0 = (e - kr * q4) * 4;
     if (j0 >= S) continue;
     const int k = kr / S, i = kr - k * S;
@@ -891,18 +907,18 @@ __global__ void wide_grad_reduce_kernel(const T *gpart, double *G, int B, int nc
 
 template <typename T>
 __global__ void wide_root_reduce_kernel(const T *rootpart, double *dfreq, double *dprop, int nchunks, int K, int S,
-                                        int SP, int accumulate) {
+                                        int SP, int accumulate, int used) {
   const int b = blockIdx.x;
   for (int e = threadIdx.x; e < S + K; e += blockDim.x) {
     double s = 0.0;
     if (e < S) {
-      for (int c = 0; c < nchunks; ++c)
+      for (int c = 0; c < used; ++c)
         for (int k = 0; k < K; ++k) s += double(rootpart[((size_t(b) * nchunks + c) * K + k) * (SP + 1) + e]);
       double *d = dfreq + size_t(b) * S + e;
       *d = accumulate ? *d + s : s;
     } else {
       const int k = e - S;
-      for (int c = 0; c < nchunks; ++c) s += double(rootpart[((size_t(b) * nchunks + c) * K + k) * (SP + 1) + SP]);
+      for (int c = 0; c < used; ++c) s += double(rootpart[((size_t(b) * nchunks + c) * K + k) * (SP + 1) + SP]);
       double *d = dprop + size_t(b) * K + k;
       *d = accumulate ? *d + s : s;
     }
