@@ -535,7 +535,7 @@ int tt_plan_create(tt_plan **plan, int32_t tip_count, const int32_t *postorder,
   } else if (tt::td_smem_bytes(p->K, 256, p->slots_ws, false) <= size_t(smem_max) &&
              tt::td_smem_bytes(p->K, 256, p->slots_bwd, true) <= size_t(smem_max)) {
     p->tile_f = p->tile_b = tt::td_tile_patterns(p->K);
-    // adjoint CTAs (one warp each) per sample: kTdCtasPerSm on every SM over the batch, fewer where
+    // adjoint CTAs per sample: kTdCtasPerSm on every SM over the batch, fewer where
     // the shared memory of a deep tree's stack holds fewer
     const size_t smem = tt::td_smem_bytes(p->K, 16, p->slots_bwd, true) + 1024;
     const int per_sm = std::max(1, std::min(tt::kTdCtasPerSm, int(size_t(smem_max) / smem)));

@@ -34,9 +34,9 @@ cudaError_t launch_td(const PruneArgs<double> &a, bool backward, int batch, cuda
   cudaError_t e = backward ? kernel_smem(td_backward_kernel<KP>, smem, true) : kernel_smem(td_forward_kernel<KP>, smem, true);
   if (e != cudaSuccess) return e;
   if (backward)
-    td_backward_kernel<KP><<<dim3(a.nslots, batch), 32, smem, stream>>>(a);
+    td_backward_kernel<KP><<<dim3(a.nslots, batch), 64, smem, stream>>>(a);
   else
-    td_forward_kernel<KP><<<dim3(a.ntiles, batch), 32, smem, stream>>>(a);
+    td_forward_kernel<KP><<<dim3(a.ntiles, batch), 64, smem, stream>>>(a);
   return cudaGetLastError();
 }
 

@@ -4,9 +4,10 @@
 // (measured: 31 ns for DFMA, DADD and DMUL alike, whatever the number of
 // chains; fmax 3.4 and a division 9 of those), so the count of FP64
 // instructions is the time and everything else hides behind it.  Hence:
-//  * one warp per CTA and per tile of 32 / KP patterns (KP = categories padded
-//    to 1, 2, 4 or 8), one thread per (pattern, category): no block barrier, and
-//    a small alignment still spreads over as many SM quarters as it has warps;
+//  * a tile of 32 / KP patterns (KP = categories padded to 1, 2, 4 or 8), one thread
+//    per (pattern, category), on a CTA of two warps: one walks the tree, the other
+//    stages the steps and, in the adjoint, sums the gradients, so that little but FP64
+//    instructions is on the walk, which is all the time of a small alignment;
 //  * a tip with an unambiguous state takes its matrix's column (no product), and
 //    its gradient is one addition per pattern and row, its state picking the
 //    accumulator by selects;
@@ -22,10 +23,11 @@
 // its share of the matrices, its own child vectors, the tip codes and exponents
 // into a ring by cp.async, two or three steps ahead.
 //
-// Measured (GB300), post-order / adjoint, before (64-pattern CTAs, one thread
-// per pattern, all categories, tips as products) -> now:
-//   87 taxa x 611 patterns x 3:      681 / 1,847 ->   135 / 355 us
-//   500 taxa x 6,584 patterns x 4: 4,996 / 31,916 -> 2,526 / 7,385 us
+// Measured (GB300), post-order / adjoint: 64-pattern CTAs, one thread per pattern, all
+// categories, tips as products -> one warp per tile -> two warps per tile:
+//   69 taxa x 238 patterns x 1:                         109 / 283 ->    95 / 179 us
+//   87 taxa x 611 patterns x 3:      681 / 1,847 ->     135 / 355 ->   118 / 230 us
+//   500 taxa x 6,584 patterns x 4: 4,996 / 31,916 -> 2,526 / 7,385 -> 2,394 / 7,000 us
 #pragma once
 
 #include "tt_common.cuh"
@@ -67,7 +69,7 @@ __host__ __device__ inline TdLayout td_layout(int K, int C, int slots, bool back
   L.sexp = off;
   if (backward) off += slots * 32 * 4;
   L.ubuf = off;
-  if (backward) off += 8 * KP * (PW * 8 + 16);
+  if (backward) off += 2 * 8 * KP * (PW * 8 + 16);
   L.total = off;
   return L;
 }
@@ -203,41 +205,66 @@ __device__ __forceinline__ void td_load_table(const PruneArgs<double> &a, double
   }
 }
 
+// The two warps of a CTA pass stages and u by named barriers, two of each kind in turn
+// (one warp may be a step ahead); every arrival has its wait.  (Immediate barrier
+// numbers: a number in a register would take all sixteen, and CTAs per SM with them.)
+constexpr int kTdBarFull = 1, kTdBarU = 3, kTdBarFree = 5;  // stage landed, u written, stage read
+template <int BAR>
+__device__ __forceinline__ void td_arrive(int j) {
+  __syncwarp();
+  if (j & 1) asm volatile("bar.arrive %0, 64;" ::"n"(BAR + 1) : "memory");
+  else asm volatile("bar.arrive %0, 64;" ::"n"(BAR) : "memory");
+}
+template <int BAR>
+__device__ __forceinline__ void td_await(int j) {
+  __syncwarp();
+  if (j & 1) asm volatile("bar.sync %0, 64;" ::"n"(BAR + 1) : "memory");
+  else asm volatile("bar.sync %0, 64;" ::"n"(BAR) : "memory");
+}
 // -------------------------------------------------------------- post-order
+// The first warp walks the tree, the second stages its steps.
 template <int KP>
-__global__ void __launch_bounds__(32) td_forward_kernel(const PruneArgs<double> a) {
+__global__ void __launch_bounds__(64) td_forward_kernel(const PruneArgs<double> a) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int PW = 32 / KP, NST = kTdFwdStages;
-  const int lane = threadIdx.x, k = lane / PW, p = lane % PW;
+  const int lane = threadIdx.x % 32, k = lane / PW, p = lane % PW;
   const int tile = blockIdx.x, b = blockIdx.y, n = tile * PW + p, K = a.K, nst = a.n_steps;
   const bool act = n < a.N, kact = k < K;
   const int kk = kact ? k : 0;  // padded lanes read category 0 and contribute zeros
   const TdLayout L = td_layout(K, a.C, a.slots, false);
   double *tab = reinterpret_cast<double *>(smem + L.table);
   unsigned char *onehot = smem + L.onehot, *stack = smem + L.stack;
-  td_load_table(a, tab, onehot, lane);
-  int4 nxt[3];
-  load_rec(nxt, a.steps_ws, 0);
-  for (int s = 0; s < NST - 1; ++s) {
-    if (s < nst) {
-      const int4 cur[3] = {nxt[0], nxt[1], nxt[2]};
-      if (s + 1 < nst) load_rec(nxt, a.steps_ws, s + 1);
-      td_issue<KP, false>(a, L, smem + L.stages + s * L.stage, cur, s, b, tile, lane);
+  if (threadIdx.x >= 32) {
+    int4 nxt[3];
+    load_rec(nxt, a.steps_ws, 0);
+    auto issue = [&](int t) {  // step t, and its group (empty past the last)
+      if (t < nst) {
+        const int4 cur[3] = {nxt[0], nxt[1], nxt[2]};
+        if (t + 1 < nst) load_rec(nxt, a.steps_ws, t + 1);
+        td_issue<KP, false>(a, L, smem + L.stages + (t % NST) * L.stage, cur, t, b, tile, lane);
+      }
+      cp_async_commit();
+    };
+    for (int s = 0; s < NST; ++s) issue(s);
+    cp_async_wait<NST - 1>();
+    td_arrive<kTdBarFull>(0);
+    for (int s = 0; s < nst; ++s) {
+      if (s + 1 < nst) {
+        cp_async_wait<NST - 2>();
+        td_arrive<kTdBarFull>(s + 1);
+      }
+      td_await<kTdBarFree>(s);
+      issue(s + NST);
     }
-    cp_async_commit();
+    return;
   }
+  td_load_table(a, tab, onehot, lane);
+  __syncwarp();
   double carry[4] = {0.0, 0.0, 0.0, 0.0};  // the previous step's partial
   int E = 0;
   double ll = 0.0;
   for (int s = 0; s < nst; ++s) {
-    cp_async_wait<NST - 2>();
-    __syncwarp();  // stage s landed for every lane; stage s - 1 is free
-    if (const int t = s + NST - 1; t < nst) {
-      const int4 cur[3] = {nxt[0], nxt[1], nxt[2]};
-      if (t + 1 < nst) load_rec(nxt, a.steps_ws, t + 1);
-      td_issue<KP, false>(a, L, smem + L.stages + (t % NST) * L.stage, cur, t, b, tile, lane);
-    }
-    cp_async_commit();
+    td_await<kTdBarFull>(s);
     const unsigned char *stg = smem + L.stages + (s % NST) * L.stage;
     const int4 r0 = reinterpret_cast<const int4 *>(stg + L.rec)[0], r1 = reinterpret_cast<const int4 *>(stg + L.rec)[1];
     const double *Pl = reinterpret_cast<const double *>(stg + L.pm) + kk * 16, *Pr = Pl + K * 16;
@@ -254,6 +281,7 @@ __global__ void __launch_bounds__(32) td_forward_kernel(const PruneArgs<double> 
       for (int i = 0; i < 4; ++i) v[i] = carry[i];
     }
     td_product(ar, Pr, r1.x == -1, stg[L.codes + 32 + p], onehot, tab, v);
+    td_arrive<kTdBarFree>(s);
 #pragma unroll
     for (int i = 0; i < 4; ++i) prod[i] = kact ? prod[i] * ar[i] : 0.0;
     int e = 0;
@@ -297,8 +325,12 @@ __global__ void __launch_bounds__(32) td_forward_kernel(const PruneArgs<double> 
 //  B  two unambiguous tips: 1 addition per row and pattern;
 //  C  one of each: every lane takes half (8 / KP-th) of the patterns of both a
 //     row of the internal child and one of the tip, then the halves are joined.
+//
+// The second warp of the CTA also sums the gradients, of the step before while the
+// first is at the next one's products: a step's copies and a third of its FP64
+// instructions leave the walk.  u passes between them in two buffers.
 template <int KP>
-__global__ void __launch_bounds__(32) td_backward_kernel(const PruneArgs<double> a) {
+__global__ void __launch_bounds__(64) td_backward_kernel(const PruneArgs<double> a) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int PW = 32 / KP, NST = kTdBwdStages;
   constexpr int ROWS = 4 * KP;                       // rows of one side
@@ -308,15 +340,17 @@ __global__ void __launch_bounds__(32) td_backward_kernel(const PruneArgs<double>
   constexpr int QA = 2 * ROWS < 32 ? 16 / ROWS : 1;  // A, B: pattern chunks per row
   constexpr int CA = PW / QA;                        // patterns per chunk
   constexpr int QC = 32 / ROWS, CC = PW / QC;        // C: chunks per row, patterns per chunk (4)
-  const int lane = threadIdx.x, k = lane / PW, p = lane % PW;
+  const int lane = threadIdx.x % 32, k = lane / PW, p = lane % PW;
+  const bool walks = threadIdx.x < 32;  // the other warp stages and sums
   const int b = blockIdx.y, slot = blockIdx.x, K = a.K, nst = a.n_steps, KSS = K * 16;
   const bool kact = k < K;
   const int kk = kact ? k : 0;
   const TdLayout L = td_layout(K, a.C, a.slots, true);
-  double *tab = reinterpret_cast<double *>(smem + L.table), *ub = reinterpret_cast<double *>(smem + L.ubuf);
+  double *tab = reinterpret_cast<double *>(smem + L.table), *const ubuf = reinterpret_cast<double *>(smem + L.ubuf);
   unsigned char *onehot = smem + L.onehot, *stack = smem + L.stack;
   int *sexp = reinterpret_cast<int *>(smem + L.sexp);
-  td_load_table(a, tab, onehot, lane);
+  if (walks) td_load_table(a, tab, onehot, lane);
+  __syncthreads();
   double pk = kact ? a.props[b * K + k] : 0.0, fr[4], rpi[4] = {0.0, 0.0, 0.0, 0.0}, rc = 0.0;
 #pragma unroll
   for (int i = 0; i < 4; ++i) fr[i] = a.freqs[b * 4 + i];
@@ -327,94 +361,112 @@ __global__ void __launch_bounds__(32) td_backward_kernel(const PruneArgs<double>
     const double w = act ? a.weights[n] : 0.0;
     __syncwarp();  // the ring of the previous tile is free
     int4 nxt[3];
-    load_rec(nxt, a.steps, nst - 1);
-    for (int j = 0; j < NST - 1; ++j) {
-      if (j < nst) {
-        const int4 cur[3] = {nxt[0], nxt[1], nxt[2]};
-        if (j + 1 < nst) load_rec(nxt, a.steps, nst - 2 - j);
-        td_issue<KP, true>(a, L, smem + L.stages + j * L.stage, cur, nst - 1 - j, b, tile, lane);
-      }
-      cp_async_commit();
-    }
-    for (int j = 0; j < nst; ++j) {
-      cp_async_wait<NST - 2>();
-      __syncwarp();  // stage j landed for every lane; stage j - 1 and u are free
-      if (const int t = j + NST - 1; t < nst) {
+    auto issue = [&](int t) {  // reversed step t, and its group (empty past the last)
+      if (t < nst) {
         const int4 cur[3] = {nxt[0], nxt[1], nxt[2]};
         if (t + 1 < nst) load_rec(nxt, a.steps, nst - 2 - t);
         td_issue<KP, true>(a, L, smem + L.stages + (t % NST) * L.stage, cur, nst - 1 - t, b, tile, lane);
       }
       cp_async_commit();
+    };
+    if (!walks) {
+      load_rec(nxt, a.steps, nst - 1);
+      for (int j = 0; j < NST; ++j) issue(j);
+      cp_async_wait<NST - 1>();
+      td_arrive<kTdBarFull>(0);
+    }
+    for (int j = 0; j < nst; ++j) {
       const unsigned char *stg = smem + L.stages + (j % NST) * L.stage;
       const int4 *rec = reinterpret_cast<const int4 *>(stg + L.rec);
-      const int4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
-      const int left = r0.y, right = r0.z, slot_in = r1.z, slot_l = r1.w, slot_r = r2.x;
+      double *const ub = ubuf + (j & 1 ? 2 * ROWS * USTR : 0);
+      if (walks) {
+        td_await<kTdBarFull>(j);
+        const int4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
+        const int slot_in = r1.z, slot_l = r1.w, slot_r = r2.x;
+        const bool ltip = r0.y < a.tip_count, rtip = r0.z < a.tip_count;
+        const double *Pl = reinterpret_cast<const double *>(stg + L.pm) + kk * 16, *Pr = Pl + K * 16;
+        const double *kids = reinterpret_cast<const double *>(stg + L.kids);
+        const int cl = stg[L.codes + p], cr = stg[L.codes + 32 + p];
+        double pre[4], al[4], ar[4], v[4];
+        if (!ltip) load_vec<double, 4>(v, kids + k * KSTR + p * 4);
+        td_product(al, Pl, ltip, cl, onehot, tab, v);
+        if (!rtip) load_vec<double, 4>(v, kids + (KP + k) * KSTR + p * 4);
+        td_product(ar, Pr, rtip, cr, onehot, tab, v);
+        int q = 0;
+        if (slot_in >= 0) {
+          td_stack_load(pre, stack, slot_in, lane);
+          q = sexp[slot_in * 32 + lane];
+        } else {  // root: L of the pattern over all categories, and the root gradients
+          double den = 0.0, r[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            r[i] = kact ? al[i] * ar[i] : 0.0;
+            pre[i] = pk * fr[i];
+            den = fma(pre[i], r[i], den);
+          }
+#pragma unroll
+          for (int o = PW; o < 32; o <<= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+          const double coef = act && den > 0.0 ? w / den : 0.0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            pre[i] *= coef;
+            if (act) {
+              rpi[i] = fma(coef * pk, r[i], rpi[i]);
+              rc = fma(coef * fr[i], r[i], rc);
+            }
+          }
+        }
+        // u of both sides to shared memory as rows, the children's outside partials to the stack
+        double ul[4], ur[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          ul[i] = kact && act ? pre[i] * ar[i] : 0.0;
+          ur[i] = kact && act ? pre[i] * al[i] : 0.0;
+        }
+        // the rows the gradients sum, at the pattern's true scale
+        {
+          double sl[4], sr[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) sl[i] = ul[i], sr[i] = ur[i];
+          td_scale(sl, -q);
+          td_scale(sr, -q);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            ub[(k * 4 + i) * USTR + p] = sl[i];
+            ub[(ROWS + k * 4 + i) * USTR + p] = sr[i];
+          }
+        }
+        td_arrive<kTdBarU>(j);
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+          if (side ? rtip : ltip) continue;
+          const double *P = side ? Pr : Pl;
+          double o[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            double row[4];
+            load_vec<double, 4>(row, P + i * 4);
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj) o[jj] = fma(row[jj], side ? ur[i] : ul[i], o[jj]);
+          }
+          const int e = td_exponent<KP>(o), to = side ? slot_r : slot_l;
+          td_scale(o, e);
+          td_stack_store(o, stack, to, lane);
+          sexp[to * 32 + lane] = q + e - (act ? reinterpret_cast<const int *>(stg + L.expo)[side * PW + p] : 0);
+        }
+        td_arrive<kTdBarFree>(j);
+        continue;
+      }
+      if (j + 1 < nst) {
+        cp_async_wait<NST - 2>();
+        td_arrive<kTdBarFull>(j + 1);
+      }
+      td_await<kTdBarU>(j);
+      const int left = rec[0].y, right = rec[0].z;
       const bool ltip = left < a.tip_count, rtip = right < a.tip_count;
-      const double *Pl = reinterpret_cast<const double *>(stg + L.pm) + kk * 16, *Pr = Pl + K * 16;
       const double *kids = reinterpret_cast<const double *>(stg + L.kids);
       const int cl = stg[L.codes + p], cr = stg[L.codes + 32 + p];
       const unsigned amb = __ballot_sync(0xffffffffu, (ltip && onehot[cl] > 3) || (rtip && onehot[cr] > 3));
-      double pre[4], al[4], ar[4], v[4];
-      if (!ltip) load_vec<double, 4>(v, kids + k * KSTR + p * 4);
-      td_product(al, Pl, ltip, cl, onehot, tab, v);
-      if (!rtip) load_vec<double, 4>(v, kids + (KP + k) * KSTR + p * 4);
-      td_product(ar, Pr, rtip, cr, onehot, tab, v);
-      int q = 0;
-      if (slot_in >= 0) {
-        td_stack_load(pre, stack, slot_in, lane);
-        q = sexp[slot_in * 32 + lane];
-      } else {  // root: L of the pattern over all categories, and the root gradients
-        double den = 0.0, r[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          r[i] = kact ? al[i] * ar[i] : 0.0;
-          pre[i] = pk * fr[i];
-          den = fma(pre[i], r[i], den);
-        }
-#pragma unroll
-        for (int o = PW; o < 32; o <<= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
-        const double coef = act && den > 0.0 ? w / den : 0.0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          pre[i] *= coef;
-          if (act) {
-            rpi[i] = fma(coef * pk, r[i], rpi[i]);
-            rc = fma(coef * fr[i], r[i], rc);
-          }
-        }
-      }
-      // u of both sides to shared memory as rows, the children's outside partials to the stack
-      double ul[4], ur[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        ul[i] = kact && act ? pre[i] * ar[i] : 0.0;
-        ur[i] = kact && act ? pre[i] * al[i] : 0.0;
-      }
-#pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        if (side ? rtip : ltip) continue;
-        const double *P = side ? Pr : Pl;
-        double o[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          double row[4];
-          load_vec<double, 4>(row, P + i * 4);
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) o[jj] = fma(row[jj], side ? ur[i] : ul[i], o[jj]);
-        }
-        const int e = td_exponent<KP>(o), to = side ? slot_r : slot_l;
-        td_scale(o, e);
-        td_stack_store(o, stack, to, lane);
-        sexp[to * 32 + lane] = q + e - (act ? reinterpret_cast<const int *>(stg + L.expo)[side * PW + p] : 0);
-      }
-      td_scale(ul, -q);
-      td_scale(ur, -q);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        ub[(k * 4 + i) * USTR + p] = ul[i];
-        ub[(ROWS + k * 4 + i) * USTR + p] = ur[i];
-      }
-      __syncwarp();
       double *gl = a.gpart + ((size_t(b) * a.branch_count + left) * a.nslots + slot) * KSS;
       double *gr = a.gpart + ((size_t(b) * a.branch_count + right) * a.nslots + slot) * KSS;
       if (amb == 0 && ltip != rtip) {  // C
@@ -518,8 +570,11 @@ __global__ void __launch_bounds__(32) td_backward_kernel(const PruneArgs<double>
           }
         }
       }
+      td_await<kTdBarFree>(j);
+      issue(j + NST);
     }
   }
+  if (!walks) return;
   // root gradients: frequencies over every lane, category weights over a category's lanes
 #pragma unroll
   for (int i = 0; i < 4; ++i) rpi[i] = warp_sum(rpi[i]);
