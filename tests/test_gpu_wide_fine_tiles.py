@@ -18,3 +18,13 @@ def test_fine_tiles_match_oracle(budget, N, K, b, extra, monkeypatch):
     if budget:  # bytes: no room for products (and slabs of the smallest size)
         monkeypatch.setenv("TT_GRADIENT_BUDGET_BYTES", budget)
     _against_oracle("f64", 61, N, K, b, extra)
+
+
+@pytest.mark.parametrize("budget", [None, "1"])
+@pytest.mark.parametrize("S,N,K,b,extra", [(20, 1, 1, 1, 0), (20, 129, 4, 2, 1), (20, 300, 2, 1, 5), (7, 257, 3, 1, 2),
+                                           (20, 200, 2, 1, 60), (33, 130, 2, 1, 1)])
+def test_kept_products_match_oracle(budget, S, N, K, b, extra, monkeypatch):
+    """The same with 20 and other state counts."""
+    if budget:
+        monkeypatch.setenv("TT_GRADIENT_BUDGET_BYTES", budget)
+    _against_oracle("f64", S, N, K, b, extra)

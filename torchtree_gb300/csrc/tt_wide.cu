@@ -43,7 +43,7 @@ struct WideState {
   int bchunk = 8, nbchunks = 1;
   bool tc = false;  // FP32 codon post-order on the tensor cores
   bool store_products = false;  // FP32 codon: the adjoint reads the post-order's children's products
-  bool room_products = false;   // FP64 codon: ... of internal children, where there is room (product_room)
+  bool room_products = false;   // FP64: ... of internal children, where there is room (product_room)
   bool tc_bwd = false;  // FP32 codon adjoint on the tensor cores (needs the stored products)
   float *d_pimg = nullptr;  // its GEMM2 operands: split P^T images [b][B][K][2][64][64]
   float *d_pimg_f = nullptr;  // the tensor-core post-order's B operands: split P images, same shape
@@ -384,7 +384,7 @@ struct Wide {
       if (w.tc_bwd && a.prod && w.d_pimg) return backward_tc(p, a, g, accumulate, s);
     }
     constexpr int NT = WideCfg<T, SP, PTB>::NT;
-    const size_t smem = wide_bwd_smem<T, SP, PTB>(std::is_same<T, float>::value && a.prod);
+    const size_t smem = wide_bwd_smem<T, SP, PTB>(!kChildProducts<T> && a.prod);
     // FP32 20-state plans: a chunk count per level (three CTAs per SM), as the tensor-core adjoint does
     constexpr bool per_level = std::is_same<T, float>::value && SP == 20;
     const int bk = p->batch * p->K, target = 8 * 152 * 3;
@@ -589,7 +589,7 @@ int wide_create(tt_plan *p) {
      // states the extra stores cost more than the products they save
     const char *env = getenv("TT_WIDE_STORE_PRODUCTS");
     w->store_products = f32 && SP == 64 && !(env && atoi(env) == 0);
-    w->room_products = !f32 && SP == 64 && !(env && atoi(env) == 0);
+    w->room_products = !f32 && !(env && atoi(env) == 0);
   }
   {  // tensor-core adjoint for those plans (TT_WIDE_TC_BWD=0 selects the CUDA-core kernel)
     const char *env = getenv("TT_WIDE_TC_BWD");
@@ -651,8 +651,8 @@ SlabBuffers slab_buffers(const tt_plan *p, int n, bool slab) {
   return x;
 }
 
-// Whether an FP64 codon plan keeps its internal children's products beside buffers of `total` bytes:
-// they save the adjoint a third of its FP64 operations and are as large as the partials.  They are
+// Whether an FP64 plan keeps its internal children's products beside buffers of `total` bytes: they save
+// the adjoint a third of its products and are as large as the partials.  They are
 // no reason for slabs (choose_slab does not count them): kept if they take at most a quarter of the
 // device's free memory and stay within TT_GRADIENT_BUDGET_BYTES.
 bool product_room(size_t bytes, size_t total) {

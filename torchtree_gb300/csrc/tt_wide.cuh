@@ -63,6 +63,16 @@ struct WideCfg {
 // more such codes take the product).
 constexpr int kTipRows = 4;
 
+// FP64 plans that, with the room for it, keep the internal children's products of the
+// post-order for the adjoint, by child: [b][I][K][SP][Npad] (a tip's are columns of
+// P).  A third of the adjoint's products, and these plans are bound by FP64 arithmetic.
+// FP32 codon plans keep both children's of every node, for the tensor cores; in FP32
+// 20-state plans the stores cost what they save (post-order 789 -> 959 us, adjoint
+// 3,271 -> 3,266 us at 200 taxa x 4,246 patterns x 4).  FP64, 20 states, 200 taxa x
+// 1,000 patterns x 2: adjoint 7,032 -> 5,784 us.
+template <typename T>
+constexpr bool kChildProducts = sizeof(T) == 8;
+
 // shared-memory bytes of the two kernels
 template <typename T, int SP, int PT>
 constexpr size_t wide_fwd_smem() {
@@ -360,7 +370,7 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
   else wide_product<T, SP, XS>(al, plt, xs, a.S, ib, pb);
   if (look_r) wide_tip_product<T, SP>(a, ar, plt + PS, r, n0 + pb * PQ, ib);
   else wide_product<T, SP, XS>(ar, plt + PS, xs + SP * XS, a.S, ib, pb);
-  if (sizeof(T) == 8 && SP == 64 && a.prod) {  // internal children's products, at the child's block
+  if (kChildProducts<T> && a.prod) {  // internal children's products, at the child's block
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int child = c ? r : l;
@@ -506,9 +516,8 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
   // stored products: FP32 codon plans only (the other instantiations keep GEMM1)
   constexpr bool kProd = sizeof(T) == 4 && SP == 64;
   const bool prod = kProd && a.prod != nullptr;
-  // FP64 codon plans with the room for it keep the internal children's products, [b][I][K][SP][Npad]
-  const bool prod_l = sizeof(T) == 8 && SP == 64 && a.prod && a.left[a.nodes[blockIdx.y] - a.tips] >= a.tips;
-  const bool prod_r = sizeof(T) == 8 && SP == 64 && a.prod && a.right[a.nodes[blockIdx.y] - a.tips] >= a.tips;
+  const bool prod_l = kChildProducts<T> && a.prod && a.left[a.nodes[blockIdx.y] - a.tips] >= a.tips;
+  const bool prod_r = kChildProducts<T> && a.prod && a.right[a.nodes[blockIdx.y] - a.tips] >= a.tips;
   constexpr int PS = (SP + kTipRows) * SP;
   T *plt = reinterpret_cast<T *>(smem);       // [2][SP j + tip rows][SP perm i]   P^T (GEMM1, absent with stored products)
   T *pl = prod ? plt : plt + 2 * PS;          // [2][SP i][SP perm j]   P   (GEMM2); a tip's gradient in FP64 plans

@@ -197,6 +197,13 @@ __global__ void __launch_bounds__(kColThreads, 3) wide_col_forward_kernel(const 
         for (int j = 0; j < SP; ++j)
 #pragma unroll
           for (int q = 0; q < PP; ++q) y[q].fma_row(pt + c * SP * SP + j * SP, x[j][q]);
+        if (kChildProducts<T> && a.prod) {
+          T *pd = a.prod + blk * SP * npad + n;
+#pragma unroll
+          for (int i = 0; i < SP; ++i)
+#pragma unroll
+            for (int q = 0; q < PP; ++q) pd[i * npad + q] = y[q].get(i);
+        }
       }
 #pragma unroll
       for (int q = 0; q < PP; ++q)
