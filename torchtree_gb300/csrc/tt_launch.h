@@ -46,8 +46,8 @@ constexpr int kCodeAlign = 128;
 inline int kmax_for(int K) { return K <= 1 ? 1 : (K <= 4 ? 4 : 8); }
 
 template <typename T>
-size_t prune_smem_bytes(int S, int K, int C, int slots, int tile, bool backward) {
-  return stack_layout<T>(S, K, C, slots, tile, kStages, kmax_for(K), backward).total;
+size_t prune_smem_bytes(int S, int K, int C, int slots, int tile) {
+  return stack_layout<T>(S, K, C, slots, tile, kStages).total;
 }
 
 // patterns per CTA of the producer-warp post-order (kTlPartTile-wide stored tiles)

@@ -211,7 +211,7 @@ extern "C" int tt_log_likelihood_static(int32_t tip_count, const int32_t *postor
   if (rc != TT_OK) return rc;
   int tile = 0;
   for (int t : tt::kFwdTilesF64)
-    if (!tile && tt::prune_smem_bytes<double>(S, K, kTableRows, slots, t, false) <= size_t(smem_max)) tile = t;
+    if (!tile && tt::prune_smem_bytes<double>(S, K, kTableRows, slots, t) <= size_t(smem_max)) tile = t;
   if (!tile) return fail(TT_ERR_UNSUPPORTED, "tree needs more shared memory than one CTA can hold");
   const int ntiles = (N + tile - 1) / tile;
   const int code_stride = (N + tt::kCodeAlign - 1) / tt::kCodeAlign * tt::kCodeAlign;

@@ -10,19 +10,14 @@
 //
 // Everything a step reads from global memory is staged into a shared-memory
 // ring a few steps ahead by the TMA engine (cp.async.bulk, completion on one
-// mbarrier per stage): the step record, the pair of transition matrices, the
-// tip-code rows of tip children and, in the adjoint, the stored partial
-// tiles of internal children.  The warps then read shared memory only.
+// mbarrier per stage): the step record, the pair of transition matrices and the
+// tip-code rows of tip children.  The warps then read shared memory only.
 //
-// Forward (replaces tree_likelihood.py:40-75 / 186-221): HBM traffic is the
-// write of each non-root internal partial (only when the gradient needs it).
-// Adjoint (replaces autograd through the same lines): walks the schedule in
-// reverse (a pre-order), keeps the outside partials in the shared-memory
-// stack, reads each stored partial once, and reduces dlnL/dP of each branch
-// over the tile through a shared-memory transpose.
+// prune_forward_kernel (replaces tree_likelihood.py:40-75 / 186-221) serves the
+// allocation-free entry point; plans take the kernels of tt_prune_t*.cuh, which
+// share the arguments, the step records and the layouts described here.
 //
-// Global partial layout: [batch][internal node - T][K][N][S], S innermost:
-// one category of one tile is a contiguous TILE*S run (one bulk copy).
+// Global partial layout: [batch][internal node - T][K][N][S], S innermost.
 // Tip codes: [T][code_stride] bytes, rows padded so each tile's run of
 // codes is 16-byte aligned.
 #pragma once
@@ -107,13 +102,13 @@ struct MultiPrune {
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
-// Layout of one ring stage: step record | matrix pair | 2 code rows | 2 child tiles
+// Layout of one ring stage: step record | matrix pair | 2 code rows
 struct StageLayout {
-  size_t rec, pm, codes, kids, bytes;
+  size_t rec, pm, codes, bytes;
 };
 
 template <typename T>
-__host__ __device__ inline StageLayout stage_layout(int S, int K, int tile, bool backward) {
+__host__ __device__ inline StageLayout stage_layout(int S, int K, int tile) {
   StageLayout g;
   size_t off = 0;
   g.rec = off;
@@ -122,22 +117,19 @@ __host__ __device__ inline StageLayout stage_layout(int S, int K, int tile, bool
   off = align16(off + size_t(2) * K * S * S * sizeof(T));
   g.codes = off;
   off = align16(off + size_t(2) * tile);
-  g.kids = off;
-  if (backward) off = align16(off + size_t(2) * K * tile * S * sizeof(T));
   g.bytes = off;
   return g;
 }
 
 struct StackLayout {
-  size_t stages, bars, table, stack, xbuf, red, red_root, total;
+  size_t stages, bars, table, stack, total;
 };
 
 // Shared-memory carve-up shared by the host (launch size) and the kernels.
 template <typename T>
-__host__ __device__ inline StackLayout stack_layout(int S, int K, int C, int slots, int tile, int nstage,
-                                                    int kmax, bool backward) {
+__host__ __device__ inline StackLayout stack_layout(int S, int K, int C, int slots, int tile, int nstage) {
   StackLayout L;
-  const StageLayout g = stage_layout<T>(S, K, tile, backward);
+  const StageLayout g = stage_layout<T>(S, K, tile);
   size_t off = 0;
   L.stages = off;
   off = align16(off + size_t(nstage) * g.bytes);
@@ -147,17 +139,7 @@ __host__ __device__ inline StackLayout stack_layout(int S, int K, int C, int slo
   off = align16(off + size_t(C) * S * sizeof(T));
   L.stack = off;
   off = align16(off + size_t(slots) * K * tile * S * sizeof(T));
-  L.xbuf = off;
-  if (backward) off = align16(off + size_t(2) * tile * (K * S + 16 / sizeof(T)) * sizeof(T));
-  L.red = off;
-  // per-row partial sums of the transpose reduction, double-buffered
-  const int rows = 2 * K * S;
-  const int q = tile >= rows ? tile / rows : 1;
-  if (backward) off = align16(off + size_t(2) * rows * q * S * sizeof(T));
-  L.red_root = off;
-  if (backward) off = align16(off + size_t(tile / 32) * (S + kmax) * sizeof(T));
   L.total = off;
-  (void)kmax;
   return L;
 }
 
@@ -196,7 +178,7 @@ __device__ __forceinline__ void rescale_pow2(T (&v)[KMAX][S], int K, int &E) {
 
 // Producer side of the ring (one thread): stage everything step `s` needs.
 // `rec` is the step's record (already loaded by the caller).
-template <typename T, int S, bool BACKWARD>
+template <typename T, int S>
 __device__ __forceinline__ void issue_step(const PruneArgs<T> &a, unsigned char *stage, uint64_t *bar,
                                            const int4 (&rec)[3], int s, int b, int tile, int TILE,
                                            const StageLayout &g) {
@@ -207,27 +189,17 @@ __device__ __forceinline__ void issue_step(const PruneArgs<T> &a, unsigned char 
   r[1] = rec[1];
   r[2] = rec[2];
   const int left = rec[0].y, right = rec[0].z;
-  const int rem = min(TILE, a.N - tile * TILE);
   const uint32_t pbytes = uint32_t(2 * kss * sizeof(T));
-  const uint32_t kid_bytes = uint32_t(rem) * S * sizeof(T);
   uint32_t total = pbytes;
   total += (left < a.tip_count ? TILE : 0) + (right < a.tip_count ? TILE : 0);
-  if (BACKWARD) total += (left >= a.tip_count ? K * kid_bytes : 0) + (right >= a.tip_count ? K * kid_bytes : 0);
   mbar_arrive_expect_tx(bar, total);
   bulk_copy_g2s(stage + g.pm, a.pmat + (size_t(b) * a.n_steps + s) * 2 * kss, pbytes, bar);
   const int child[2] = {left, right};
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    if (child[c] < a.tip_count) {
+    if (child[c] < a.tip_count)
       bulk_copy_g2s(stage + g.codes + c * TILE, a.codes + size_t(child[c]) * a.code_stride + size_t(tile) * TILE,
                     uint32_t(TILE), bar);
-    } else if (BACKWARD) {
-      const T *src = a.partials +
-                     ((size_t(b) * (a.n_steps - 1) + (child[c] - a.tip_count)) * K) * size_t(a.N) * S +
-                     size_t(tile) * TILE * S;
-      T *dst = reinterpret_cast<T *>(stage + g.kids) + size_t(c) * K * TILE * S;
-      for (int k = 0; k < K; ++k) bulk_copy_g2s(dst + size_t(k) * TILE * S, src + size_t(k) * a.N * S, kid_bytes, bar);
-    }
   }
 }
 
@@ -257,8 +229,8 @@ __global__ void __launch_bounds__(TILE) prune_forward_kernel(const PruneArgs<T> 
   const bool act = n < a.N;
   const int K = a.K;
   const int nst = a.n_steps;
-  const StackLayout L = stack_layout<T>(S, K, a.C, a.slots, TILE, NSTAGE, KMAX, false);
-  const StageLayout G = stage_layout<T>(S, K, TILE, false);
+  const StackLayout L = stack_layout<T>(S, K, a.C, a.slots, TILE, NSTAGE);
+  const StageLayout G = stage_layout<T>(S, K, TILE);
   unsigned char *stages = smem + L.stages;
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
   T *tab = reinterpret_cast<T *>(smem + L.table);
@@ -282,7 +254,7 @@ __global__ void __launch_bounds__(TILE) prune_forward_kernel(const PruneArgs<T> 
     for (int s = 0; s < NSTAGE - 1 && s < nst; ++s) {
       int4 cur[3] = {nxt[0], nxt[1], nxt[2]};
       if (s + 1 < nst) load_rec(nxt, a.steps, s + 1);
-      issue_step<T, S, false>(a, stages + s * G.bytes, &bars[s], cur, s, b, tile, TILE, G);
+      issue_step<T, S>(a, stages + s * G.bytes, &bars[s], cur, s, b, tile, TILE, G);
     }
   }
   bool timed_out = !mbar_wait_bounded(&bars[0], 0, a.timeout_ns);
@@ -298,7 +270,7 @@ __global__ void __launch_bounds__(TILE) prune_forward_kernel(const PruneArgs<T> 
       const int sp = s + NSTAGE - 1;
       int4 cur[3] = {nxt[0], nxt[1], nxt[2]};
       if (sp + 1 < nst) load_rec(nxt, a.steps, sp + 1);
-      issue_step<T, S, false>(a, stages + (sp % NSTAGE) * G.bytes, &bars[sp % NSTAGE], cur, sp, b, tile, TILE, G);
+      issue_step<T, S>(a, stages + (sp % NSTAGE) * G.bytes, &bars[sp % NSTAGE], cur, sp, b, tile, TILE, G);
     }
     const unsigned char *stg = stages + (s % NSTAGE) * G.bytes;
     const int4 *rec = reinterpret_cast<const int4 *>(stg + G.rec);

@@ -11,7 +11,7 @@ namespace {
 
 template <int KMAX, int TILE>
 cudaError_t launch_one(const PruneArgs<double> &a, int batch, cudaStream_t stream) {
-  const size_t smem = prune_smem_bytes<double>(4, a.K, a.C, a.slots, TILE, false);
+  const size_t smem = prune_smem_bytes<double>(4, a.K, a.C, a.slots, TILE);
   auto kern = prune_forward_kernel<double, 4, KMAX, TILE, kStages>;
   cudaError_t e = kernel_smem(kern, smem);
   if (e != cudaSuccess) return e;
