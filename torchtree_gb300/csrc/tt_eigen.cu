@@ -260,12 +260,6 @@ struct EigPair {
     sort();
   }
 };
-// offset of element (u, v) of a symmetric matrix held in its upper triangle
-template <int LD>
-__device__ __forceinline__ int eig_at(int u, int v) {
-  return min(u, v) * LD + max(u, v);
-}
-
 // (u, v) <- (c u - s v, s u + c v), rounded alike wherever it is inlined: a matrix's
 // system does not depend on the number of CTAs
 __device__ __forceinline__ void eig_mix(float2 cs, float &u, float &v) {
@@ -527,7 +521,7 @@ __global__ void __launch_bounds__(kEigThreads) eigen_orth_kernel(int n, double *
 // triangle) and X (in U); FP64 Jacobi sweeps on S, accumulated into X, to 1e-14 of
 // the Frobenius norm; a matrix that does not converge in 30 sweeps sets the status
 // word.  Eigenvalues ascending, with U = Pi^-1/2 X and W = X^T Pi^1/2.
-// Every CTA keeps a copy of A's upper triangle, in two buffers.  A round: every CTA
+// Every CTA keeps a copy of A, in two buffers.  A round: every CTA
 // forms the same rotations from its copy; of the blocks of four elements that two
 // rotations mix, each CTA updates its share, two threads a block, a row of it each,
 // rows first and columns then, and writes the results into every CTA's other buffer
@@ -535,9 +529,10 @@ __global__ void __launch_bounds__(kEigThreads) eigen_orth_kernel(int n, double *
 // coalesce; the rotations of a round read the buffer that nobody writes); while they
 // travel it rotates its own rows of X.  One cluster barrier a round.  Bound by FP64
 // latency and arithmetic (64 cycles per warp instruction and SM quarter).  61 states:
-// 1 matrix 528 -> 352 us, 16 matrices 531 -> 431 us, against 4 CTAs with full copies
+// 1 matrix 528 -> 401 us, 16 matrices 531 -> 488 us, against 4 CTAs with full copies
 // and rows and columns in separate passes.  Up to 32 states one CTA (20 states:
-// 216 -> 83 us).
+// 216 -> 93 us).  With the upper triangle alone (352 / 431 / 83 us) the last
+// bits change, and with them the rounding of FP32 transition matrices.
 constexpr int kEigCluster = 8;
 
 template <int NMAX, int C>
@@ -551,7 +546,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kEigThreads)
     eigen_finish_kernel(const double *pi, int n, double *lam, double *U, double *W, int *status) {
   namespace cg = cooperative_groups;
   constexpr int NT = kEigThreads, NW = NT / 32, LD = NMAX + 1, H = NMAX / 2, BUF = NMAX * LD;
-  constexpr int NB = ((H * (H + 1) / 2 + C - 1) / C + 31) / 32 * 32;  // this CTA's blocks, at most
+  constexpr int NB = ((H * H + C - 1) / C + 31) / 32 * 32;            // this CTA's blocks, at most
   constexpr int HB = (2 * NB + NT - 1) / NT;                          // half blocks per thread
   extern __shared__ __align__(16) double fsm[];
   double *A = fsm;                                        // [2][n + 1][LD]
@@ -568,24 +563,22 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kEigThreads)
   for (int i = tid; i < n; i += NT) sq[i] = sqrt(pi[size_t(b) * n + i]);
   for (int i = warp; i < m; i += NW)
     for (int j = lane; j < m; j += 32) {
-      if (i <= j) A[i * LD + j] = j < n ? W[mo + size_t(i) * n + j] : 0.0;  // a dummy player of zeros
+      A[i * LD + j] = i < n && j < n ? W[mo + size_t(min(i, j)) * n + max(i, j)] : 0.0;  // a dummy player of zeros
       if (i % C == rank) V[i / C * LD + j] = i < n && j < n ? U[mo + size_t(i) * n + j] : 0.0;
     }
   if constexpr (C > 1) cluster.sync();  // every CTA has read U and W before any writes its outputs
   else __syncthreads();
-  // this thread's half blocks, pairs i <= j and which row of pair i, and its lane's pair
+  // this thread's half blocks: pairs of rows and columns and which row of the two; its lane's pair
   int hi[HB], hj[HB];
-  const int blocks = npairs * (npairs + 1) / 2, share = (blocks + C - 1) / C;
+  const int blocks = npairs * npairs, share = (blocks + C - 1) / C;
   EigPair row_pair(tid % H, m), pi_[HB], pj[HB];
 #pragma unroll
   for (int k = 0; k < HB; ++k) {
-    const int h = tid + k * NT, at = h < NB ? h : h - NB;  // a warp's lanes along a row of the second pair
-    int e = rank * share + at, i = 0;
-    hi[k] = hj[k] = -1;
-    if (h >= 2 * NB || at >= share || e >= blocks) continue;
-    while (e >= npairs - i) e -= npairs - i, ++i;
-    hi[k] = i;
-    hj[k] = i + e;
+    const int h = tid + k * NT, at = h < NB ? h : h - NB, e = rank * share + at;  // a warp's lanes along a row
+    const bool mine = h < 2 * NB && at < share && e < blocks;
+    hi[k] = mine ? e / npairs : -1;
+    hj[k] = mine ? e % npairs : -1;
+    if (!mine) continue;
     pi_[k] = EigPair(hi[k], m);
     pj[k] = EigPair(hj[k], m);
   }
@@ -594,10 +587,10 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kEigThreads)
   for (int sweep = 0; sweep <= 30; ++sweep) {
     double off = 0.0, tot = 0.0;
     for (int i = warp; i < n; i += NW)
-      for (int j = i + lane; j < n; j += 32) {
+      for (int j = lane; j < n; j += 32) {
         const double v = cur[i * LD + j];
-        if (i != j) off = fma(v, v, off);
-        else tot = fma(v, v, tot);
+        tot += v * v;
+        if (i != j) off += v * v;
       }
     for (int o = 16; o; o >>= 1) {
       off += __shfl_xor_sync(0xffffffffu, off, o);
@@ -611,10 +604,10 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kEigThreads)
     if (tid == 0) {
       double so = 0.0, st = 0.0;
       for (int w = 0; w < NW; ++w) {
-        so += 2.0 * red[w];
+        so += red[w];
         st += red[NW + w];
       }
-      flag = !(so > 1e-28 * (st + so));
+      flag = !(so > 1e-28 * st) || n == 1;
     }
     __syncthreads();
     if (flag) {
@@ -635,11 +628,10 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kEigThreads)
       for (int k = 0; k < HB; ++k) {
         if (hi[k] < 0) continue;
         const double2 ri = rot[hi[k]], rj = rot[hj[k]];
-        const bool second = tid + k * NT >= NB, diag = hi[k] == hj[k];
-        const int own = second ? pi_[k].q : pi_[k].p;
-        const int o0 = eig_at<LD>(own, pj[k].p), o1 = eig_at<LD>(own, pj[k].q);
-        const double app = cur[eig_at<LD>(pi_[k].p, pj[k].p)], apq = cur[eig_at<LD>(pi_[k].p, pj[k].q)];
-        const double aqp = cur[eig_at<LD>(pi_[k].q, pj[k].p)], aqq = cur[eig_at<LD>(pi_[k].q, pj[k].q)];
+        const bool second = tid + k * NT >= NB;
+        const double *rp = cur + pi_[k].p * LD, *rq = cur + pi_[k].q * LD;
+        const int o0 = (second ? pi_[k].q : pi_[k].p) * LD + pj[k].p, o1 = o0 + pj[k].q - pj[k].p;
+        const double app = rp[pj[k].p], apq = rp[pj[k].q], aqp = rq[pj[k].p], aqq = rq[pj[k].q];
         pi_[k].advance(hi[k], m);
         pj[k].advance(hj[k], m);
         // the row of pair i: c p - s q, or s p + c q
@@ -650,7 +642,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kEigThreads)
 #pragma unroll
         for (int o = 0; o < C; ++o) {
           double *dst = C > 1 ? cluster.map_shared_rank(A, o) + base : nxt;
-          if (!(diag && second)) dst[o0] = n0;  // (q, p) is (p, q)
+          dst[o0] = n0;
           dst[o1] = n1;
         }
       }
