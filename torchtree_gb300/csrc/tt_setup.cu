@@ -36,12 +36,31 @@ __device__ __forceinline__ double lane_sum(double v) {  // the same bits in ever
   return v;
 }
 
+// term(0) + .. + term(n - 1) in the order in which the tensor compositions' row sums run
+// (L = the largest power of two up to 32 that is at most n: lane l takes l, l + L, ..; then
+// pairs of neighbours, of neighbouring pairs, ..), in every lane: rates and rate matrices
+// keep the compositions' bits, which FP32 transition matrices are rounded from.
+template <typename F>
+__device__ __forceinline__ double row_sum(int n, F term) {
+  const int lane = threadIdx.x & 31, L = n >= 32 ? 32 : 1 << (31 - __clz(n));
+  double s = 0.0;
+  if (lane < L)
+    for (int j = lane; j < n; j += L) s = __dadd_rn(s, term(j));
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) s = __dadd_rn(s, __shfl_down_sync(kAll, s, o));
+  return __shfl_sync(kAll, s, 0);
+}
+
 // Mean-one rates and their shape derivative from lane k's raw rate r and dr
 // (one warp, lanes >= K zero); equal category weights 1 / K.
 __device__ __forceinline__ void finish_rates(double r, double dr, int K, int b, double *rates, double *drates,
                                              double *probs) {
   const int k = threadIdx.x & 31;
-  const double w = 1.0 / K, m = lane_sum(r * w), dm = lane_sum(dr * w);
+  const double w = 1.0 / K, dm = lane_sum(dr * w);
+  __shared__ double rw[32];
+  rw[k] = __dmul_rn(r, w);
+  __syncwarp();
+  const double m = row_sum(K, [&](int j) { return rw[j]; });
   if (k < K) {
     const double rho = r / m;
     rates[size_t(b) * K + k] = rho;
@@ -142,11 +161,11 @@ __global__ void __launch_bounds__(256) exch_q_kernel(const __grid_constant__ Exc
     const int i = e / S, j = e - i * S;
     if (i != j) qb[e] = x.value(b, m, upper_index(i, j, S)) * pb[j];
   }
-  for (int i = threadIdx.x; i < S; i += blockDim.x) {
-    double s = 0.0;
-    for (int j = 0; j < S; ++j)
-      if (j != i) s += x.value(b, m, upper_index(i, j, S)) * pb[j];
-    qb[i * S + i] = -s;
+  for (int i = threadIdx.x >> 5; i < S; i += blockDim.x >> 5) {
+    const double s = row_sum(S, [&](int j) {
+      return j == i ? 0.0 : __dmul_rn(x.value(b, m, upper_index(i, j, S)), pb[j]);
+    });
+    if ((threadIdx.x & 31) == 0) qb[i * S + i] = -s;
   }
 }
 
@@ -231,9 +250,7 @@ __global__ void __launch_bounds__(256) prepare_kernel(const double *q, const dou
   const int b = blockIdx.x, tid = threadIdx.x;
   const double *qb = q + size_t(b) * S * S, *pb = pi + size_t(b) * S;
   if (tid < 32) {
-    double s = 0.0;
-    for (int i = tid; i < S; i += 32) s += qb[i * S + i] * pb[i];
-    s = -lane_sum(s);
+    const double s = -row_sum(S, [&](int i) { return __dmul_rn(qb[i * S + i], pb[i]); });
     if (tid == 0) smu = s, w.mu[b] = s;
   }
   __syncthreads();
