@@ -286,7 +286,7 @@ constexpr int kEigStartSweeps = 6;
 template <int NMAX>
 constexpr int eig_start_threads() { return NMAX == 64 ? 512 : 256; }
 template <int NMAX>
-constexpr size_t eig_start_smem() {  // A, this round's rotations, all rounds' rotations
+constexpr size_t eig_start_smem() {  // A and all rounds' rotations
   return (size_t(NMAX) * (NMAX + 1) + 2 * size_t(kEigStartSweeps) * (NMAX - 1) * (NMAX / 2)) * sizeof(float);
 }
 
