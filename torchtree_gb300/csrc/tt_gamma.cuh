@@ -38,6 +38,16 @@ namespace tt {
 #define TT_HD
 #endif
 
+// acc + digamma of a >= 10
+TT_HD inline double digamma_tail(double a, double acc) {
+  const double r = 1.0 / a, r2 = r * r;
+  // ln a - 1/(2a) - sum_k B_2k / (2k a^2k), k = 1..6
+  const double series =
+      r2 * (1.0 / 12.0 - r2 * (1.0 / 120.0 - r2 * (1.0 / 252.0 - r2 * (1.0 / 240.0 - r2 * (1.0 / 132.0 -
+                                                                                          r2 * (691.0 / 32760.0))))));
+  return acc + log(a) - 0.5 * r - series;
+}
+
 // digamma for a > 0
 TT_HD inline double digamma_pos(double a) {
   double acc = 0.0;
@@ -45,12 +55,7 @@ TT_HD inline double digamma_pos(double a) {
     acc -= 1.0 / a;
     a += 1.0;
   }
-  const double r = 1.0 / a, r2 = r * r;
-  // ln a - 1/(2a) - sum_k B_2k / (2k a^2k), k = 1..6
-  const double series =
-      r2 * (1.0 / 12.0 - r2 * (1.0 / 120.0 - r2 * (1.0 / 252.0 - r2 * (1.0 / 240.0 - r2 * (1.0 / 132.0 -
-                                                                                          r2 * (691.0 / 32760.0))))));
-  return acc + log(a) - 0.5 * r - series;
+  return digamma_tail(a, acc);
 }
 
 // log(x^a e^-x / Gamma(a)).  For a >= 10 the large terms a ln x, x and
@@ -86,11 +91,12 @@ TT_HD inline bool gamma_p_series(double a, double x, double lga, double &p, doub
   return false;
 }
 
-// The iteration ends with a step below this share of x: Halley's method is of
-// third order, so the error left after such a step is rounding alone.  (A bound
-// at rounding itself, 4e-16, is met by chance only: the steps then wander by an
-// ulp or two until the iteration limit.)
-constexpr double kGammaStep = 1e-13;
+// The iteration ends with a step below kGammaStop of x, at most kGammaSteps steps, and
+// counts as converged when the last one is below kGammaStep.  Rounding leaves steps of
+// an ulp or two, so which of the neighbouring values the iteration ends with depends on
+// every rounding on its way.
+constexpr int kGammaSteps = 100;
+constexpr double kGammaStop = 4e-16, kGammaStep = 1e-13;
 
 // the starting point of the iteration (Numerical Recipes 6.2.1)
 TT_HD inline double gamma_start(double a, double q) {
@@ -109,13 +115,12 @@ TT_HD inline double gamma_start(double a, double q) {
   return x;
 }
 
-// Halley's step from x to xn, from p = P(a, x) and scale = x^a e^-x / Gamma(a);
-// false when the density is not usable
-TT_HD inline bool gamma_halley(double a, double q, double x, double p, double scale, double &xn) {
-  const double dfdx = scale / x;  // x^(a-1) e^-x / Gamma(a)
-  if (!(dfdx > 0.0) || !isfinite(dfdx)) return false;
-  const double u = (p - q) / dfdx;
-  xn = x - u / (1.0 - 0.5 * fmin(1.0, u * ((a - 1.0) / x - 1.0)));
+// Halley's step from x to xn, from p = P(a, x), the density x^(a-1) e^-x / Gamma(a) and
+// curve = (a - 1) / x; false when the density is not usable
+TT_HD inline bool gamma_step(double q, double x, double p, double density, double curve, double &xn) {
+  if (!(density > 0.0) || !isfinite(density)) return false;
+  const double u = (p - q) / density;
+  xn = x - u / (1.0 - 0.5 * fmin(1.0, u * (curve - 1.0)));
   if (xn <= 0.0) xn = 0.5 * x;
   return true;
 }
@@ -126,14 +131,14 @@ TT_HD inline bool gamma_quantile(double a, double q, double &x_out, double &dxda
   const double lga = lgamma(a);
   double x = gamma_start(a, q);
   double p = 0.0, z = 0.0, scale = 0.0, delta = 0.0;
-  for (int it = 0; it < 100; ++it) {
+  for (int it = 0; it < kGammaSteps; ++it) {
     if (!(x > 0.0)) x = 1e-300;
     if (!gamma_p_series(a, x, lga, p, z, scale)) return false;
     double xn;
-    if (!gamma_halley(a, q, x, p, scale, xn)) return false;
+    if (!gamma_step(q, x, p, scale / x, (a - 1.0) / x, xn)) return false;
     delta = fabs(xn - x);
     x = xn;
-    if (delta <= kGammaStep * x) break;
+    if (delta <= kGammaStop * x) break;
   }
   if (!(delta <= kGammaStep * x)) return false;
   if (!gamma_p_series(a, x, lga, p, z, scale)) return false;
@@ -143,117 +148,125 @@ TT_HD inline bool gamma_quantile(double a, double q, double &x_out, double &dxda
 }
 
 #ifdef __CUDACC__
-// The device form: one warp per quantile, every lane with the same a, q and x.
-// The serial series is a chain of two FP64 divisions and two multiplications
-// per term (2.0 ms for any batch that fits the GPU: the chain, not the
-// throughput, bounds it).  Here lane j holds term 32 c + j + 1 of chunk c: one
-// division per lane, the running product T_n and the harmonic sum H_n by warp
-// scans, the sums by butterflies (every lane ends with the same bits).  Most
-// quantiles of a site model need one chunk.  4 quantiles 1,094 -> 35 us, 256
-// quantiles 2,101 -> 37 us.
-__device__ inline bool gamma_p_series_warp(double a, double x, double lga, bool want_z, double &p, double &z,
-                                           double &scale) {
-  constexpr unsigned kAll = 0xffffffffu;
+// The device form: one warp per quantile, every lane with the same a, q and x, and
+// gamma_quantile's value to the last bit: FP32 transition matrices are rounded from
+// the category rates, and rates that move by 1e-16 take some of 1e8 entries to the
+// neighbouring FP32 value and gradients by 1e-9 with them.  So every rounding of the
+// serial form stays (its products and sums are not contracted), and the time goes out elsewhere:
+//  * the divisions of 28 terms and three more run at once, one per lane (an FP64
+//    division is nine instructions of 64 cycles, the chain of term and sum only two);
+//  * the sums stop where a term can no longer round into them, on the integer pipe;
+//  * an iteration that never comes below kGammaStop wanders through a few neighbouring
+//    values, the next a function of the last: the lanes keep all values, and once one
+//    comes back, where step kGammaSteps ends is known without taking the steps.
+// Shapes around 0.5, 4 categories: 1 / 16 / 64 samples 49 / 82 / 95 us (the longest of
+// their iterations).  One thread per quantile, every step taken: 1,094 us for 4
+// quantiles, 2,101 for 256.
+constexpr unsigned kGammaLanes = 0xffffffffu;
+constexpr int kGammaChunk = 28;  // terms per round of divisions; lanes 28 - 30 hold three other quotients
+
+__device__ __forceinline__ int gamma_exponent(double v) { return __double2hiint(v) >> 20; }  // biased; v >= 0
+
+// gamma_p_series and, for gamma_step, density = scale / x and curve = (a - 1) / x
+template <bool WANT_Z>
+__device__ __forceinline__ bool gamma_p_series_warp(double a, double x, double lga, double &p, double &z,
+                                                    double &scale, double &density, double &curve) {
   const int lane = threadIdx.x & 31;
   scale = exp(gamma_log_scale(a, x, lga));
-  double term = scale / a, h = 1.0 / a;  // of the last term added
-  p = term;
-  z = term * h;
-  for (int n0 = 1; n0 < 200000; n0 += 32) {
+  if (!isfinite(scale)) return false;
+  double term = 0.0, h = 0.0;  // of the last term added
+  for (int n0 = 1; n0 < 200000; n0 += kGammaChunk) {
     const double d = a + double(n0 + lane);
-    double prod = x / d, sum = want_z ? 1.0 / d : 0.0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double y = __shfl_up_sync(kAll, prod, o);
-      const double g = want_z ? __shfl_up_sync(kAll, sum, o) : 0.0;
-      if (lane >= o) {
-        prod *= y;
-        if (want_z) sum += g;
+    const double num = lane < kGammaChunk ? x : lane == 30 ? a - 1.0 : scale;
+    const double den = lane < kGammaChunk ? d : lane == 28 ? a : x;
+    const double ratio = num / den;
+    double inv = 0.0;
+    if constexpr (WANT_Z) inv = 1.0 / (lane < kGammaChunk ? d : a);
+    if (n0 == 1) {
+      p = term = __shfl_sync(kGammaLanes, ratio, 28);
+      density = __shfl_sync(kGammaLanes, ratio, 29);
+      curve = __shfl_sync(kGammaLanes, ratio, 30);
+      if constexpr (WANT_Z) {
+        h = __shfl_sync(kGammaLanes, inv, 28);
+        z = __dmul_rn(term, h);
       }
     }
-    const double tn = term * prod, hn = h + sum;
-    double ps = tn, zs = want_z ? tn * hn : 0.0;
+#pragma unroll 1
+    for (int j0 = 0; j0 < kGammaChunk; j0 += 4) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      ps += __shfl_xor_sync(kAll, ps, o);
-      if (want_z) zs += __shfl_xor_sync(kAll, zs, o);
+      for (int j = 0; j < 4; ++j) {
+        term = __dmul_rn(term, __shfl_sync(kGammaLanes, ratio, j0 + j));
+        p = __dadd_rn(p, term);
+        if constexpr (WANT_Z) {
+          h = __dadd_rn(h, __shfl_sync(kGammaLanes, inv, j0 + j));
+          z = __dadd_rn(z, __dmul_rn(term, h));
+        }
+      }
+      // a term below 2^-55 of the sum does not change it, nor do those after it
+      const int ep = gamma_exponent(p), et = gamma_exponent(term);
+      bool done = ep < 64 ? term <= p * 1e-17 : ep - et >= 56;  // (the exponents of tiny sums do not tell)
+      if constexpr (WANT_Z) {
+        const int ez = gamma_exponent(z), eh = gamma_exponent(h) - 1023;
+        done = done && (ez < 64 ? term * h <= z * 1e-17 : ez - (et + eh + 1) >= 56);
+      }
+      if (done) return true;
     }
-    p += ps;
-    z += zs;
-    term = __shfl_sync(kAll, tn, 31);
-    h = __shfl_sync(kAll, hn, 31);
-    if (term <= p * 1e-17 && (!want_z || term * h <= z * 1e-17)) return true;
   }
   return false;
 }
 
-// digamma for a > 0 by a warp: the recurrence's terms across the lanes
+// digamma_pos by a warp: the recurrence's divisions across the lanes, its sum in order
 __device__ inline double digamma_pos_warp(double a) {
-  const int m = a < 10.0 ? int(ceil(10.0 - a)) : 0, lane = threadIdx.x & 31;
-  double acc = lane < m ? 1.0 / (a + lane) : 0.0;
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);  // m <= 10: lanes 0-15
-  acc = __shfl_sync(0xffffffffu, acc, 0);
-  return digamma_pos(a + m) - acc;
-}
-
-// The quantile to about 1e-6 in FP32, by the same iteration: an FP64 step of it takes
-// about 3 us (64 cycles per instruction and SM quarter), an FP32 one a tenth of that.
-// 0 where FP32 does not serve: shapes outside [0.05, 20] (underflow, cancellation in
-// the scale) or no convergence.  Rates of one sample: 44 -> 26 us.
-__device__ inline float gamma_quantile_f32_warp(float a, float q, float lga, float x) {
-  constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  if (!(a >= 0.05f && a <= 20.0f && x > 1e-30f && x < 1e30f)) return 0.0f;
-  for (int it = 0; it < 12; ++it) {
-    const float scale = expf(a * logf(x) - x - lga);
-    float term = scale / a, p = term;
-    for (int n0 = 1; n0 < 512 && term > p * 1e-8f; n0 += 32) {
-      float prod = x / (a + float(n0 + lane));
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float y = __shfl_up_sync(kAll, prod, o);
-        if (lane >= o) prod *= y;
-      }
-      const float tn = term * prod;
-      float ps = tn;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) ps += __shfl_xor_sync(kAll, ps, o);
-      p += ps;
-      term = __shfl_sync(kAll, tn, 31);
-    }
-    const float dfdx = scale / x;
-    if (!(dfdx > 1e-30f) || !isfinite(dfdx)) return 0.0f;
-    const float u = (p - q) / dfdx;
-    float xn = x - u / (1.0f - 0.5f * fminf(1.0f, u * ((a - 1.0f) / x - 1.0f)));
-    if (xn <= 0.0f) xn = 0.5f * x;
-    const float delta = fabsf(xn - x);
-    x = xn;
-    if (!(x > 1e-30f) || !isfinite(x)) return 0.0f;
-    if (delta <= 1e-5f * x) return x;
+  double mine = a, acc = 0.0;
+  int m = 0;
+  for (; a < 10.0; ++m) {  // at most 10
+    if (lane == m) mine = a;
+    a += 1.0;
   }
-  return 0.0f;
+  const double inv = 1.0 / mine;
+  for (int j = 0; j < m; ++j) acc -= __shfl_sync(kGammaLanes, inv, j);
+  return digamma_tail(a, acc);
 }
 
 // gamma_quantile by a warp; the same result in every lane
 __device__ inline bool gamma_quantile_warp(double a, double q, double &x_out, double &dxda_out) {
   if (!(a > 0.0) || !(q > 0.0) || !(q < 1.0) || !isfinite(a)) return false;
+  const int lane = threadIdx.x & 31;
   const double lga = lgamma(a);
-  double x = gamma_start(a, q), p = 0.0, z = 0.0, scale = 0.0, delta = 0.0;
-  const float x32 = gamma_quantile_f32_warp(float(a), float(q), float(lga), float(x));
-  if (x32 > 0.0f) x = double(x32);
-  for (int it = 0; it < 100; ++it) {
+  double x = gamma_start(a, q), p = 0.0, z = 0.0, scale = 0.0, delta = 0.0, density = 0.0, curve = 0.0;
+  double seen[4] = {0.0, 0.0, 0.0, 0.0};  // the value at step 32 s + lane
+  static_assert(kGammaSteps <= 128, "four values per lane");
+  auto value_at = [&](int i) {
+    const int s = i >> 5;
+    return __shfl_sync(kGammaLanes, s == 0 ? seen[0] : s == 1 ? seen[1] : s == 2 ? seen[2] : seen[3], i & 31);
+  };
+  for (int it = 0; it < kGammaSteps; ++it) {
     if (!(x > 0.0)) x = 1e-300;
-    if (!gamma_p_series_warp(a, x, lga, false, p, z, scale)) return false;
+    int back = -1;  // the step that had this value
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const unsigned hit = __ballot_sync(kGammaLanes, seen[s] == x);
+      if (hit) back = 32 * s + __ffs(hit) - 1;
+    }
+    if (back >= 0) {  // no step of this cycle ends the iteration
+      const int period = it - back;
+      x = value_at(back + (kGammaSteps - back) % period);
+      delta = fabs(x - value_at(back + (kGammaSteps - 1 - back) % period));
+      break;
+    }
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+      if (it == 32 * s + lane) seen[s] = x;
+    if (!gamma_p_series_warp<false>(a, x, lga, p, z, scale, density, curve)) return false;
     double xn;
-    if (!gamma_halley(a, q, x, p, scale, xn)) return false;
+    if (!gamma_step(q, x, p, density, curve, xn)) return false;
     delta = fabs(xn - x);
     x = xn;
-    // an error of 1e-6 before the step is one of about 1e-18 after it (third order)
-    if (delta <= (x32 > 0.0f ? 1e-6 : kGammaStep) * x) break;
+    if (delta <= kGammaStop * x) break;
   }
-  if (!(delta <= (x32 > 0.0f ? 1e-6 : kGammaStep) * x)) return false;
-  if (!gamma_p_series_warp(a, x, lga, true, p, z, scale)) return false;
+  if (!(delta <= kGammaStep * x)) return false;
+  if (!gamma_p_series_warp<true>(a, x, lga, p, z, scale, density, curve)) return false;
   x_out = x;
   dxda_out = -x * (p * (log(x) - digamma_pos_warp(a)) - z) / scale;
   return true;
