@@ -350,7 +350,7 @@ struct Wide {
       }
       if constexpr (std::is_same<T, double>::value && SP == 64) {
         if (g.fine && wide_fine_level(nodes, p->batch * p->K, n)) {
-          wide_forward_kernel<T, SP, 16><<<dim3((n + 15) / 16, nodes, plan_run_samples(p) * p->K),
+          wide_forward_kernel<T, SP, 16><<<dim3(2 * g.ntiles_f, nodes, plan_run_samples(p) * p->K),
                                            WideCfg<T, SP, 16>::NT, wide_fwd_smem<T, SP, 16>(), s>>>(a);
           p->launches += 1;
           continue;
@@ -395,7 +395,7 @@ struct Wide {
         if (g.fine && wide_fine_level(nodes, bk, n)) {
           WideArgs<T> af = a;
           af.ntiles = (n + 15) / 16;
-          wide_backward_kernel<T, SP, 16><<<dim3(af.ntiles, nodes, plan_run_samples(p) * p->K),
+          wide_backward_kernel<T, SP, 16><<<dim3(2 * g.ntiles_b, nodes, plan_run_samples(p) * p->K),
                                             WideCfg<T, SP, 16>::NT, wide_bwd_smem<T, SP, 16>(), s>>>(af);
           p->launches += 1;
           continue;

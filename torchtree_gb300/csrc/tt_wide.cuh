@@ -73,6 +73,13 @@ constexpr int kTipRows = 4;
 template <typename T>
 constexpr bool kChildProducts = sizeof(T) == 8;
 
+// The instantiations for the FP64 codon levels that take tiles of 16 patterns
+// (wide_fine_level).  The node that such a level writes may be read in tiles of 32,
+// whose padding columns the gradient multiplies by 0: they have to be finite, so the
+// level is launched over whole tiles of 32 and a tile past the last pattern is cleared.
+template <typename T, int SP, int PT>
+constexpr bool kFineTiles = sizeof(T) == 8 && SP == 64 && PT == 16;
+
 // shared-memory bytes of the two kernels
 template <typename T, int SP, int PT>
 constexpr size_t wide_fwd_smem() {
@@ -259,6 +266,16 @@ __device__ __forceinline__ void wide_stage_child(const WideArgs<T> &a, int child
   }
 }
 
+// Zeros in columns [n0, n0 + PT) of an internal node's rows (and exponents).
+template <typename T, int SP, int PT>
+__device__ __forceinline__ void wide_clear_tile(const WideArgs<T> &a, T *rows, int *expo, int node, int b, int k, int n0) {
+  const size_t blk = (size_t(b) * a.I + (node - a.tips)) * a.K + k;
+  for (int e = threadIdx.x; e < SP * PT; e += WideCfg<T, SP, PT>::NT)
+    rows[(blk * SP + e / PT) * a.Npad + n0 + e % PT] = T(0);
+  if (expo)
+    for (int e = threadIdx.x; e < PT; e += WideCfg<T, SP, PT>::NT) expo[blk * a.Npad + n0 + e] = 0;
+}
+
 template <typename T>
 __device__ __forceinline__ int wide_child_expo(const WideArgs<T> &a, int child, int b, int k, int n) {
   return child < a.tips ? 0 : a.expo[((size_t(b) * a.I + (child - a.tips)) * a.K + k) * a.Npad + n];
@@ -350,6 +367,13 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT) wide_forward_kernel(co
   const int n0 = blockIdx.x * PT;
   const int l = a.left[v - a.tips], r = a.right[v - a.tips];
   const bool is_root = v == 2 * a.tips - 2;
+  if constexpr (kFineTiles<T, SP, PT>)
+    if (n0 >= a.N) {  // the rest of a 32-pattern tile past the last pattern
+      if (!is_root) wide_clear_tile<T, SP, PT>(a, a.part, a.expo, v, b, k, n0);
+      if (a.prod && l >= a.tips) wide_clear_tile<T, SP, PT>(a, a.prod, nullptr, l, b, k, n0);
+      if (a.prod && r >= a.tips) wide_clear_tile<T, SP, PT>(a, a.prod, nullptr, r, b, k, n0);
+      return;
+    }
 
   for (int e = tid; e < 2 * SP * SP; e += NT) {
     const int c = e / (SP * SP), ij = e - c * SP * SP, i = ij / SP, j = ij - i * SP;
@@ -534,6 +558,12 @@ __global__ void __launch_bounds__(WideCfg<T, SP, PT>::NT, wide_bwd_min_blocks<T,
   const int l = a.left[v - a.tips], r = a.right[v - a.tips];
   const bool is_root = v == 2 * a.tips - 2;
   const double wk = a.props[size_t(b) * a.K + k];
+  if constexpr (kFineTiles<T, SP, PT>)
+    if (chunk * PT >= a.N) {  // as in the post-order; nothing for the gradient
+      if (l >= a.tips) wide_clear_tile<T, SP, PT>(a, a.part, a.expo, l, b, k, chunk * PT);
+      if (r >= a.tips) wide_clear_tile<T, SP, PT>(a, a.part, a.expo, r, b, k, chunk * PT);
+      return;
+    }
 
   for (int e = tid; e < 2 * SP * SP; e += NT) {
     const int c = e / (SP * SP), ij = e - c * SP * SP, i = ij / SP, j = ij - i * SP;
