@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import torch
 
-from .substitution import device_eigen, eigen_of_normalised, normalise
+from .substitution import device_eigen, eigen_of_normalised
 
 
 def _scale(g: torch.Tensor, x: torch.Tensor, like: torch.Tensor) -> torch.Tensor:
@@ -117,20 +117,17 @@ class EvaluateLikelihood(torch.autograd.Function):
             eng.log_likelihood(p, f, rescale=ctx.rescale, keep_partials=True)
         if not torch.is_grad_enabled():
             return (*eng.evaluate_gradient(work, g, ctx.length_count, ctx.needs_input_grad[:5]), None, None)
-        # create_graph: the graph that the separate steps would leave (through g and the normalisation)
+        # create_graph: the graph that the separate steps would leave, through g and the normalisation
+        # Qn = Q / mu, mu = -sum_i pi_i Q_ii.  (Its derivatives are written out: autograd's own, asked for q
+        # and freqs at once, would give freqs what reaches it through q as well, which q's gradient carries.)
         lam, u, w, bl, r, p, f = eng.evaluation_parts(work)
         _, dpi, dc = eng.gradient(p, f)
         dq, dt, dr = eng.rate_matrix_gradient(lam, u, w, bl, r)
-        with torch.enable_grad():
-            ins = [t for t in (q, freqs) if t.requires_grad]
-            via = iter(torch.autograd.grad(normalise(q, freqs), ins, _scale(g, dq, q), create_graph=True)
-                       if ins else ())
-        gq = next(via) if q.requires_grad else None
-        gf = _scale(g, dpi, freqs)
-        if freqs.requires_grad:
-            gf = gf + next(via)
-        return (_scale(g, dt[:, :ctx.length_count], bl), gq, gf, _scale(g, dr, rates), _scale(g, dc, props), None,
-                None)
+        gn, diag = _scale(g, dq, q), torch.diagonal(q, dim1=-2, dim2=-1)
+        mu = -(diag * freqs).sum(-1)
+        s = ((gn * q).sum((-2, -1)) / (mu * mu)).unsqueeze(-1)  # -dL/dmu
+        return (_scale(g, dt[:, :ctx.length_count], bl), gn / mu[..., None, None] + torch.diag_embed(s * freqs),
+                _scale(g, dpi, freqs) + s * diag, _scale(g, dr, rates), _scale(g, dc, props), None, None)
 
 
 class MatrixLikelihood(torch.autograd.Function):

@@ -45,10 +45,13 @@ def _stream(t):
 
 
 def _again(compose, inputs, outputs_grad):
-    """Gradients of ``compose(*inputs)`` with a graph of their own."""
+    """Gradients of ``compose(*inputs)`` with a graph of their own.  Each with respect to an
+    alias: an input made from another one would pass its share on to that one here, and again
+    in the graph that this backward is part of."""
     with torch.enable_grad():
-        out = compose(*inputs)
-        want = [t for t in inputs if t.requires_grad]
+        own = [t.view_as(t) if t.requires_grad else t for t in inputs]
+        out = compose(*own)
+        want = [t for t in own if t.requires_grad]
         got = iter(torch.autograd.grad(out, want, outputs_grad, create_graph=True, allow_unused=True))
     return tuple(next(got) if t.requires_grad else None for t in inputs)
 
