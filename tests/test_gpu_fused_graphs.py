@@ -82,3 +82,19 @@ def test_rate_matrix_gradient_where_frequencies_depend_on_rates():
         outs.append((first, torch.autograd.grad((first * first).sum(), r)[0]))
     for a, b in zip(*outs):
         _close(a, b)
+
+
+@pytest.mark.parametrize("site", ["weibull", "gamma"])
+def test_batches_of_incoming_gradients(site):
+    """``is_grads_batched`` and the vectorised Jacobian, with and without a graph."""
+    fused, separate, leaves = _model(site)
+    eye = torch.eye(B, dtype=torch.float64, device="cuda")
+    outs = [torch.autograd.grad(f(*leaves), leaves, eye, is_grads_batched=True) for f in (fused, separate)]
+    for a, b in zip(*outs):
+        assert not a.requires_grad
+        _close(a, b)
+    for graph in (False, True):
+        outs = [torch.autograd.functional.jacobian(f, leaves, vectorize=True, create_graph=graph)
+                for f in (fused, separate)]
+        for a, b in zip(*outs):
+            _close(a, b)

@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import torch
 
+from .fused import plain_cuda
 from .substitution import device_eigen, eigen_of_normalised
 
 
@@ -115,9 +116,10 @@ class EvaluateLikelihood(torch.autograd.Function):
             lam, u, w, bl, r, p, f = eng.evaluation_parts(work)
             eng.set_eigen(lam, u, w, bl, r)
             eng.log_likelihood(p, f, rescale=ctx.rescale, keep_partials=True)
-        if not torch.is_grad_enabled():
+        if not torch.is_grad_enabled() and plain_cuda(g):
             return (*eng.evaluate_gradient(work, g, ctx.length_count, ctx.needs_input_grad[:5]), None, None)
-        # create_graph: the graph that the separate steps would leave, through g and the normalisation
+        # a batch of incoming gradients, or create_graph: tensor operations, and with them the graph that the
+        # separate steps would leave, through g and the normalisation
         # Qn = Q / mu, mu = -sum_i pi_i Q_ii.  (Its derivatives are written out: autograd's own, asked for q
         # and freqs at once, would give freqs what reaches it through q as well, which q's gradient carries.)
         lam, u, w, bl, r, p, f = eng.evaluation_parts(work)

@@ -16,7 +16,7 @@ from . import _native
 from ._native import check
 
 try:  # the transforms and modes under which an operation must stay a composition of tensor operations
-    from torch._C import _len_torch_dispatch_stack, _len_torch_function_stack
+    from torch._C import _has_storage, _len_torch_dispatch_stack, _len_torch_function_stack
     from torch._C._functorch import peek_interpreter_stack
     from torch.autograd import forward_ad
 except ImportError:  # a torch without these names: never take the kernels
@@ -32,7 +32,7 @@ def plain_cuda(*tensors) -> bool:
     first = tensors[0].device
     for t in tensors:
         if (type(t) not in (torch.Tensor, torch.nn.Parameter) or t.dtype != torch.float64 or t.device != first
-                or t.numel() == 0):
+                or t.numel() == 0 or not _has_storage(t)):  # (a batch of tensors has none)
             return False
     return (first.type == "cuda" and first.index == torch.cuda.current_device() and peek_interpreter_stack() is None
             and forward_ad._current_level < 0 and _len_torch_dispatch_stack() == 0
@@ -45,14 +45,15 @@ def _stream(t):
 
 
 def _again(compose, inputs, outputs_grad):
-    """Gradients of ``compose(*inputs)`` with a graph of their own.  Each with respect to an
+    """Gradients of ``compose(*inputs)``, with a graph of their own where one is wanted.  Each with respect to an
     alias: an input made from another one would pass its share on to that one here, and again
     in the graph that this backward is part of."""
+    create = torch.is_grad_enabled()
     with torch.enable_grad():
         own = [t.view_as(t) if t.requires_grad else t for t in inputs]
         out = compose(*own)
         want = [t for t in own if t.requires_grad]
-        got = iter(torch.autograd.grad(out, want, outputs_grad, create_graph=True, allow_unused=True))
+        got = iter(torch.autograd.grad(out, want, outputs_grad, create_graph=create, allow_unused=True))
     return tuple(next(got) if t.requires_grad else None for t in inputs)
 
 
@@ -79,6 +80,8 @@ class CategoryRates(torch.autograd.Function):
         shape, drates = ctx.saved_tensors
         if torch.is_grad_enabled():
             return (*_again(ctx.compose, (shape,), grad), None, None, None)
+        if not plain_cuda(grad):  # a batch of incoming gradients
+            return (grad * drates).sum(-1, keepdim=True), None, None, None
         grad = grad.contiguous()
         out = torch.empty(shape.shape, dtype=torch.float64, device=shape.device)
         check(_native.load().tt_rates_backward(shape.numel(), drates.shape[-1], grad.data_ptr(), drates.data_ptr(),
@@ -108,7 +111,7 @@ class ExchangeabilityQ(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         pi, *params = ctx.saved_tensors
-        if torch.is_grad_enabled():
+        if torch.is_grad_enabled() or not plain_cuda(grad):
             gpi, *rest = _again(lambda f, *p: ctx.compose(*p, f), (pi, *params), grad)
             return (gpi, None, None, *rest)
         b, S = pi.shape
