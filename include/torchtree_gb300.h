@@ -180,7 +180,9 @@ int tt_rate_matrix_gradient(tt_plan *plan, const double *eigenvalues,
 
 /*
  * Device status word: TT_OK, or TT_ERR_DEVICE_TIMEOUT when a kernel's
- * bounded wait gave up since the last reset.  Synchronises the stream.  No
+ * bounded wait gave up since the last reset, or TT_ERR_UNSUPPORTED when
+ * tt_evaluate met a rate matrix whose eigen system did not converge.
+ * Synchronises the stream.  No
  * reference counterpart: the reference has no device waits and reports
  * numeric trouble in-band (a -inf lnL, tree_likelihood.py:378-388).
  */
@@ -429,7 +431,8 @@ int tt_exchangeability_q_backward(int32_t batch, int32_t state_count,
  * weights with a row stride (0: one row for all samples).
  *   tt_evaluate_workspace: doubles of `work` (kept from tt_evaluate to
  *     tt_evaluate_gradient) and of `scratch`.
- *   tt_evaluate: tt_reversible_eigen + tt_update_transition_matrices +
+ *   tt_evaluate: tt_reversible_eigen (its status in the plan's status word,
+ *     tt_plan_device_status) + tt_update_transition_matrices +
  *     tt_log_likelihood; log_likelihood [b].
  *   tt_evaluate_gradient: tt_gradient + tt_rate_matrix_gradient, chained to
  *     the unnormalised rate matrix, each sample times grad_log_likelihood

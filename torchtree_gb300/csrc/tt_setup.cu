@@ -220,12 +220,12 @@ __global__ void __launch_bounds__(256) exch_q_backward_kernel(const __grid_const
 
 // ------------------------------------------------------- whole evaluations
 // What one evaluation leaves for its gradient (doubles, per plan): normalised
-// Q, mu, node lengths, rates, category weights, frequencies, eigen system, status.
+// Q, mu, node lengths, rates, category weights, frequencies, eigen system.
 struct Work {
-  double *qn, *mu, *bl, *rates, *props, *pi, *lam, *u, *w, *status;
+  double *qn, *mu, *bl, *rates, *props, *pi, *lam, *u, *w;
   static size_t count(const tt_plan *p) {
     const size_t b = p->batch, S = p->S;
-    return b * (3 * S * S + 2 * S + p->B + 2 * size_t(p->K) + 1) + 1;
+    return b * (3 * S * S + 2 * S + p->B + 2 * size_t(p->K) + 1);
   }
   Work(const tt_plan *p, double *base) {
     const size_t b = p->batch, S = p->S;
@@ -237,7 +237,7 @@ struct Work {
     };
     qn = take(b * S * S), u = take(b * S * S), w = take(b * S * S);
     lam = take(b * S), pi = take(b * S);
-    bl = take(b * p->B), rates = take(b * p->K), props = take(b * p->K), mu = take(b), status = take(1);
+    bl = take(b * p->B), rates = take(b * p->K), props = take(b * p->K), mu = take(b);
   }
 };
 
@@ -428,8 +428,7 @@ int tt_evaluate(tt_plan *p, const double *q, const double *frequencies, const do
   prepare_kernel<<<p->batch, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       q, frequencies, branch_lengths, lengths_per_sample, rates, category_weights, weights_stride, p->S, p->B, p->K, w);
   int rc = sdone(cudaGetLastError(), "evaluation set-up launch");
-  if (!rc)
-    rc = tt_reversible_eigen(p->batch, p->S, w.qn, w.pi, w.lam, w.u, w.w, reinterpret_cast<int32_t *>(w.status), stream);
+  if (!rc) rc = tt_reversible_eigen(p->batch, p->S, w.qn, w.pi, w.lam, w.u, w.w, p->d_status, stream);
   if (!rc) rc = tt_update_transition_matrices(p, w.lam, w.u, w.w, w.bl, w.rates, stream);
   if (!rc) rc = tt_log_likelihood(p, w.props, w.pi, rescale, keep_partials, log_likelihood, nullptr, stream);
   return rc;
