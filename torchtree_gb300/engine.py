@@ -62,7 +62,7 @@ class LikelihoodEngine:
         with torch.cuda.device(self.device):
             check(self.lib.tt_plan_set_tips(self._plan, ptr(codes), ptr(table), int(table.shape[0]),
                                             ptr(w)))
-        self.token = 0  # bumped by every forward that keeps partials
+        self.token = 0  # bumped by whatever the next gradient would read: matrices, partials
         self._eval_sizes = None  # doubles of evaluate's work and scratch buffers
 
     # ---------------------------------------------------------------- lifetime
@@ -120,6 +120,7 @@ class LikelihoodEngine:
         args = [_dev(x, self.device) for x in (lam, u, w, branch_lengths, rates)]
         self._check_shapes(*args)
         check(self.lib.tt_update_transition_matrices(self._plan, *map(ptr, args), _stream()))
+        self.token += 1
         self._keep = args  # keep alive until the launch has consumed them
 
     def set_matrices(self, mats):
@@ -129,6 +130,7 @@ class LikelihoodEngine:
         if tuple(m.shape) != exp:
             raise ValueError(f"matrices must have shape {exp}, got {tuple(m.shape)}")
         check(self.lib.tt_set_transition_matrices(self._plan, ptr(m), _stream()))
+        self.token += 1
         self._keep = [m]
 
     def log_likelihood(self, props, freqs, rescale: bool = True, keep_partials: bool = False,
@@ -141,8 +143,7 @@ class LikelihoodEngine:
                                device=self.device) if site else None
         check(self.lib.tt_log_likelihood(self._plan, ptr(p), ptr(f), int(rescale), int(keep_partials),
                                          ptr(out), ptr(site_out), _stream()))
-        if keep_partials:
-            self.token += 1
+        self.token += 1
         self._root_inputs = (p, f)
         return (out, site_out) if site else out
 
@@ -186,8 +187,7 @@ class LikelihoodEngine:
                                    rates.data_ptr(), props.data_ptr(), props.stride(0), rescale, keep_partials,
                                    work.data_ptr(), lnl.data_ptr(),
                                    torch.cuda.current_stream(self.device).cuda_stream))
-        if keep_partials:
-            self.token += 1
+        self.token += 1
         return lnl, work
 
     def evaluation_parts(self, work):
@@ -285,8 +285,7 @@ def plans_log_likelihood(engines, props, freqs, rescale: bool = True, keep_parti
         check(lib.tt_plans_log_likelihood(len(engines), plans, _ptr_array(p), _ptr_array(f), int(rescale),
                                           int(keep_partials), _ptr_array(outs), _stream()))
     for e, pi, fi in zip(engines, p, f):
-        if keep_partials:
-            e.token += 1
+        e.token += 1
         e._root_inputs = (pi, fi)
     return outs
 
