@@ -81,8 +81,8 @@ int tt_plan_workspace_bytes(const tt_plan *plan, size_t *bytes);
  *   codes:      host uint8 [T][N], every value < code_count
  *   code_table: host double [code_count][S], code_count <= 256
  *   weights:    host double [N] (the reference's int64 pattern counts)
- * A pass captured in a CUDA graph follows tips set anew with as many codes; it
- * has to be captured again when code_count changes.
+ * A pass captured in a CUDA graph follows tips that are set anew; a 4-state
+ * plan's has to be captured again when code_count changes.
  */
 int tt_plan_set_tips(tt_plan *plan, const uint8_t *codes,
                      const double *code_table, int32_t code_count,

@@ -72,7 +72,7 @@ struct WideState {
   void *d_gpart = nullptr;
   void *d_rootpart = nullptr;
   double *d_pgpart = nullptr;
-  uint8_t *d_tip_row = nullptr;  // [258] code -> row of the staged P^T (WideArgs::tip_row)
+  uint8_t *d_tip_row = nullptr;  // [259] code -> row of the staged P^T (WideArgs::tip_row)
   void *d_tip_amb = nullptr;     // [kTipRows][SP] the ambiguous code vectors
   void *d_prod = nullptr;  // the children's products of the post-order, read by the adjoint
 };
@@ -457,7 +457,7 @@ struct Wide {
       a.nodes = w.d_bwd + w.bwd_off[lv];
       a.tiles_per_chunk = (ntc + chunks - 1) / chunks;
       const dim3 grid(chunks, nodes, plan_run_samples(p) * p->K);
-      wide_backward_tc_kernel<<<grid, tcb::kThreads, tcb::kSmem, s>>>(a, maps, w.d_pimg, p->C, p->d_status,
+      wide_backward_tc_kernel<<<grid, tcb::kThreads, tcb::kSmem, s>>>(a, maps, w.d_pimg, p->d_status,
                                                                        2000000000ull);
       p->launches += 1;
     }
@@ -580,7 +580,7 @@ int wide_create(tt_plan *p) {
   if (!rc) rc = walloc(p, &w->d_branch_lvn, size_t(p->B) * sizeof(int), "branch levels");
   if (!rc) rc = walloc(p, &p->d_codes, size_t(T) * p->code_stride, "tip codes");
   if (!rc) rc = walloc(p, &p->d_table, 256 * SP * es, "code table");
-  if (!rc) rc = walloc(p, &w->d_tip_row, 258, "tip rows");
+  if (!rc) rc = walloc(p, &w->d_tip_row, 259, "tip rows");
   if (!rc) rc = walloc(p, &w->d_tip_amb, kTipRows * SP * es, "ambiguous code vectors");
   if (!rc) rc = walloc(p, &p->d_weights, size_t(p->N) * sizeof(double), "weights");
   if (!rc) rc = walloc(p, &p->d_pmat, b * p->B * K * SP * SP * es, "transition matrices");
@@ -788,7 +788,7 @@ int wide_set_tips(tt_plan *p, const uint8_t *codes, const double *code_table, in
     }
   // codes whose product is a row of the staged P^T: unit vectors, and the first kTipRows others
   WideState &w = *p->wide;
-  std::vector<uint8_t> rows(258, 0);
+  std::vector<uint8_t> rows(259, 0);
   std::vector<unsigned char> amb(size_t(kTipRows) * SP * p->elem, 0);
   int ambs = 0;
   bool ok = true;
@@ -819,6 +819,7 @@ int wide_set_tips(tt_plan *p, const uint8_t *codes, const double *code_table, in
   }
   rows[256] = ok;
   rows[257] = uint8_t(ambs);
+  rows[258] = uint8_t(code_count - 1);
   cudaError_t e = cudaMemset(p->d_codes, 0, size_t(p->T) * p->code_stride);
   if (e == cudaSuccess) e = cudaMemcpy(w.d_tip_row, rows.data(), rows.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(w.d_tip_amb, amb.data(), amb.size(), cudaMemcpyHostToDevice);

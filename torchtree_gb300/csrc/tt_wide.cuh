@@ -221,7 +221,8 @@ struct WideArgs {
   const uint8_t *codes;     // [tips][code_stride]
   const T *table;           // [C][SP]
   // [256] row of the staged P^T that is the code's product; [256] whether every code has one, [257] how
-  // many ambiguous codes: read on the device, so that a captured pass follows tips that are set anew
+  // many ambiguous codes, [258] how many codes less one: read on the device, so that a captured pass follows
+  // tips that are set anew
   const uint8_t *tip_row;
   const T *tip_amb;         // [kTipRows][SP] code vectors of rows SP .. SP + tip_row[257] - 1
   const T *pmat;            // [b][B][K][SP][SP]
@@ -279,6 +280,11 @@ __device__ __forceinline__ void wide_clear_tile(const WideArgs<T> &a, T *rows, i
 template <typename T>
 __device__ __forceinline__ int wide_child_expo(const WideArgs<T> &a, int child, int b, int k, int n) {
   return child < a.tips ? 0 : a.expo[((size_t(b) * a.I + (child - a.tips)) * a.K + k) * a.Npad + n];
+}
+
+template <typename T>
+__device__ __forceinline__ int wide_code_count(const WideArgs<T> &a) {
+  return 1 + int(__ldg(a.tip_row + 258));
 }
 
 // Largest non-negative value of a column through shared memory: values as they

@@ -175,8 +175,16 @@ __global__ void __launch_bounds__(kColThreads, 3) wide_col_forward_kernel(const 
 #pragma unroll
         for (int q = 0; q < PP; ++q) {
           const int code = cd[q];
-          if (codes > 0) {
+          if (code < codes) {
             y[q].load(tb + (c * codes + code) * SP);
+          } else if (codes > 0) {  // more codes than when this pass was captured
+#pragma unroll
+            for (int i = 0; i < SP; ++i) {
+              T acc = T(0);
+#pragma unroll 1
+              for (int j = 0; j < SP; ++j) acc = fma(pt[c * SP * SP + i * SP + j], a.table[code * SP + j], acc);
+              y[q].set(i, acc);
+            }
           } else {
             y[q].zero();
             for (int j = 0; j < SP; ++j) y[q].fma_row(pt + c * SP * SP + j * SP, a.table[code * SP + j]);

@@ -221,12 +221,28 @@ __global__ void __launch_bounds__(tc::kThreads, 2)
   if (warp == 0) tc::tmem_dealloc(tmem, tc::kTmemCols);
 }
 
-// 32 consecutive products of a tip's code, from its table row
-__device__ __forceinline__ void tc_tip_row(const float *row, float (&v)[32]) {
+// row i of a child's P times a code's vector: for a code that the table of products does not hold, as
+// tips set anew under a captured pass may have
+__device__ __forceinline__ float tc_tip_product(const WideArgs<float> &a, int child, int b, int k, int code, int i) {
+  const float *P = a.pmat + (((size_t(b) * a.B + child) * a.K + k) * 64 + i) * 64, *x = a.table + size_t(code) * 64;
+  float s = 0.0f;
+#pragma unroll 1
+  for (int j = 0; j < 64; ++j) s = fmaf(P[j], x[j], s);
+  return s;
+}
+
+// products i0 .. i0 + 31 of a tip's code, from its table (`codes` rows)
+__device__ __forceinline__ void tc_tip_row(const WideArgs<float> &a, const float *tab, int codes, int child, int b,
+                                           int k, int code, int i0, float (&v)[32]) {
+  if (code < codes) {
 #pragma unroll
-  for (int i = 0; i < 32; i += 4) {
-    const float4 t = __ldg(reinterpret_cast<const float4 *>(row + i));
-    v[i] = t.x, v[i + 1] = t.y, v[i + 2] = t.z, v[i + 3] = t.w;
+    for (int i = 0; i < 32; i += 4) {
+      const float4 t = __ldg(reinterpret_cast<const float4 *>(tab + code * 64 + i0 + i));
+      v[i] = t.x, v[i + 1] = t.y, v[i + 2] = t.z, v[i + 3] = t.w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = tc_tip_product(a, child, b, k, code, i0 + i);
   }
 }
 
@@ -369,15 +385,15 @@ __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const 
       const int n = n0 + tid;
       float *pd = a.prod ? a.prod + ((size_t(b) * a.I + (v - a.tips)) * a.K + k) * 2 * SP * size_t(a.Npad) + n
                          : nullptr;
-      const float *row_l = tab_l ? tab_l + min(int(a.codes[size_t(l) * a.code_stride + n]), codes - 1) * SP : nullptr;
-      const float *row_r = tab_r ? tab_r + min(int(a.codes[size_t(r) * a.code_stride + n]), codes - 1) * SP : nullptr;
+      const int code_l = tab_l ? a.codes[size_t(l) * a.code_stride + n] : 0;
+      const int code_r = tab_r ? a.codes[size_t(r) * a.code_stride + n] : 0;
       float L[64];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         float dl[32], dr[32];
-        if (tab_l) tc_tip_row(row_l + 32 * h, dl);
+        if (tab_l) tc_tip_row(a, tab_l, codes, l, b, k, code_l, 32 * h, dl);
         else tc::tmem_ld32(lane_addr + uint32_t(32 * h), dl);
-        if (tab_r) tc_tip_row(row_r + 32 * h, dr);
+        if (tab_r) tc_tip_row(a, tab_r, codes, r, b, k, code_r, 32 * h, dr);
         else tc::tmem_ld32(lane_addr + uint32_t(64 + 32 * h), dr);
         if (pd) {  // the children's products for the adjoint
 #pragma unroll
@@ -457,14 +473,21 @@ __global__ void __launch_bounds__(kTipPairThreads) wide_tip_pair_kernel(const Wi
   const int t0 = blockIdx.x * a.tiles_per_chunk, t1 = min(a.ntiles, t0 + a.tiles_per_chunk);
   for (int tile = t0; tile < t1; ++tile) {
     const int n = tile * kTipPairThreads + tid;
-    const float *row_l = tab + min(int(a.codes[size_t(l) * a.code_stride + n]), codes - 1) * ST;
-    const float *row_r = tab + (codes + min(int(a.codes[size_t(r) * a.code_stride + n]), codes - 1)) * ST;
+    const int code_l = a.codes[size_t(l) * a.code_stride + n], code_r = a.codes[size_t(r) * a.code_stride + n];
+    const float *row_l = tab + min(code_l, codes - 1) * ST, *row_r = tab + (codes + min(code_r, codes - 1)) * ST;
     float *pd = a.prod ? a.prod + blk * 2 * SP * npad + n : nullptr;
     float L[SP], m = 0.0f;
 #pragma unroll
     for (int i = 0; i < SP; i += 4) {
       const float4 x = *reinterpret_cast<const float4 *>(row_l + i), y = *reinterpret_cast<const float4 *>(row_r + i);
-      const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+      float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+      if (max(code_l, code_r) >= codes) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          xs[t] = tc_tip_product(a, l, b, k, code_l, i + t);
+          ys[t] = tc_tip_product(a, r, b, k, code_r, i + t);
+        }
+      }
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
         if (pd) {

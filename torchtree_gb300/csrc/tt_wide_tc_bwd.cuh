@@ -243,7 +243,7 @@ __device__ __forceinline__ bool conv_sync_any(bool flag) {
 // a.nchunks count 128-pattern tiles.
 __global__ void __launch_bounds__(tcb::kThreads, 1)
     wide_backward_tc_kernel(const WideArgs<float> a, const __grid_constant__ TcbMaps maps, const float *pimg,
-                            int code_count, int *status, unsigned long long timeout_ns) {
+                            int *status, unsigned long long timeout_ns) {
   using namespace tcb;
   constexpr int SP = 64, PT = kPT;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -461,6 +461,7 @@ __global__ void __launch_bounds__(tcb::kThreads, 1)
     // a tip child's rows of the code table: as bit masks in shared memory when every entry is 0 or 1
     // (the encodings' indicator rows) and the table is small, else read from global memory
     uint2 *tabm = reinterpret_cast<uint2 *>(smem + kOffTab);
+    const int code_count = wide_code_count(a);
     bool tab_bits = (!int0 || !int1) && code_count <= kTabRows;
     if (tab_bits) {
       bool binary = true;
