@@ -50,8 +50,8 @@ struct WideState {
   // the images hold the current transition matrices (written right after them, in one pass)
   bool img_f_valid = false, img_b_valid = false;
   // tip products of the tensor-core post-order, [b][tips][K][64 or 128 codes][64]: one for either
-  // capacity, allocated with the first tips that need it and kept (a captured pass may hold it);
-  // a plan with more codes, or without the memory, sends its tips through the MMAs
+  // capacity, allocated with the first tips whose passes use it (tip_table) and kept (a captured pass may
+  // hold it); a plan with more codes, or without the memory, sends its tips through the MMAs
   float *d_tprod[2] = {nullptr, nullptr};
   // pattern slabs (p->slab != 0): the pattern-sized buffers below hold one
   // slab; tail_valid = they still hold the last slab's post-order (from a
@@ -174,6 +174,16 @@ int walloc(tt_plan *p, P **ptr, size_t bytes, const char *what) {
   return TT_OK;
 }
 
+// Whether an FP32 codon pass of ntf 128-pattern tiles takes its tips' products from a table by
+// code: it costs each tip one tile and the pass a launch, and saves the products of all the tip's
+// tiles.  Post-order of 200 taxa, without and with it: 4 categories, 1 sample, 250 / 510 / 800 /
+// 1,500 patterns 216, 230 / 273, 273 / 363, 353 / 518, 475 us; 8 samples, 380 / 510 / 800 patterns
+// 894, 913 / 1,123, 1,108 / 1,835, 1,684 us; 1 category, 1 sample (launch-bound), 800 / 1,500
+// patterns 210, 214 / 244, 238 us.
+bool tip_table_pays(const tt_plan *p, int samples, int ntf) {
+  return ntf >= 6 && size_t(p->T) * samples * p->K * ntf >= 2048;
+}
+
 // compiled (precision, padded states) -> pattern tiles of the two passes
 void tiles_for(bool f32, int SP, int &ptf, int &ptb) {
   if (SP == 20) {
@@ -285,14 +295,8 @@ struct Wide {
     const float *tprod = nullptr;
     const int tcodes = p->C <= 64 ? 64 : 128;
     if constexpr (std::is_same<T, float>::value && SP == 64) {
-      // The tips' products by code, with every pass (a captured one has to follow the matrices).  The
-      // table costs each tip one tile and the pass a launch, and saves the products of all the tip's
-      // tiles.  Post-order of 200 taxa, without and with it: 4 categories, 1 sample, 250 / 510 / 800 /
-      // 1,500 patterns 216, 230 / 273, 273 / 363, 353 / 518, 475 us; 8 samples, 380 / 510 / 800 patterns
-      // 894, 913 / 1,123, 1,108 / 1,835, 1,684 us; 1 category, 1 sample (launch-bound), 800 / 1,500
-      // patterns 210, 214 / 244, 238 us.
-      const int ntf = g.Npad / tc::kPT;
-      if (w.tc && w.d_pimg_f && p->C <= 128 && ntf >= 6 && size_t(p->T) * plan_run_samples(p) * p->K * ntf >= 2048)
+      // the tips' products by code, with every pass (a captured one has to follow the matrices)
+      if (w.tc && w.d_pimg_f && p->C <= 128 && tip_table_pays(p, plan_run_samples(p), g.Npad / tc::kPT))
         tprod = w.d_tprod[tcodes / 128];
       if (tprod) {
         wide_tip_products_tc_kernel<<<dim3(p->T, plan_run_samples(p) * p->K), tc::kThreads, tc::kSmem, s>>>(
@@ -651,10 +655,11 @@ SlabBuffers slab_buffers(const tt_plan *p, int n, bool slab) {
   return x;
 }
 
-// Whether an FP64 plan keeps its internal children's products beside buffers of `total` bytes: they save
-// the adjoint a third of its products and are as large as the partials.  They are
-// no reason for slabs (choose_slab does not count them): kept if they take at most a quarter of the
-// device's free memory and stay within TT_GRADIENT_BUDGET_BYTES.
+// Whether there is room for `bytes` beside pattern buffers of `total` bytes, for what a plan can do without:
+// FP64 plans' products of internal children (they save the adjoint a third of its products and are as large
+// as the partials) and FP32 codon plans' tip products.  Neither is a reason for slabs (choose_slab does not
+// count them): kept if they take at most a quarter of the device's free memory and stay within
+// TT_GRADIENT_BUDGET_BYTES.
 bool product_room(size_t bytes, size_t total) {
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
@@ -679,6 +684,24 @@ void free_slab_buffers(tt_plan *p) {
     }
   p->bytes -= std::min(p->bytes, w.slab_bytes);
   w.slab_bytes = 0;
+}
+
+}  // namespace
+
+namespace {
+
+// The table of tip products of an FP32 codon plan with `codes` tip codes, where its passes use one and there
+// is room (without it the tips take products).  Never given back before the plan: a captured pass may hold it.
+void tip_table(tt_plan *p, int codes) {
+  WideState &w = *p->wide;
+  if (p->precision != TT_PRECISION_F32 || w.SP != 64 || codes > 128) return;
+  const int cap = codes <= 64 ? 64 : 128;
+  float *&tprod = w.d_tprod[cap / 128];
+  const size_t bytes = size_t(p->batch) * p->T * p->K * cap * w.SP * sizeof(float);
+  if (tprod || !tip_table_pays(p, p->batch, ((p->slab ? p->slab : p->N) + tc::kPT - 1) / tc::kPT) ||
+      !product_room(bytes, w.slab_bytes))
+    return;
+  if (walloc(p, &tprod, bytes, "tip products")) tprod = nullptr;
 }
 
 }  // namespace
@@ -713,6 +736,7 @@ int wide_alloc_slab(tt_plan *p, int slab) {
     return rc;
   }
   p->slab = slab;
+  if (p->tips_set) tip_table(p, p->C);
   return TT_OK;
 }
 
@@ -809,14 +833,7 @@ int wide_set_tips(tt_plan *p, const uint8_t *codes, const double *code_table, in
       ok = false;
     }
   }
-  if (p->precision == TT_PRECISION_F32 && SP == 64 && code_count <= 128) {
-    const int cap = code_count <= 64 ? 64 : 128;
-    float *&tprod = w.d_tprod[cap / 128];
-    if (!tprod && walloc(p, &tprod, size_t(p->batch) * p->T * p->K * cap * SP * sizeof(float), "tip products")) {
-      tprod = nullptr;
-      cudaGetLastError();
-    }
-  }
+  tip_table(p, code_count);
   rows[256] = ok;
   rows[257] = uint8_t(ambs);
   rows[258] = uint8_t(code_count - 1);
