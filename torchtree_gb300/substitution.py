@@ -155,7 +155,7 @@ UNIVERSAL_CODE = "KNKNTTTTRSRSIIMIQHQHPPPPRRRRLLLLEDEDAAAAGGGGVVVV*Y*YSSSS*CWCLF
 
 def codon_pair_masks(table: str = UNIVERSAL_CODE):
     """MG94 pair classes over sense-codon pairs in combinations order (codon.py:33-55)."""
-    ts, syn, nonsyn, m = _codon_pair_masks(table)
+    ts, syn, nonsyn, m = _codon_pair_masks(tuple(table))
     return ts.clone(), syn.clone(), nonsyn.clone(), m
 
 
@@ -182,7 +182,7 @@ def mg94_q(alpha, beta, kappa, pi, table: str = UNIVERSAL_CODE) -> torch.Tensor:
     """MG94 as torchtree computes it (codon.py:57-77): exchangeability
     kappa^ts alpha^syn beta^nonsyn; pairs differing at 2-3 positions get 1."""
     if _one_launch(pi, pi.shape[-1], alpha, beta, kappa, scalars=True):
-        index, m = _mg94_index(table)
+        index, m = _mg94_index(tuple(table))
         if m == pi.shape[-1]:
             return fused.ExchangeabilityQ.apply(pi, index, lambda a, b, k, f: _mg94(a, b, k, f, table), alpha, beta,
                                                 kappa)
