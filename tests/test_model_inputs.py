@@ -12,3 +12,11 @@ def test_codon_tables_as_sequences():
         one = torch.ones(1, dtype=torch.float64)
         pi = torch.full((61,), 1.0 / 61, dtype=torch.float64)
         assert torch.equal(sub.mg94_q(one, 2.0 * one, 3.0 * one, pi, table), sub.mg94_q(one, 2.0 * one, 3.0 * one, pi))
+
+
+def test_mg94_with_one_frequency_for_all_codons():
+    from torchtree_gb300 import substitution as sub
+
+    one = torch.ones(1, dtype=torch.float64)
+    pi = torch.tensor(1.0 / 61, dtype=torch.float64)
+    assert torch.equal(sub.mg94_q(one, 2.0 * one, 3.0 * one, pi), sub.mg94_q(one, 2.0 * one, 3.0 * one, pi.expand(61)))

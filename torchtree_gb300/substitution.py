@@ -181,7 +181,7 @@ def _codon_pair_masks(table):
 def mg94_q(alpha, beta, kappa, pi, table: str = UNIVERSAL_CODE) -> torch.Tensor:
     """MG94 as torchtree computes it (codon.py:57-77): exchangeability
     kappa^ts alpha^syn beta^nonsyn; pairs differing at 2-3 positions get 1."""
-    if _one_launch(pi, pi.shape[-1], alpha, beta, kappa, scalars=True):
+    if pi.dim() == 2 and _one_launch(pi, pi.shape[1], alpha, beta, kappa, scalars=True):
         index, m = _mg94_index(tuple(table))
         if m == pi.shape[-1]:
             return fused.ExchangeabilityQ.apply(pi, index, lambda a, b, k, f: _mg94(a, b, k, f, table), alpha, beta,
