@@ -35,8 +35,8 @@ def _finish(rates, categories, invariant, mu):
 
 def _one_launch(shape, categories, invariant, mu) -> bool:
     """The plain model of FP64 device shapes: rates, weights and shape derivative from one kernel."""
-    return (invariant is None and mu is None and 1 <= categories <= 32 and shape.dim() > 0 and shape.shape[-1] == 1
-            and fused.plain_cuda(shape))
+    return (invariant is None and mu is None and isinstance(categories, int) and 1 <= categories <= 32
+            and shape.dim() > 0 and shape.shape[-1] == 1 and fused.plain_cuda(shape))
 
 
 def _fused_rates(shape, categories, kind, compose):
