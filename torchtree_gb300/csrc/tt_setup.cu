@@ -74,7 +74,8 @@ __global__ void __launch_bounds__(32) weibull_rates_kernel(const double *shape, 
   const int b = blockIdx.x, k = threadIdx.x;
   double r = 0.0, dr = 0.0;
   if (k < K) {
-    const double q = (2.0 * k + 1.0) / (2.0 * K), x = -log(1.0 - q), inv = 1.0 / shape[b];
+    // (a tensor over a number is multiplied by the number's reciprocal)
+    const double q = __dmul_rn(2.0 * k + 1.0, 1.0 / (2.0 * K)), x = -log(1.0 - q), inv = 1.0 / shape[b];
     r = pow(x, inv);
     dr = -r * log(x) * inv * inv;
   }
