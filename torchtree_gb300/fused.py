@@ -24,7 +24,7 @@ except ImportError:  # a torch without these names: never take the kernels
 
 
 def plain_cuda(*tensors) -> bool:
-    """Whether every tensor is an ordinary non-empty FP64 CUDA tensor of the
+    """Whether every tensor is an ordinary non-empty FP64 CUDA tensor (no lazy negation) of the
     current device, used outside of transforms (vmap, forward mode), modes,
     tracing and compilation."""
     if peek_interpreter_stack is None:
@@ -32,7 +32,7 @@ def plain_cuda(*tensors) -> bool:
     first = tensors[0].device
     for t in tensors:
         if (type(t) not in (torch.Tensor, torch.nn.Parameter) or t.dtype != torch.float64 or t.device != first
-                or t.numel() == 0 or not _has_storage(t)):  # (a batch of tensors has none)
+                or t.numel() == 0 or t.is_neg() or not _has_storage(t)):  # (a batch of tensors has none)
             return False
     return (first.type == "cuda" and first.index == torch.cuda.current_device() and peek_interpreter_stack() is None
             and forward_ad._current_level < 0 and _len_torch_dispatch_stack() == 0

@@ -82,7 +82,7 @@ class PhyloLikelihood:
         b, S, K = self.batch, self.state_count, self.category_count
         for t, shape in ((branch_lengths, (b, self.engine.branch_count - 1)), (q, (b, S, S)), (frequencies, (b, S)),
                          (rates, (b, K)), (props, (b, K))):
-            if t.dtype != torch.float64 or t.device != self.device or t.shape != shape:
+            if t.dtype != torch.float64 or t.device != self.device or t.shape != shape or t.is_neg():
                 return False
         return (branch_lengths.is_contiguous() and q.is_contiguous() and frequencies.is_contiguous()
                 and rates.is_contiguous() and (K == 1 or props.stride(1) == 1)
