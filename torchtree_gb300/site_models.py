@@ -70,7 +70,7 @@ class _GammaQuantile(torch.autograd.Function):
         from . import _native
 
         lib = _native.load()
-        a = alpha.detach().to(torch.float64).reshape(-1).contiguous()
+        a = alpha.detach().resolve_neg().to(torch.float64).reshape(-1).contiguous()
         b = a.shape[0]
         x = torch.empty(b, categories, dtype=torch.float64, device=alpha.device)
         dx = torch.empty_like(x)
