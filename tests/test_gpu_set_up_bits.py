@@ -58,3 +58,24 @@ def test_normalised_matrix_and_eigen_system_of_an_evaluation(S, b):
     assert torch.equal(work[:q.numel()].view_as(q), qn)
     for got, want in zip(eng.evaluation_parts(work), sub.device_eigen(qn, pi)):
         assert torch.equal(got, want)
+
+
+def test_numbers_that_are_not_finite():
+    """NaN and infinities go where the compositions put them, zeros keep their sign."""
+    from torchtree_gb300 import site_models, substitution as sub
+
+    rng = np.random.default_rng(5)
+    odd = [np.nan, np.inf, -np.inf, 0.0, -0.0, 1e-310]
+    r, pi = rng.gamma(1.0, 1.0, (12, 6)), rng.dirichlet(5.0 * np.ones(4), 12)
+    for i, v in enumerate(odd):
+        r[i, i % 6] = v
+        pi[6 + i, i % 4] = v
+    for got, want in ((sub.gtr_q(_t(r), _t(pi)), sub._general(_t(r), _t(pi), 4)),
+                      (sub.hky_q(_t(r[:, :1]), _t(pi)), sub._hky(_t(r[:, :1]), _t(pi)))):
+        np.testing.assert_array_equal(got.cpu().numpy(), want.cpu().numpy())
+        np.testing.assert_array_equal(np.signbit(got.cpu().numpy()), np.signbit(want.cpu().numpy()))
+    shape = _t(np.array(odd + [-1.0, 1e300, 1e-3])[:, None])
+    for kind in ("weibull", "gamma"):
+        for k in (1, 4, 6):
+            rates, _ = getattr(site_models, kind + "_rates")(shape, k)
+            np.testing.assert_array_equal(rates.cpu().numpy(), getattr(site_models, "_" + kind)(shape, k)[0].cpu().numpy())

@@ -140,9 +140,10 @@ struct Exch {
     }
     return reinterpret_cast<const int8_t *>(sm);
   }
+  // (plus 0: the composition adds the upper triangle to a transposed one of zeros, so no -0)
   __device__ __forceinline__ double value(int b, const int8_t *m, int e) const {
-    if constexpr (kMapped) return param(b, m[e]) * param(b, m[count + e]);
-    else return p[0][size_t(b) * n[0] + e];
+    if constexpr (kMapped) return __dadd_rn(__dmul_rn(param(b, m[e]), param(b, m[count + e])), 0.0);
+    else return __dadd_rn(p[0][size_t(b) * n[0] + e], 0.0);
   }
 };
 
@@ -164,9 +165,9 @@ __global__ void __launch_bounds__(256) exch_q_kernel(const __grid_constant__ Exc
   }
   for (int i = threadIdx.x >> 5; i < S; i += blockDim.x >> 5) {
     const double s = row_sum(S, [&](int j) {
-      return j == i ? 0.0 : __dmul_rn(x.value(b, m, upper_index(i, j, S)), pb[j]);
+      return __dmul_rn(j == i ? 0.0 : x.value(b, m, upper_index(i, j, S)), pb[j]);  // (0 of a NaN or infinity is NaN)
     });
-    if ((threadIdx.x & 31) == 0) qb[i * S + i] = -s;
+    if ((threadIdx.x & 31) == 0) qb[i * S + i] = __dsub_rn(__dmul_rn(0.0, pb[i]), s);
   }
 }
 
