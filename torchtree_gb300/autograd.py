@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import torch
 
-from .fused import plain_cuda
+from .fused import plain_gradient
 from .substitution import device_eigen, eigen_of_normalised
 
 
@@ -116,7 +116,7 @@ class EvaluateLikelihood(torch.autograd.Function):
             lam, u, w, bl, r, p, f = eng.evaluation_parts(work)
             eng.set_eigen(lam, u, w, bl, r)
             eng.log_likelihood(p, f, rescale=ctx.rescale, keep_partials=True)
-        if not torch.is_grad_enabled() and plain_cuda(g):
+        if not torch.is_grad_enabled() and plain_gradient(g):
             return (*eng.evaluate_gradient(work, g, ctx.length_count, ctx.needs_input_grad[:5]), None, None)
         # a batch of incoming gradients, or create_graph: tensor operations, and with them the graph that the
         # separate steps would leave, through g and the normalisation

@@ -22,6 +22,9 @@ try:  # the transforms and modes under which an operation must stay a compositio
 except ImportError:  # a torch without these names: never take the kernels
     peek_interpreter_stack = None
 
+    def _has_storage(_):
+        return False
+
 
 def plain_cuda(*tensors) -> bool:
     """Whether every tensor is an ordinary non-empty FP64 CUDA tensor (no lazy negation) of the
@@ -38,6 +41,12 @@ def plain_cuda(*tensors) -> bool:
             and forward_ad._current_level < 0 and _len_torch_dispatch_stack() == 0
             and _len_torch_function_stack() == 0 and not torch.jit.is_tracing()
             and not torch.compiler.is_compiling())
+
+
+def plain_gradient(g) -> bool:
+    """Whether a backward's incoming gradient (of a plain output's type and device) is an
+    ordinary tensor: no batch of them, no lazy negation."""
+    return type(g) is torch.Tensor and _has_storage(g) and not g.is_neg()
 
 
 def _stream(t):
@@ -80,7 +89,7 @@ class CategoryRates(torch.autograd.Function):
         shape, drates = ctx.saved_tensors
         if torch.is_grad_enabled():
             return (*_again(ctx.compose, (shape,), grad), None, None, None)
-        if not plain_cuda(grad):  # a batch of incoming gradients
+        if not plain_gradient(grad):  # a batch of incoming gradients
             return (grad * drates).sum(-1, keepdim=True), None, None, None
         grad = grad.contiguous()
         out = torch.empty(shape.shape, dtype=torch.float64, device=shape.device)
@@ -111,7 +120,7 @@ class ExchangeabilityQ(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         pi, *params = ctx.saved_tensors
-        if torch.is_grad_enabled() or not plain_cuda(grad):
+        if torch.is_grad_enabled() or not plain_gradient(grad):
             gpi, *rest = _again(lambda f, *p: ctx.compose(*p, f), (pi, *params), grad)
             return (gpi, None, None, *rest)
         b, S = pi.shape
