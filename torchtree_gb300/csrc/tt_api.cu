@@ -504,12 +504,10 @@ int tt_plan_create(tt_plan **plan, int32_t tip_count, const int32_t *postorder,
     const int slots = bwd ? p->slots_bwd : p->slots_fwd;
     const int ns = bwd ? p->nstage_b : p->nstage_f;
     return std::max({tt::tl_smem_bytes(p->K, 256, slots, bwd, ns), tt::tq_smem_bytes(p->K, 256, slots, bwd, ns),
-                           bwd ? size_t(0) : tt::tl_ws_smem_bytes(p->K, 256, p->slots_ws, ns),
-                           bwd ? std::max(tt::ta_smem_bytes(p->K, 256, ns), tt::tp_smem_bytes(p->K, 256, ns))
-                               : size_t(0)});
+                     bwd ? size_t(0) : tt::tl_ws_smem_bytes(p->K, 256, p->slots_ws, ns),
+                     bwd ? std::max(tt::ta_smem_bytes(p->K, 256, ns), tt::tp_smem_bytes(p->K, 256, ns)) : size_t(0)});
   };
-  // optional overrides for tuning sweeps: TT_FWD_TILE / TT_BWD_TILE.  FP32 rings
-  // shrink (down to 3 stages) before a smaller tile is tried.
+  // FP32 rings shrink (down to 3 stages) to fit
   auto fits = [&](bool bwd) {
     int &ns = bwd ? p->nstage_b : p->nstage_f;
     const int want = ns;
@@ -518,20 +516,9 @@ int tt_plan_create(tt_plan **plan, int32_t tip_count, const int32_t *postorder,
     ns = want;
     return false;
   };
-  auto pick = [&](const int *cand, bool bwd, const char *env) {
-    const char *o = getenv(env);
-    if (o) {
-      const int want = atoi(o);
-      for (int i = 0; i < 2; ++i)
-        if (cand[i] == want && fits(bwd)) return want;
-    }
-    for (int i = 0; i < 2; ++i)
-      if (fits(bwd)) return cand[i];
-    return 0;
-  };
   if (f32) {
-    p->tile_f = pick(tt::kFwdTilesF32, false, "TT_FWD_TILE");
-    p->tile_b = pick(tt::kBwdTilesF32, true, "TT_BWD_TILE");
+    p->tile_f = fits(false) ? tt::kTlTile : 0;
+    p->tile_b = fits(true) ? tt::kTlTile : 0;
   } else if (tt::td_smem_bytes(p->K, 256, p->slots_ws, false) <= size_t(smem_max) &&
              tt::td_smem_bytes(p->K, 256, p->slots_bwd, true) <= size_t(smem_max)) {
     p->tile_f = p->tile_b = tt::td_tile_patterns(p->K);

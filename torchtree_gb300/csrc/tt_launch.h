@@ -23,15 +23,13 @@ cudaError_t kernel_smem(F *func, size_t bytes, bool max_carveout = false) {
   return kernel_smem(reinterpret_cast<const void *>(func), bytes, max_carveout);
 }
 
-// Pattern tile widths compiled per precision and pass (preferred first).
+// Pattern tile widths compiled per precision (FP64: of the allocation-free post-order, preferred first).
 // FP32 plans: both passes use one tile width (the stored partials are laid
 // out per tile): forward kTlFwdThreads threads x (kTlTile / kTlFwdThreads)
 // patterns each, adjoint one pattern per thread.
 constexpr int kTlTile = 64;
 constexpr int kTlFwdThreads = 64;
 constexpr int kTlBwdThreads = 64;
-constexpr int kFwdTilesF32[2] = {kTlTile, kTlTile};
-constexpr int kBwdTilesF32[2] = {kTlTile, kTlTile};
 constexpr int kFwdTilesF64[2] = {64, 32};
 constexpr int kStages = 4;
 // default staging-ring depths of the FP32 kernels (reduced to fit shared memory)
