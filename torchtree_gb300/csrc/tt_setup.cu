@@ -7,7 +7,7 @@
 // A log-likelihood with gradient at 69 taxa x 238 patterns runs 0.25 ms of
 // pruning kernels; as separate tensor operations the model set-up and its
 // backward were 80 more launches and 1.9 ms of host time (98 launches, 1,932 us per
-// call -> 26 launches, 622 us; value only at 137 taxa 660 -> 223 us).  The kernels here
+// call -> 20 launches, 612 us; value only at 137 taxa 660 -> 212 us).  The kernels here
 // are bound by launch latency (one CTA per sample, a few microseconds), so
 // they are written for few dependent steps, not for throughput.
 #include <algorithm>
