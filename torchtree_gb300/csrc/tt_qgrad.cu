@@ -273,23 +273,30 @@ __global__ void __launch_bounds__(128) qgrad_small_f64_kernel(const double *G, c
 // busy before (8 branches each), now 944.  20 states: one warp per CTA (25 of
 // 32 lanes hold a tile).  60 taxa, 61 states, FP64, 1 sample: 6,171 (exp and expm1
 // per pair of states, 8 branches per CTA) -> 520 us.
-template <int SP, int NS>
+//
+// FP32 plans of 20 states are bound by an item's chain of dependent phases: the
+// products unrolled over all 20 states, only the diagonal tiles' threads in the
+// diagonal sum (in FP64, 64 cycles an addition), and three further warps that stage
+// G and add that sum up while the first goes on.  30 taxa x 4 categories 189 (one warp,
+// the sum by shuffles over all lanes) -> 152 us, the three launches together.
+template <typename T, int SP, int NS>
 struct QgradCfg {
   static constexpr int IB = SP / 4, JB = NS / 4, TILES = IB * JB;
-  static constexpr int NT = (TILES + 31) / 32 * 32;
+  static constexpr bool kChain = sizeof(T) == 4 && SP == 20;
+  static constexpr int NT = kChain ? 128 : (TILES + 31) / 32 * 32;
   static constexpr int GS = SP + 4;  // row stride of the transposed G (its stores are down a column)
   static constexpr int SLABS = SP / NS;
-  template <typename T>
+  static constexpr int SUMS = kChain ? IB : NT / 32;  // parts of the diagonal sum
   static constexpr size_t smem() {
-    return sizeof(T) * (SP * SP + 2 * SP * NS + SP * GS + 4 * SP) + sizeof(double) * (NT / 32);
+    return sizeof(T) * (SP * SP + 2 * SP * NS + SP * GS + 4 * SP) + sizeof(double) * SUMS;
   }
 };
 
 template <typename T, int SP, int NS>
-__global__ void __launch_bounds__(QgradCfg<SP, NS>::NT)
+__global__ void __launch_bounds__(QgradCfg<T, SP, NS>::NT)
     wide_qgrad_kernel(const double *G, const double *lam, const double *U, const double *W, const double *bl,
                       const double *rates, int S, int B, int K, int ipc, double *sdiag, double *part) {
-  using C = QgradCfg<SP, NS>;
+  using C = QgradCfg<T, SP, NS>;
   constexpr int IB = C::IB, JB = C::JB, NT = C::NT, GS = C::GS;
   extern __shared__ __align__(128) unsigned char smem[];
   T *ug = reinterpret_cast<T *>(smem);  // [i][perm m] = U[i][m]
@@ -300,7 +307,7 @@ __global__ void __launch_bounds__(QgradCfg<SP, NS>::NT)
   T *lt = ls + SP;                       // lambda tau [SP]
   T *es = lt + SP;                       // exp(lambda tau) [SP]
   T *hx = es + SP;                       // frechet_exp [SP]
-  double *dred = reinterpret_cast<double *>(hx + SP);  // [NT / 32] diagonal sums
+  double *dred = reinterpret_cast<double *>(hx + SP);  // [SUMS] parts of the diagonal sum
   const int chunk = blockIdx.x, b = blockIdx.y, n0 = blockIdx.z * NS, tid = threadIdx.x;
   const int items = B * K, i0 = chunk * ipc, i1 = min(items, i0 + ipc);
   const bool tile = tid < C::TILES;
@@ -363,12 +370,18 @@ __global__ void __launch_bounds__(QgradCfg<SP, NS>::NT)
       for (int x = 0; x < 4; ++x)
 #pragma unroll
         for (int y = 0; y < 4; ++y) h[x][y] = T(0);
-#pragma unroll 4
-      for (int j = 0; j < S; ++j) {
+      auto step = [&](int j) {
         T ga[4], wa[4];
         V4<T>::ld(gt + j * GS + bm * 4, ga);
         V4<T>::ld(wt + j * NS + bn * 4, wa);
         outer4(h, ga, wa);
+      };
+      if constexpr (C::kChain) {
+#pragma unroll
+        for (int j = 0; j < SP; ++j) step(j);
+      } else {
+#pragma unroll 4
+        for (int j = 0; j < S; ++j) step(j);
       }
 #pragma unroll
       for (int x = 0; x < 4; ++x) V4<T>::st(hs + (bm + IB * x) * NS + bn * 4, h[x]);
@@ -381,12 +394,18 @@ __global__ void __launch_bounds__(QgradCfg<SP, NS>::NT)
       for (int x = 0; x < 4; ++x)
 #pragma unroll
         for (int y = 0; y < 4; ++y) M[x][y] = T(0);
-#pragma unroll 4
-      for (int i = 0; i < S; ++i) {
+      auto step = [&](int i) {
         T ua[4], ha[4];
         V4<T>::ld(ug + i * SP + bm * 4, ua);
         V4<T>::ld(hs + i * NS + bn * 4, ha);
         outer4(M, ua, ha);
+      };
+      if constexpr (C::kChain) {
+#pragma unroll
+        for (int i = 0; i < SP; ++i) step(i);
+      } else {
+#pragma unroll 4
+        for (int i = 0; i < S; ++i) step(i);
       }
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
@@ -395,16 +414,27 @@ __global__ void __launch_bounds__(QgradCfg<SP, NS>::NT)
         for (int y = 0; y < 4; ++y) {
           const int n = n0 + bn + JB * y;
           X[x][y] += frechet_e(lt[m], lt[n], hx[m], hx[n], tau) * M[x][y];
-          if (m == n && m < S) dsum += double(ls[m] * es[m] * M[x][y]);
+          if (!C::kChain && m == n && m < S) dsum += double(ls[m] * es[m] * M[x][y]);
         }
       }
+      if (C::kChain && bm == bn) {  // (one slab, square: the diagonal lies in these tiles)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int m = bm + IB * x;
+          if (m < S) dsum += double(ls[m] * es[m] * M[x][x]);
+        }
+        dred[bm] = dsum;
+      }
     }
-    dsum = warp_sum(dsum);  // fixed order: lanes, then warps
-    if ((tid & 31) == 0) dred[tid >> 5] = dsum;
+    if constexpr (!C::kChain) {
+      dsum = warp_sum(dsum);
+      if ((tid & 31) == 0) dred[tid >> 5] = dsum;
+    }
     __syncthreads();
-    if (tid == 0) {
+    if (tid == (C::kChain ? NT - 1 : 0)) {  // fixed order
       double s = 0.0;
-      for (int w = 0; w < NT / 32; ++w) s += dred[w];
+#pragma unroll
+      for (int w = 0; w < C::SUMS; ++w) s += dred[w];
       sdiag[(size_t(blockIdx.z) * gridDim.y + b) * items + item] = s;
     }
   }
@@ -516,8 +546,8 @@ QgradPlan qgrad_plan(const tt_plan *p) {
 template <typename T, int SP, int NS>
 cudaError_t launch_wide_qgrad(tt_plan *p, const double *lam, const double *U, const double *W, const double *bl,
                               const double *rates, double *sdiag, double *part, const QgradPlan &q, cudaStream_t s) {
-  using C = QgradCfg<SP, NS>;
-  constexpr size_t smem = C::template smem<T>();
+  using C = QgradCfg<T, SP, NS>;
+  constexpr size_t smem = C::smem();
   cudaError_t e = kernel_smem(wide_qgrad_kernel<T, SP, NS>, smem, true);
   if (e != cudaSuccess) return e;
   wide_qgrad_kernel<T, SP, NS><<<dim3(q.nchunks, p->batch, C::SLABS), C::NT, smem, s>>>(
