@@ -42,7 +42,8 @@ def _plan_bytes(T, N, K, b):
     (11, 640, 4, 9, 62, 0),   # five tiles of patterns
     (11, 641, 4, 9, 62, 64),  # six
     (11, 641, 4, 7, 62, 0),   # 11 x 4 x 7 x 6 products
-    (11, 704, 4, 9, 70, 128), (11, 704, 4, 9, 129, 0)])
+    (11, 704, 4, 9, 70, 0), (20, 1409, 4, 9, 70, 128),  # more than 64 codes: 8,192 products in 12 tiles of patterns
+    (20, 1409, 4, 8, 70, 0), (20, 1409, 4, 9, 129, 0)])
 def test_table_is_held_where_it_is_used(T, N, K, b, codes, capacity):
     assert _engine(T, N, K, b, codes).workspace_bytes - _plan_bytes(T, N, K, b) == b * T * K * capacity * 64 * 4
 

@@ -176,12 +176,15 @@ int walloc(tt_plan *p, P **ptr, size_t bytes, const char *what) {
 
 // Whether an FP32 codon pass of ntf 128-pattern tiles takes its tips' products from a table by
 // code: it costs each tip one tile and the pass a launch, and saves the products of all the tip's
-// tiles.  Post-order of 200 taxa, without and with it: 4 categories, 1 sample, 250 / 510 / 800 /
-// 1,500 patterns 216, 230 / 273, 273 / 363, 353 / 518, 475 us; 8 samples, 380 / 510 / 800 patterns
-// 894, 913 / 1,123, 1,108 / 1,835, 1,684 us; 1 category, 1 sample (launch-bound), 800 / 1,500
-// patterns 210, 214 / 244, 238 us.
-bool tip_table_pays(const tt_plan *p, int samples, int ntf) {
-  return ntf >= 6 && size_t(p->T) * samples * p->K * ntf >= 2048;
+// tiles.  Up to 64 codes, 4 categories, post-order that keeps its products, without and with it: 40 taxa x
+// 1,000 patterns x 2 samples 224, 224 us; 200 x 800 x 1 410, 401; 200 x 1,500 x 1 551, 504; 100 x 800 x 4
+// 590, 567; 200 x 2,608 x 8 5,203, 4,349.  Up to 128 (the lowest level's two tables then take 70 KB of a CTA):
+// 200 x 800 x 1 387, 416; 200 x 1,500 x 1 537, 535; 100 x 800 x 4 569, 596; 200 x 800 x 8 1,841, 1,809; 100 x
+// 2,600 x 1 472, 461.
+bool tip_table_pays(const tt_plan *p, int codes, int samples, int ntf) {
+  const size_t products = size_t(p->T) * samples * p->K * ntf;
+  if (codes > 64) return codes <= 128 && ntf >= 6 && products >= (ntf >= 12 ? 8192 : 32768);
+  return ntf >= 6 && products >= 2048;
 }
 
 // compiled (precision, padded states) -> pattern tiles of the two passes
@@ -212,11 +215,13 @@ struct Wide {
     if (e == cudaSuccess)  // the CTAs the shared memory allows per SM all resident
       e = cudaFuncSetAttribute(wide_backward_kernel<T, SP, PTB>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                int(cudaSharedmemCarveoutMaxShared));
-    if (std::is_same<T, float>::value && SP == 64 && e == cudaSuccess)
-      e = cudaFuncSetAttribute(wide_forward_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmem);
-    if (std::is_same<T, float>::value && SP == 64 && e == cudaSuccess)  // two CTAs per SM
-      e = cudaFuncSetAttribute(wide_forward_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               int(cudaSharedmemCarveoutMaxShared));
+    for (auto kernel : {wide_forward_tc_kernel<false>, wide_forward_tc_kernel<true>}) {
+      if (std::is_same<T, float>::value && SP == 64 && e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmem);
+      if (std::is_same<T, float>::value && SP == 64 && e == cudaSuccess)  // two CTAs per SM
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 int(cudaSharedmemCarveoutMaxShared));
+    }
     if (std::is_same<T, float>::value && SP == 64 && e == cudaSuccess)
       e = cudaFuncSetAttribute(wide_tip_products_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmem);
     if (std::is_same<T, float>::value && SP == 64 && e == cudaSuccess)
@@ -296,7 +301,7 @@ struct Wide {
     const int tcodes = p->C <= 64 ? 64 : 128;
     if constexpr (std::is_same<T, float>::value && SP == 64) {
       // the tips' products by code, with every pass (a captured one has to follow the matrices)
-      if (w.tc && w.d_pimg_f && p->C <= 128 && tip_table_pays(p, plan_run_samples(p), g.Npad / tc::kPT))
+      if (w.tc && w.d_pimg_f && tip_table_pays(p, p->C, plan_run_samples(p), g.Npad / tc::kPT))
         tprod = w.d_tprod[tcodes / 128];
       if (tprod) {
         wide_tip_products_tc_kernel<<<dim3(p->T, plan_run_samples(p) * p->K), tc::kThreads, tc::kSmem, s>>>(
@@ -330,8 +335,8 @@ struct Wide {
           at.ntiles = ntf;
           at.tiles_per_chunk = (ntf + chunks - 1) / chunks;
           const dim3 grid(chunks, nodes, plan_run_samples(p) * p->K);
-          wide_forward_tc_kernel<<<grid, tc::kThreads, tc::kSmem, s>>>(at, w.d_pimg_f, tprod, tcodes, p->d_status,
-                                                                       2000000000ull);
+          (tprod ? wide_forward_tc_kernel<true> : wide_forward_tc_kernel<false>)<<<grid, tc::kThreads, tc::kSmem, s>>>(
+              at, w.d_pimg_f, tprod, tcodes, p->d_status, 2000000000ull);
           p->launches += 1;
           continue;
         }
@@ -694,11 +699,11 @@ namespace {
 // is room (without it the tips take products).  Never given back before the plan: a captured pass may hold it.
 void tip_table(tt_plan *p, int codes) {
   WideState &w = *p->wide;
-  if (p->precision != TT_PRECISION_F32 || w.SP != 64 || codes > 128) return;
+  if (p->precision != TT_PRECISION_F32 || w.SP != 64) return;
   const int cap = codes <= 64 ? 64 : 128;
   float *&tprod = w.d_tprod[cap / 128];
   const size_t bytes = size_t(p->batch) * p->T * p->K * cap * w.SP * sizeof(float);
-  if (tprod || !tip_table_pays(p, p->batch, ((p->slab ? p->slab : p->N) + tc::kPT - 1) / tc::kPT) ||
+  if (tprod || !tip_table_pays(p, codes, p->batch, ((p->slab ? p->slab : p->N) + tc::kPT - 1) / tc::kPT) ||
       !product_room(bytes, w.slab_bytes))
     return;
   if (walloc(p, &tprod, bytes, "tip products")) tprod = nullptr;

@@ -251,11 +251,14 @@ __device__ __forceinline__ void tc_tip_row(const WideArgs<float> &a, const float
 // one 32 KB bulk copy per side; NULL stages P by the
 // threads.  The second side's child values are loaded into registers while
 // the first side's MMAs run.  A CTA walks a.tiles_per_chunk tiles of one
-// (node, sample, category), reusing its TMEM and barriers.  tprod: the tips'
-// products by code (`codes` rows each), or NULL: tips are staged and multiplied
-// as internal children are.  200 taxa x 2,608 patterns x 16 samples (half of all
-// children are tips): 9,960 us -> 6,770 here, 1,380 in the
+// (node, sample, category), reusing its TMEM and barriers.  TAB: a tip's products come
+// from the table tprod (`codes` rows each) and the next tile's values are loaded during a
+// tile's epilogue; otherwise tips are staged and multiplied as internal children are
+// (the table's branches and the loads' registers cost that form 5 %: 200 taxa x 2,608
+// patterns x 8 samples 4,550 us with them, 4,264 without).  200 taxa x 2,608 patterns x
+// 16 samples (half of all children are tips): 9,960 us -> 6,770 here, 1,380 in the
 // tips-only level (wide_tip_pair_kernel) and 240 for the table.
+template <bool TAB>
 __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const WideArgs<float> a, const float *pimg,
                                                                          const float *tprod, int codes, int *status,
                                                                          unsigned long long timeout_ns) {
@@ -286,8 +289,8 @@ __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const 
   tc::fence_after_sync();
   const uint32_t tmem = *tslot;
   // tips that have a table of products (uniform over the CTA)
-  const float *tab_l = tprod && l < a.tips ? tprod + ((size_t(b) * a.tips + l) * a.K + k) * codes * SP : nullptr;
-  const float *tab_r = tprod && r < a.tips ? tprod + ((size_t(b) * a.tips + r) * a.K + k) * codes * SP : nullptr;
+  const float *tab_l = TAB && l < a.tips ? tprod + ((size_t(b) * a.tips + l) * a.K + k) * codes * SP : nullptr;
+  const float *tab_r = TAB && r < a.tips ? tprod + ((size_t(b) * a.tips + r) * a.K + k) * codes * SP : nullptr;
   const bool two = !tab_l && !tab_r;
   // per side c: stage, then one thread issues the side's MMAs into TMEM
   // columns [64c, 64c + 64); the next side's staging waits for their completion
@@ -312,10 +315,14 @@ __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const 
       for (int j = 0; j < SP; ++j) xv[j] = __ldg(src + size_t(j) * a.Npad);
     }
   };
-  if (!tab_l) load_x(l, n0);
-  else if (!tab_r) load_x(r, n0);
+  auto load_first = [&](int n0) {
+    if (!tab_l) load_x(l, n0);
+    else if (!tab_r) load_x(r, n0);
+  };
+  if (TAB) load_first(n0);
   for (int tile = t0; tile < t1 && ok; ++tile) {
     n0 = tile * tc::kPT;
+    if (!TAB) load_first(n0);
     for (int c = 0; c < 2 && ok; ++c) {
       if (c ? tab_r : tab_l) continue;
       const int child = c ? r : l;
@@ -376,10 +383,7 @@ __global__ void __launch_bounds__(tc::kThreads, 2) wide_forward_tc_kernel(const 
       if (ok) phase ^= 1;
     }
     if (ok) {
-      if (tile + 1 < t1) {  // the next tile's first values travel during this one's epilogue
-        if (!tab_l) load_x(l, n0 + tc::kPT);
-        else if (!tab_r) load_x(r, n0 + tc::kPT);
-      }
+      if (TAB && tile + 1 < t1) load_first(n0 + tc::kPT);
       // this thread's pattern = TMEM lane 32 * warp + lane
       const uint32_t lane_addr = tmem + (uint32_t(32 * warp) << 16);
       const int n = n0 + tid;
