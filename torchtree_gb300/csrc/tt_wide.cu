@@ -343,7 +343,12 @@ struct Wide {
       }
       const int nodes = w.fwd_off[lv + 1] - w.fwd_off[lv];
       if constexpr (SP == kColStates) {
-        if (lv + 2 < w.fwd_off.size()) {  // every level but the root's: about eight waves of three CTAs per SM
+        // Every level but the root's, in FP32 those that fill the GPU: below 256 (node, sample, category, 128
+        // patterns) the table of every CTA is on the level's chain.  32 levels of one node with a tip, without and
+        // with it: 32 units 316, 373 us, 128 units 316, 372, 256 units 374, 375, 512 units 438, 439; levels of
+        // internal children, 16 to 2 nodes: 16 units a node 108, 105, 512 units a node 437, 340.
+        const bool fills = sizeof(T) == 8 || size_t(nodes) * p->batch * p->K * (g.Npad / 128) >= 256;
+        if (lv + 2 < w.fwd_off.size() && fills) {  // about eight waves of three CTAs per SM
           constexpr int tile = kColThreads * kColPatterns<T>;
           WideArgs<T> ac = a;
           ac.ntiles = (g.Npad + tile - 1) / tile;
